@@ -24,8 +24,10 @@ struct TrainView {
   float4* final_rgba;         // [npx] final colour of the forward
   float4* out_rgba;           // forward: [npx] caller's image, or null
   const float4* dl_drgba;     // backward: [npx] dL/dRGBA
-  uint2* work;                // [work_cap] (pixel, segment) items the forward appends
-  unsigned* work_count;       // [0] items appended
+  // (pixel, segment) items the forward appends: segments with a sample outside
+  // empty macrocells from the front, all-empty segments from the back
+  uint2* work;                // [work_cap]
+  unsigned* work_count;       // [0] items at the front, [1] at the back, [2..3] samples (64 bits) of the latter
   int* overflow;              // set when a pixel needs more checkpoints than ckpt_cap
   const int* chunk_order;     // forward: 8x4 chunk ids in the order to march them, or null (ring order)
   unsigned ckpt_cap;          // checkpoints per pixel
@@ -63,12 +65,14 @@ struct TrainArgs {
   const int* run_views;
   // Backward: items [item_base[v], item_base[v+1]) are view slot v's
   // (pixel, segment) items; item_base[n_views] is the launch's item count.
+  // empty_base is the same for the all-empty segments.
   const unsigned* item_base;
-  unsigned* grab;             // the launch's item counter (zero before it)
+  const unsigned* empty_base;
+  unsigned* grab;             // the launch's item counters (zero before it): [0], and [1] for all-empty segments
   // Backward of one view (n_views == 1): the view itself and its item count,
   // in the launch parameters instead of tv / item_base.
   TrainView one;
-  unsigned one_items;
+  unsigned one_items, one_empty;
   float* dtf;                 // [n_tf*4] accumulated
   float4* dgrid4;             // density gradient in x-quads: element (x,y,z) holds the
                               // contributions to voxels x, x+1, x+2 (w unused)
@@ -84,6 +88,9 @@ cudaError_t launch_forward_train(const TrainArgs& a, unsigned items, int max_gri
 int forward_train_blocks_per_sm(int n_tf, bool many);
 // One persistent backward over the launch's views' items (a.tv, a.item_base).
 cudaError_t launch_backward(const TrainArgs& a, int grid, cudaStream_t s);
+// The all-empty segments of the same views (a.empty_base): the gradient of
+// the transfer function's alpha entries (a.dtf).  `sms` CTA groups.
+cudaError_t launch_backward_empty(const TrainArgs& a, int sms, cudaStream_t s);
 // out[v] += quads[v].x + quads[v-1].y + quads[v-2].z along x, for a grid of
 // dims; every quad of the grid is zero afterwards.
 cudaError_t launch_fold_quads(float4* quads, float* out, const int dims[3], cudaStream_t s);

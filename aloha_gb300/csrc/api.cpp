@@ -1457,22 +1457,22 @@ int backward_views(aloha_ctx* c, int n_views, const int* view_ids, const float* 
   CUDA_TRY(c, cudaSetDevice(c->device));
   // every view's overflow flag and segment count, read with one wait
   std::vector<int> overflow(n_views, 0);
-  std::vector<unsigned> segments(n_views, 0);
+  std::vector<unsigned> segments(2 * (size_t)n_views, 0);  // per view: with full samples, all-empty
   for (int i = 0; i < n_views; ++i) {
     const TrainState& t = c->views[view_ids[i]].train;
     CUDA_TRY(c, cudaMemcpyAsync(&overflow[i], t.overflow, sizeof(int), cudaMemcpyDeviceToHost, s));
-    CUDA_TRY(c, cudaMemcpyAsync(&segments[i], t.work_count, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+    CUDA_TRY(c, cudaMemcpyAsync(&segments[2 * (size_t)i], t.work_count, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost,
+                                s));
   }
   CUDA_TRY(c, cudaStreamSynchronize(s));
-  std::vector<unsigned> item_base(n_views + 1, 0);
+  unsigned long long all_segments = 0;
   for (int i = 0; i < n_views; ++i) {
     if (overflow[i])
       return c->fail(ALOHA_ERR_OUT_OF_RANGE, "a ray of view %d needed more checkpoints than reserved", view_ids[i]);
-    const TrainState& t = c->views[view_ids[i]].train;
-    const unsigned long long n = std::min<unsigned long long>(segments[i], t.npx * t.cap);
-    if (item_base[i] + n >= 0xffffffffull)
+    // the two lists share t.npx * t.cap entries
+    all_segments += (unsigned long long)segments[2 * (size_t)i] + segments[2 * (size_t)i + 1];
+    if (all_segments >= 0xffffffffull)
       return c->fail(ALOHA_ERR_UNSUPPORTED, "too many checkpoint segments in one backward");
-    item_base[i + 1] = item_base[i] + (unsigned)n;
   }
   const size_t tf_bytes = (size_t)c->n_tf * 4 * sizeof(float), g_bytes = grid_elems * sizeof(float);
   const bool h_tf = dl_dtf && !is_device_pointer(dl_dtf), h_grid = with_density && !is_device_pointer(dl_ddensity);
@@ -1521,7 +1521,7 @@ int backward_views(aloha_ctx* c, int n_views, const int* view_ids, const float* 
     if (done[first]) continue;
     const unsigned k = c->views[view_ids[first]].train.k;
     std::vector<TrainView> tvs;
-    std::vector<unsigned> base{0};
+    std::vector<unsigned> base{0}, empty_base{0};
     for (int i = first; i < n_views; ++i) {
       if (done[i] || c->views[view_ids[i]].train.k != k) continue;
       done[i] = 1;
@@ -1529,11 +1529,13 @@ int backward_views(aloha_ctx* c, int n_views, const int* view_ids, const float* 
       tv.dl_drgba = off_dl[i] != SIZE_MAX ? reinterpret_cast<const float4*>(st + off_dl[i])
                                           : reinterpret_cast<const float4*>(dl_drgba[i]);
       tvs.push_back(tv);
-      base.push_back(base.back() + (item_base[i + 1] - item_base[i]));
+      base.push_back(base.back() + segments[2 * (size_t)i]);
+      empty_base.push_back(empty_base.back() + segments[2 * (size_t)i + 1]);
     }
     std::vector<char*> dev;
     rc = upload_train_tables(c, {{tvs.data(), tvs.size() * sizeof(TrainView)},
-                                 {base.data(), base.size() * sizeof(unsigned)}}, s, dev);
+                                 {base.data(), base.size() * sizeof(unsigned)},
+                                 {empty_base.data(), empty_base.size() * sizeof(unsigned)}}, s, dev);
     if (rc) return rc;
     TrainArgs a = train_args(c);
     a.k = k;
@@ -1551,19 +1553,23 @@ int backward_views(aloha_ctx* c, int n_views, const int* view_ids, const float* 
     bool all_large = true;
     for (size_t i = 0; i + 1 < base.size(); ++i)
       if ((unsigned long long)(base[i + 1] - base[i]) < 16 * resident) all_large = false;
+    a.tv = reinterpret_cast<const TrainView*>(dev[1]);
+    a.empty_base = reinterpret_cast<const unsigned*>(dev[3]);
     if (tvs.size() == 1 || all_large) {
       for (size_t i = 0; i < tvs.size(); ++i) {
-        if (i > 0) CUDA_TRY(c, cudaMemsetAsync(a.grab, 0, sizeof(unsigned), s));
+        if (i > 0) CUDA_TRY(c, cudaMemsetAsync(a.grab, 0, 2 * sizeof(unsigned), s));
         a.n_views = 1;
         a.one = tvs[i];
         a.one_items = base[i + 1] - base[i];
+        a.one_empty = empty_base[i + 1] - empty_base[i];
         CUDA_TRY(c, launch_backward(a, c->num_sms * per_sm, s));
+        if (dtf && a.one_empty) CUDA_TRY(c, launch_backward_empty(a, c->num_sms, s));
       }
     } else {
-      a.tv = reinterpret_cast<const TrainView*>(dev[1]);
       a.n_views = (int)tvs.size();
       a.item_base = reinterpret_cast<const unsigned*>(dev[2]);
       CUDA_TRY(c, launch_backward(a, c->num_sms * per_sm, s));
+      if (dtf && empty_base.back()) CUDA_TRY(c, launch_backward_empty(a, c->num_sms, s));
     }
   }
   if (with_density) {

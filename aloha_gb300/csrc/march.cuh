@@ -378,7 +378,8 @@ __device__ __forceinline__ void composite_step(float4& color, const float4 c, fl
 // t, the samples already taken in the brick and the colour so far.  The
 // render passes NoHook; the differentiable forward stores checkpoints.  An
 // active hook keeps `left`, the samples it lets pass before it needs to see
-// one again, so runs of skipped samples only stop where it does.
+// one again, so runs of skipped samples only stop where it does, and is told
+// of full samples through `full_segment`.
 struct NoHook {
   static constexpr bool kActive = false;
   __device__ __forceinline__ void operator()(float, uint32_t, const float4&) {}
@@ -530,6 +531,7 @@ __device__ __forceinline__ uint32_t march_brick(const DevBrick& b, const float4*
       t_cell = tb;
     }
     hook(t, n, color);
+    if constexpr (Hook::kActive) hook.full_segment = true;
     ++n;
     StencilOut s;
     if constexpr (Loads::kStaged)
