@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(128, MINB) forward_train_kernel(TrainArgs a, u
     } else if (!ring_chunk(pos, cxn, cyn, ccx, ccy)) {
       continue;
     }
-    n += train_subtile(a, tv, v, tf_s, ccx * 8 + (lane & 7), ccy * 4 + (lane >> 3), lane);
+    n += train_subtile(a, tv, v, tf_s, ccx * 8 + tile_x(lane), ccy * 4 + tile_y(lane), lane);
   }
   count_samples(a.counter, n);
 }

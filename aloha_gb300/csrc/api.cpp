@@ -794,8 +794,7 @@ static int upload_brick(aloha_ctx* c, int b, const float* src) {
   const DevBrick& db = c->dev_bricks[b];
   float4* alloc = static_cast<float4*>(c->voxels.ptr) + c->brick_offset[b];
   CUDA_TRY(c, cudaMemset(c->flag.ptr, 0, sizeof(int)));
-  CUDA_TRY(c, launch_pad_brick(dsrc, nx, ny, nz, alloc, db.sy, db.sz / db.sy, nz + 2 * kApron,
-                               static_cast<int*>(c->flag.ptr), 0));
+  CUDA_TRY(c, launch_pad_brick(dsrc, nx, ny, nz, alloc, db.sy, db.sz, static_cast<int*>(c->flag.ptr), 0));
   CUDA_TRY(c, launch_macrocell_range(db, static_cast<float2*>(c->mc_ranges.ptr) + c->mc_offset[b], 0));
   c->empty_dirty = true;
   int bad = 0;  // this copy also waits for the two kernels above
@@ -825,15 +824,15 @@ int aloha_set_bricks(aloha_ctx* c, const aloha_brick_desc* descs, const float* c
       if (!(std::isfinite(d.space_lo[a]) && std::isfinite(d.space_hi[a]) && d.space_lo[a] < d.space_hi[a]))
         return c->fail(ALOHA_ERR_INVALID_ARGUMENT, "brick %d: empty or non-finite space range", b);
     }
-    // rows padded to an even number of quads (32-byte aligned rows)
-    const int px = ((nsz[0] + 2 * kApron) + 1) & ~1, py = nsz[1] + 2 * kApron, pz = nsz[2] + 2 * kApron;
-    const size_t elems = (size_t)px * py * pz;
+    const int px = row_pitch(nsz[0]), pz = nsz[2] + 2 * kApron;
+    const long long slice = slice_pitch(px, nsz[1]);
+    const size_t elems = (size_t)slice * pz;
     if (elems >= (size_t)1 << 31)
       return c->fail(ALOHA_ERR_INVALID_ARGUMENT, "brick %d too large for 32-bit voxel offsets; split it", b);
     offs[b] = total;
     total += (elems + 15) & ~(size_t)15;  // 256-byte aligned bricks (in quads)
     db[b].sy = px;
-    db[b].sz = px * py;
+    db[b].sz = (int)slice;
     for (int a = 0; a < 3; ++a) {
       db[b].n[a] = nsz[a];
       db[b].lo[a] = (float)d.voxel_lo[a];

@@ -18,6 +18,24 @@ namespace aloha {
 // from four rows and hit L1 less often).  Quads cut the loads per sample from
 // 20 to 7 at four times the HBM footprint.
 constexpr int kApron = 2;
+// Pitches of the padded array, in quads.  A warp's 16-byte loads are served a
+// quarter warp at a time, and quads of different 128-byte lines collide when
+// they lie at the same offset (of eight) in their line.  Neighbouring rays
+// read neighbouring voxels, along any axis, so the pitches are chosen for
+// steps along y and z to land on other offsets: rows of 2 or 6 (mod 8) quads,
+// slices of 4 (mod 8).  With rows of nx + 4 and slices of their product, a
+// brick of 128, 256 or 512 voxels had slices of 0 (mod 8), so all rays of a
+// pixel row that ran along z collided.  Together with the 2x4 quarter warps
+// of tile_x / tile_y: uneven 24-view batch 10.46 -> 10.01 ms, 512^3
+// transfer-function step 6.35 -> 6.16 ms, odd volume's frame 681 -> 626 us.
+inline int row_pitch(int nx) {
+  const int px = nx + 2 * kApron;
+  return px + ((2 - px) & 3);
+}
+inline long long slice_pitch(int px, int ny) {
+  const long long sz = (long long)px * (ny + 2 * kApron);
+  return sz + ((4 - sz) & 7);
+}
 constexpr int kMaxViews = 4096;
 constexpr int kMaxTF = 2048;  // (n + 4) float4 entries stay under 48 KB of shared memory
 
@@ -156,7 +174,8 @@ cudaError_t launch_composite_f32(const float4* imgs, const int* order, int n_ran
                                  cudaStream_t s);
 cudaError_t launch_composite_u8(const uint32_t* imgs, const int* order, int n_ranks, int npx, uint32_t* fb,
                                 cudaStream_t s);
-cudaError_t launch_pad_brick(const float* src, int nx, int ny, int nz, float4* dst_alloc, int px, int py, int pz,
+// Fills a brick's padded array (pitches px, sz in quads).
+cudaError_t launch_pad_brick(const float* src, int nx, int ny, int nz, float4* dst_alloc, int px, int sz,
                              int* nonfinite_flag, cudaStream_t s);
 // Persistent render launch; `batch` selects the instance tuned for batches.
 constexpr int kSingleRenderBlocks = 5, kBatchRenderBlocks = 7;  // CTAs per SM

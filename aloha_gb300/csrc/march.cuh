@@ -894,6 +894,12 @@ __device__ __forceinline__ uint32_t render_pixel(const FrameArgs& a, const DevVi
   return total;
 }
 
+// Pixel of a lane in its warp's 8x4 tile: each quarter warp, the unit in which
+// 16-byte loads are served, takes a 2x4 block, whose rays read fewer distinct
+// quads than a row of eight does.
+__device__ __forceinline__ int tile_x(int lane) { return (lane & 1) | ((lane >> 2) & 6); }
+__device__ __forceinline__ int tile_y(int lane) { return (lane >> 1) & 3; }
+
 // Work slot k of a view -> chunk (cx, cy) in centre-out square rings; false
 // for slots outside the chunk grid.  Ring r >= 1 holds slots
 // [(2r-1)^2, (2r+1)^2), walked up the right edge, left along the top, down

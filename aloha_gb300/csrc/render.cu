@@ -91,8 +91,8 @@ __global__ void __launch_bounds__(kRenderThreads, MINB) render_warps_kernel(Batc
     const int x0 = ccx * CW, y0 = ccy * CH;
 #pragma unroll 1
     for (int sub = 0; sub < (CW / 8) * (CH / 4); ++sub) {
-      const int x = x0 + (sub % (CW / 8)) * 8 + (lane & 7);
-      const int y = y0 + (sub / (CW / 8)) * 4 + (lane >> 3);
+      const int x = x0 + (sub % (CW / 8)) * 8 + tile_x(lane);
+      const int y = y0 + (sub / (CW / 8)) * 4 + tile_y(lane);
       if (x < v.width && y < v.height)
         n += render_pixel(b.f, v, tf_s, x, y, fb, (size_t)x + (size_t)v.width * y, loads);
     }
@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(kRenderThreads, MINB) render_split_kernel(Spli
     const int slot = (int)(code >> 7), k = (int)(code & 127u);
     int cx, cy;
     split_chunk(s, slot, cxn, cyn, cx, cy);
-    const int x = cx * 8 + (lane & 7), y = cy * 4 + (lane >> 3);
+    const int x = cx * 8 + tile_x(lane), y = cy * 4 + tile_y(lane);
     const bool valid = x < W && y < H;
     const int pixel = x + W * y;
     const unsigned long long mask = __ldg(s.masks + slot);
@@ -368,8 +368,8 @@ __global__ void composite_u8_kernel(const uint32_t* __restrict__ imgs, const int
 // their threads the row's elements, so the index arithmetic is one division
 // per row; a row reads four source rows, each coalesced along x.
 __global__ void pad_brick_kernel(const float* __restrict__ src, int nx, int ny, int nz, float4* __restrict__ dst,
-                                 int px, int py, int pz, int* nonfinite) {
-  const int rows = py * pz;
+                                 int px, int sz, int* nonfinite) {
+  const int py = ny + 2 * kApron, rows = py * (nz + 2 * kApron);
   bool bad = false;
   for (int r = blockIdx.x; r < rows; r += gridDim.x) {
     const int y = r % py, z = r / py;
@@ -379,7 +379,7 @@ __global__ void pad_brick_kernel(const float* __restrict__ src, int nx, int ny, 
     const float* __restrict__ r10 = src + ((size_t)z0 * ny + y1) * nx;
     const float* __restrict__ r01 = src + ((size_t)z1 * ny + y0) * nx;
     const float* __restrict__ r11 = src + ((size_t)z1 * ny + y1) * nx;
-    float4* __restrict__ out = dst + (size_t)r * px;
+    float4* __restrict__ out = dst + ((size_t)z * sz + (size_t)y * px);
     for (int x = threadIdx.x; x < px; x += blockDim.x) {
       const int sx = min(max(x - kApron, 0), nx - 1);
       const float4 v = make_float4(__ldg(r00 + sx), __ldg(r10 + sx), __ldg(r01 + sx), __ldg(r11 + sx));
@@ -579,11 +579,11 @@ cudaError_t launch_composite_u8(const uint32_t* imgs, const int* order, int n_ra
   return cudaGetLastError();
 }
 
-cudaError_t launch_pad_brick(const float* src, int nx, int ny, int nz, float4* dst, int px, int py, int pz,
-                             int* nonfinite, cudaStream_t s) {
-  const int rows = py * pz;
+cudaError_t launch_pad_brick(const float* src, int nx, int ny, int nz, float4* dst, int px, int sz, int* nonfinite,
+                             cudaStream_t s) {
+  const int rows = (ny + 2 * kApron) * (nz + 2 * kApron);
   const int g = rows < 152 * 32 ? rows : 152 * 32;  // CTAs of 128 threads take rows
-  pad_brick_kernel<<<g < 1 ? 1 : g, 128, 0, s>>>(src, nx, ny, nz, dst, px, py, pz, nonfinite);
+  pad_brick_kernel<<<g < 1 ? 1 : g, 128, 0, s>>>(src, nx, ny, nz, dst, px, sz, nonfinite);
   return cudaGetLastError();
 }
 
