@@ -61,7 +61,7 @@ __device__ __forceinline__ const int* rank_bricks(const TrainArgs& a, const DevV
 //
 // With CAN_STOP the walk also ends, before the next sample, once *stop is set
 // (by the visitor).
-template <bool SKIP, bool CAN_STOP = false, class Visit>
+template <bool INNER, bool SKIP, bool CAN_STOP = false, class Visit>
 __device__ __forceinline__ uint32_t walk_samples(const TrainArgs& a, const DevView& v, const float4* tf_s,
                                                  const Ray& ray, uint32_t pixel, Walk w, float t_resume,
                                                  uint32_t nb0, bool resume, float4& color, uint32_t max_samples,
@@ -133,9 +133,9 @@ __device__ __forceinline__ uint32_t walk_samples(const TrainArgs& a, const DevVi
           continue;
         }
       }
-      const StencilOut s = stencil<true>(b.base, b.sy, b.sz, b.n[0], b.n[1], b.n[2], ux, uy, uz);
+      const StencilOut s = stencil<INNER, true>(b.base, b.sy, b.sz, b.n[0], b.n[1], b.n[2], ux, uy, uz);
       const float shade = shade_factor(s, ray);
-      const float4 c = tf_lookup(tf_s, a.n_tf, nf, s.value);
+      const float4 c = tf_lookup<INNER>(tf_s, a.n_tf, nf, s.value);
       visit(b, t, w, nb, ux, uy, uz, s, shade, c, color);
       composite_step(color, c, shade);
       ++n;
@@ -203,6 +203,7 @@ struct CheckpointHook {
 // colour is the render's bit for bit), checkpoints, final colour, and the
 // warp-aggregated append of (pixel, segment) items.  Returns the lane's
 // sample count.
+template <bool INNER>
 __device__ __forceinline__ uint32_t train_subtile(const TrainArgs& a, const TrainView& tv, const DevView& v,
                                                   const float4* tf_s, int x, int y, int lane) {
   const bool active = x < v.width && y < v.height;
@@ -222,7 +223,7 @@ __device__ __forceinline__ uint32_t train_subtile(const TrainArgs& a, const Trai
       if (!slab(ray, b.space_lo, b.space_hi, hook.tmin, 1e10f, t0, t1)) continue;
       const float ils = jitter(a.jitter_mode, a.jitter_value, pixel, (uint32_t)a.accum_id, hook.draw++);
       hook.j = j;
-      n += march_brick(b, tf_s, a.n_tf, ray, t0, t1, ils, a.dt, a.et_alpha, color, hook);
+      n += march_brick<INNER>(b, tf_s, a.n_tf, ray, t0, t1, ils, a.dt, a.et_alpha, color, hook);
       hook.tmin = t1 + 1e-20f;
       if (!(color.w < a.et_alpha)) break;
     }
@@ -294,7 +295,7 @@ __device__ __forceinline__ void forward_item(const TrainArgs& a, unsigned item, 
 // Persistent training forward over the launch's views: warps pull items
 // (a view's 8 x 4 chunk, in its cost order when it has one, else
 // centre-out, as the render does) from the launch's counter.
-template <int MINB>
+template <int MINB, bool INNER>
 __global__ void __launch_bounds__(128, MINB) forward_train_kernel(TrainArgs a, unsigned items) {
   extern __shared__ float4 tf_s[];
   load_tf(tf_s, a.tf, a.n_tf);
@@ -319,7 +320,7 @@ __global__ void __launch_bounds__(128, MINB) forward_train_kernel(TrainArgs a, u
     } else if (!ring_chunk(pos, cxn, cyn, ccx, ccy)) {
       continue;
     }
-    n += train_subtile(a, tv, v, tf_s, ccx * 8 + tile_x(lane), ccy * 4 + tile_y(lane), lane);
+    n += train_subtile<INNER>(a, tv, v, tf_s, ccx * 8 + tile_x(lane), ccy * 4 + tile_y(lane), lane);
   }
   count_samples(a.counter, n);
 }
@@ -485,12 +486,13 @@ struct OpaqueEvent {
 // transmittance is below 2^-24 (the rest cannot move the result) or the ray
 // ends.  Skipped samples (alpha 0) leave R unchanged, so empty space is
 // stepped over.  Returns (R_rgb, R_a).
+template <bool INNER>
 __device__ __forceinline__ float4 suffix_composite(const TrainArgs& a, const DevView& v, const float4* tf_s,
                                                    const Ray& ray, uint32_t pixel, const OpaqueEvent& e) {
   float r0 = 0.f, r1 = 0.f, r2 = 0.f, tp = 1.0f;
   bool stop = false;
   float4 col = e.after;
-  walk_samples<true, true>(
+  walk_samples<INNER, true, true>(
       a, v, tf_s, ray, pixel, e.w, e.t_next, e.nb_next, true, col, 0xffffffffu,
       [&](const DevBrick&, float, const Walk&, uint32_t, float, float, float, const StencilOut&, float shade,
           const float4& c, const float4&) {
@@ -511,7 +513,7 @@ constexpr unsigned kBackwardGrab = 256;  // most items a backward warp takes per
 // One backward item: the replay of segment (pixel, ck) of view v and its
 // adjoint, added to dtf_s (shared, WITH_TF) and the x-quad density gradient
 // (WITH_DENSITY).  Returns the samples replayed.
-template <bool WITH_TF, bool WITH_DENSITY>
+template <bool INNER, bool WITH_TF, bool WITH_DENSITY>
 __device__ __forceinline__ uint32_t backward_item(const TrainArgs& a, const DevView& v, const int* __restrict__ rb,
                                                   const float4* tf_s, float* dtf_s, float nf, uint32_t pixel,
                                                   const Checkpoint& ck, const float4 F, const float4 g) {
@@ -526,7 +528,7 @@ __device__ __forceinline__ uint32_t backward_item(const TrainArgs& a, const DevV
   float pend[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   OpaqueEvent events[kMaxEvents];
   int n_events = 0;
-  const uint32_t n = walk_samples<!WITH_TF>(
+  const uint32_t n = walk_samples<INNER, !WITH_TF>(
       a, v, tf_s, ray, pixel, w0, ck.t, ck.nb, true, color, a.k,
       [&](const DevBrick& b, float t, const Walk& wcur, uint32_t nb, float ux, float uy, float uz,
           const StencilOut& s, float shade, const float4& c, const float4& col) {
@@ -608,7 +610,7 @@ __device__ __forceinline__ uint32_t backward_item(const TrainArgs& a, const DevV
   // near-opaque samples: correct the alpha adjoint by the true one
   for (int k = 0; k < n_events; ++k) {
     const OpaqueEvent& e = events[k];
-    const float4 R = suffix_composite(a, v, tf_s, ray, pixel, e);
+    const float4 R = suffix_composite<INNER>(a, v, tf_s, ray, pixel, e);
     const float gtrue = fmaf(g.w, R.w, -fmaf(g.x, R.x, fmaf(g.y, R.y, g.z * R.z)));
     const float dd = e.oma * (gtrue - e.gA);  // change of dL/d(alpha of the sample)
     if (dd == 0.f) continue;
@@ -641,7 +643,7 @@ __device__ __forceinline__ uint32_t backward_item(const TrainArgs& a, const DevV
 // item looks its view up; else to the one view passed in the parameters
 // (a.one), whose pointers then stay in the constant bank, as the replay's
 // register budget wants.
-template <bool WITH_TF, bool WITH_DENSITY, bool MULTI>
+template <bool INNER, bool WITH_TF, bool WITH_DENSITY, bool MULTI>
 __global__ void __launch_bounds__(128, 5) backward_kernel(TrainArgs a) {
   extern __shared__ float4 smem[];
   float4* tf_s = smem;                                         // n_tf + 4 entries
@@ -688,12 +690,12 @@ __global__ void __launch_bounds__(128, 5) backward_kernel(TrainArgs a) {
         const DevView v = a.views[tv.view];
         const uint2 wk = tv.work[item - __ldg(a.item_base + slot)];
         const Checkpoint ck = tv.ckpt[(size_t)wk.x * tv.ckpt_cap + wk.y];
-        nsamp += backward_item<WITH_TF, WITH_DENSITY>(a, v, rank_bricks(a, v), tf_s, dtf_s, nf, wk.x, ck,
+        nsamp += backward_item<INNER, WITH_TF, WITH_DENSITY>(a, v, rank_bricks(a, v), tf_s, dtf_s, nf, wk.x, ck,
                                                       tv.final_rgba[wk.x], tv.dl_drgba[wk.x]);
       } else {
         const uint2 wk = a.one.work[item];
         const Checkpoint ck = a.one.ckpt[(size_t)wk.x * a.one.ckpt_cap + wk.y];
-        nsamp += backward_item<WITH_TF, WITH_DENSITY>(a, v1, rb1, tf_s, dtf_s, nf, wk.x, ck, a.one.final_rgba[wk.x],
+        nsamp += backward_item<INNER, WITH_TF, WITH_DENSITY>(a, v1, rb1, tf_s, dtf_s, nf, wk.x, ck, a.one.final_rgba[wk.x],
                                                       a.one.dl_drgba[wk.x]);
       }
     }
@@ -724,7 +726,7 @@ __global__ void __launch_bounds__(128, 5) backward_kernel(TrainArgs a) {
 // the replayed ones and 3.34 ms here; the density-only replay of 6 views of
 // 256^3, which only loses the empty rows between its lanes, went from 2.2 to
 // 1.3 ms.
-template <bool MULTI>
+template <bool INNER, bool MULTI>
 __global__ void __launch_bounds__(128, kBackwardEmptyBlocks) backward_empty_kernel(TrainArgs a) {
   extern __shared__ float4 smem[];
   float4* tf_s = smem;                                         // n_tf + 4 entries
@@ -790,7 +792,7 @@ __global__ void __launch_bounds__(128, kBackwardEmptyBlocks) backward_empty_kern
         const float lox = b.lo[0], loy = b.lo[1], loz = b.lo[2];
         while (t < t1 && nb < cap && n < a.k) {
           const StencilOut s =
-              stencil<true>(base, sy, sz, nx, ny, nz, fmaf(t, ray.d[0], ray.o[0]) - lox,
+              stencil<INNER, true>(base, sy, sz, nx, ny, nz, fmaf(t, ray.d[0], ray.o[0]) - lox,
                             fmaf(t, ray.d[1], ray.o[1]) - loy, fmaf(t, ray.d[2], ray.o[2]) - loz);
           const float ex = s.gx + 1e-4f, ey = s.gy + 1e-4f, ez = s.gz + 1e-4f;
           const float inv = rsqrtf(fmaf(ex, ex, fmaf(ey, ey, ez * ez)));
@@ -840,38 +842,48 @@ size_t backward_smem(int n_tf, bool with_tf) {
 
 }  // namespace
 
-cudaError_t launch_forward_train(const TrainArgs& a, unsigned items, int max_grid, bool many, cudaStream_t s) {
+using TrainKernel = void (*)(TrainArgs, unsigned);
+static TrainKernel forward_train(bool many, bool inner) {
+  if (many) return inner ? forward_train_kernel<kTrainForwardBlocksMany, true>
+                         : forward_train_kernel<kTrainForwardBlocksMany, false>;
+  return inner ? forward_train_kernel<kTrainForwardBlocks, true> : forward_train_kernel<kTrainForwardBlocks, false>;
+}
+
+cudaError_t launch_forward_train(const TrainArgs& a, unsigned items, int max_grid, bool many, bool inner,
+                                 cudaStream_t s) {
   int grid = (int)std::min<unsigned>((items + 3) / 4, (unsigned)max_grid);
   if (grid < 1) grid = 1;
   const size_t smem = (size_t)(a.n_tf + 4) * sizeof(float4);
-  if (many)
-    forward_train_kernel<kTrainForwardBlocksMany><<<grid, 128, smem, s>>>(a, items);
-  else
-    forward_train_kernel<kTrainForwardBlocks><<<grid, 128, smem, s>>>(a, items);
+  forward_train(many, inner)<<<grid, 128, smem, s>>>(a, items);
   return cudaGetLastError();
 }
 
 int forward_train_blocks_per_sm(int n_tf, bool many) {
   int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-          &n, many ? forward_train_kernel<kTrainForwardBlocksMany> : forward_train_kernel<kTrainForwardBlocks>, 128,
-          (size_t)(n_tf + 4) * sizeof(float4)) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, forward_train(many, true), 128,
+                                                    (size_t)(n_tf + 4) * sizeof(float4)) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
   return n;
 }
 
-cudaError_t launch_backward(const TrainArgs& a, int grid, cudaStream_t s) {
+using BackwardKernel = void (*)(TrainArgs);
+template <bool INNER>
+static BackwardKernel backward(bool with_tf, bool with_density, bool multi) {
+  if (multi)
+    return !with_tf ? backward_kernel<INNER, false, true, true>
+                    : (with_density ? backward_kernel<INNER, true, true, true> : backward_kernel<INNER, true, false, true>);
+  return !with_tf ? backward_kernel<INNER, false, true, false>
+                  : (with_density ? backward_kernel<INNER, true, true, false> : backward_kernel<INNER, true, false, false>);
+}
+
+cudaError_t launch_backward(const TrainArgs& a, int grid, bool inner, cudaStream_t s) {
   const bool with_tf = a.dtf != nullptr, with_density = a.dgrid4 != nullptr;
   if (!with_tf && !with_density) return cudaErrorInvalidValue;
   const size_t smem = backward_smem(a.n_tf, with_tf);
   const bool multi = a.n_views > 1;
-  void (*k)(TrainArgs) =
-      multi ? (!with_tf ? backward_kernel<false, true, true>
-                        : (with_density ? backward_kernel<true, true, true> : backward_kernel<true, false, true>))
-            : (!with_tf ? backward_kernel<false, true, false>
-                        : (with_density ? backward_kernel<true, true, false> : backward_kernel<true, false, false>));
+  const BackwardKernel k = inner ? backward<true>(with_tf, with_density, multi) : backward<false>(with_tf, with_density, multi);
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -880,12 +892,12 @@ cudaError_t launch_backward(const TrainArgs& a, int grid, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_backward_empty(const TrainArgs& a, int sms, cudaStream_t s) {
+cudaError_t launch_backward_empty(const TrainArgs& a, int sms, bool inner, cudaStream_t s) {
   const size_t smem = (size_t)(a.n_tf + 4) * (sizeof(float4) + sizeof(float));
-  if (a.n_views > 1)
-    backward_empty_kernel<true><<<sms * kBackwardEmptyBlocks, 128, smem, s>>>(a);
-  else
-    backward_empty_kernel<false><<<sms * kBackwardEmptyBlocks, 128, smem, s>>>(a);
+  const bool multi = a.n_views > 1;
+  const BackwardKernel k = inner ? (multi ? backward_empty_kernel<true, true> : backward_empty_kernel<true, false>)
+                                 : (multi ? backward_empty_kernel<false, true> : backward_empty_kernel<false, false>);
+  k<<<sms * kBackwardEmptyBlocks, 128, smem, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -902,13 +914,13 @@ int backward_blocks_per_sm(int n_tf) {
   // the instance with the transfer-function gradient needs more shared memory
   const size_t smem = backward_smem(n_tf, true);
   if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(backward_kernel<true, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+      cudaFuncSetAttribute(backward_kernel<true, true, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
           cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
   int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, backward_kernel<true, true, true>, 128, smem) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, backward_kernel<true, true, true, true>, 128, smem) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }

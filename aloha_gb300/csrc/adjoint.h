@@ -83,14 +83,16 @@ struct TrainArgs {
 
 // One persistent training forward over the launch's views (a.tv, a.runs).
 // `many` selects the instance for launches of many chunks per resident warp
-// (kTrainForwardBlocksMany CTAs per SM instead of kTrainForwardBlocks).
-cudaError_t launch_forward_train(const TrainArgs& a, unsigned items, int max_grid, bool many, cudaStream_t s);
+// (kTrainForwardBlocksMany CTAs per SM instead of kTrainForwardBlocks); `inner`
+// (here and below): every brick and view of the launch is InnerCoords.
+cudaError_t launch_forward_train(const TrainArgs& a, unsigned items, int max_grid, bool many, bool inner,
+                                 cudaStream_t s);
 int forward_train_blocks_per_sm(int n_tf, bool many);
 // One persistent backward over the launch's views' items (a.tv, a.item_base).
-cudaError_t launch_backward(const TrainArgs& a, int grid, cudaStream_t s);
+cudaError_t launch_backward(const TrainArgs& a, int grid, bool inner, cudaStream_t s);
 // The all-empty segments of the same views (a.empty_base): the gradient of
 // the transfer function's alpha entries (a.dtf).  `sms` CTA groups.
-cudaError_t launch_backward_empty(const TrainArgs& a, int sms, cudaStream_t s);
+cudaError_t launch_backward_empty(const TrainArgs& a, int sms, bool inner, cudaStream_t s);
 // out[v] += quads[v].x + quads[v-1].y + quads[v-2].z along x, for a grid of
 // dims; every quad of the grid is zero afterwards.
 cudaError_t launch_fold_quads(float4* quads, float* out, const int dims[3], cudaStream_t s);

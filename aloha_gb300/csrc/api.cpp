@@ -112,8 +112,11 @@ struct aloha_ctx {
   std::vector<Box> boxes;
   std::vector<DevBrick> dev_bricks;
   std::vector<char> brick_present;
+  std::vector<char> brick_inner_box;  // the box part of DevBrick::inner
   std::vector<size_t> brick_offset;  // quad offset of each padded brick in `voxels`
   DeviceBuffer voxels, bricks_dev, staging_in;
+  DeviceBuffer scene_inner;  // int: every brick is InnerCoords
+  int scene_inner_host = 0;
   float bounds_lo[3] = {0, 0, 0}, bounds_hi[3] = {0, 0, 0};
   // transfer function
   DeviceBuffer tf;
@@ -277,6 +280,33 @@ std::vector<int> rank_screen_rects(const aloha_ctx* c, const ViewState& v) {
   return rects;
 }
 
+// DevView::inner: the eye near enough, and every pixel's direction of a proper
+// length.  The pixels' unnormalised directions lie on the plane through dir_00
+// spanned by dir_du and dir_dv; its distance from the origin bounds their
+// lengths from below, against the magnitude of the sums they are rounded in.
+bool view_inner(const ViewState& v) {
+  for (int a = 0; a < 3; ++a)
+    if (!(std::fabs(v.org[a]) <= kInnerEye)) return false;
+  const double* d[3];
+  double m[3][3];
+  for (int a = 0; a < 3; ++a) {
+    m[0][a] = v.dir_00[a];
+    m[1][a] = (double)v.dir_du[a] * v.width;
+    m[2][a] = (double)v.dir_dv[a] * v.height;
+  }
+  for (int k = 0; k < 3; ++k) d[k] = m[k];
+  double cross[3], area2 = 0.0, dot = 0.0, sum = 0.0;
+  for (int a = 0; a < 3; ++a) {
+    const int b = (a + 1) % 3, e = (a + 2) % 3;
+    cross[a] = d[1][b] * d[2][e] - d[1][e] * d[2][b];
+    area2 += cross[a] * cross[a];
+    dot += cross[a] * d[0][a];
+    for (int k = 0; k < 3; ++k) sum += std::fabs(d[k][a]);
+  }
+  if (!(area2 > 0.0) || !(sum > 1e-9 && sum < 1e9)) return false;
+  return std::fabs(dot) / std::sqrt(area2) >= 1e-3 * sum;
+}
+
 // Upload dirty view state (camera, size, schedule) for `view` on `s`.
 int prepare_view(aloha_ctx* c, int view, cudaStream_t s) {
   if (c->descs.empty()) return c->fail(ALOHA_ERR_NOT_READY, "no bricks uploaded");
@@ -346,6 +376,7 @@ int prepare_view(aloha_ctx* c, int view, cudaStream_t s) {
     }
     dv.max_depth = std::sqrt(s2) + std::sqrt(s1);
   }
+  dv.inner = view_inner(v);
   dv.n_ranks = c->n_ranks;
   dv.sched = view * stride;
   dv.rects = view * stride + 2 * c->n_ranks + 1 + nb;
@@ -569,6 +600,11 @@ int launch_single(aloha_ctx* c, const FrameArgs& f, int view, cudaStream_t s) {
   return ALOHA_OK;
 }
 
+// FrameArgs::inner.
+bool params_inner(const aloha_render_params& p) {
+  return p.dt <= kInnerStep && (p.jitter_mode != ALOHA_JITTER_CONST || std::fabs(p.jitter_value) <= kInnerJitter);
+}
+
 FrameArgs frame_args(aloha_ctx* c) {
   const aloha_render_params& p = c->params;
   FrameArgs a{};
@@ -590,6 +626,8 @@ FrameArgs frame_args(aloha_ctx* c) {
   a.composite_mode = p.composite_mode;
   a.island_id = p.island_id;
   a.num_islands = p.num_islands;
+  a.inner = params_inner(p);
+  a.scene_inner = static_cast<const int*>(c->scene_inner.ptr);
   a.counter = static_cast<unsigned long long*>(c->counter.ptr);
   return a;
 }
@@ -742,7 +780,8 @@ int aloha_create(int device, aloha_ctx** out) {
   aloha_default_render_params(&c->params);
   if (c->views_dev.ensure(sizeof(DevView) * kMaxViews) != cudaSuccess ||
       c->counter.ensure(sizeof(unsigned long long)) != cudaSuccess || c->flag.ensure(sizeof(int)) != cudaSuccess ||
-      c->work.ensure(sizeof(unsigned int)) != cudaSuccess) {
+      c->work.ensure(sizeof(unsigned int)) != cudaSuccess || c->scene_inner.ensure(sizeof(int)) != cudaSuccess ||
+      cudaMemset(c->scene_inner.ptr, 0, sizeof(int)) != cudaSuccess) {
     delete c;
     return ALOHA_ERR_OUT_OF_MEMORY;
   }
@@ -758,7 +797,7 @@ int aloha_destroy(aloha_ctx* c) {
     if (v.accum) cudaFree(v.accum);
     v.train.release();
   }
-  for (DeviceBuffer* b : {&c->voxels, &c->bricks_dev, &c->staging_in, &c->tf, &c->views_dev, &c->sched_dev,
+  for (DeviceBuffer* b : {&c->voxels, &c->bricks_dev, &c->scene_inner, &c->staging_in, &c->tf, &c->views_dev, &c->sched_dev,
                           &c->counter, &c->flag, &c->staging_out, &c->mc_ranges, &c->mc_empty, &c->tf_prefix,
                           &c->work, &c->grad4, &c->split_images, &c->split_masks, &c->split_items,
                           &c->split_done, &c->chunk_order})
@@ -781,6 +820,15 @@ int aloha_set_render_params(aloha_ctx* c, const aloha_render_params* p) {
 }
 
 // Uploads one brick's voxels into its padded slot.
+static int upload_scene_inner(aloha_ctx* c) {
+  int all = 1;
+  for (const DevBrick& b : c->dev_bricks) all &= b.inner;
+  if (all == c->scene_inner_host) return ALOHA_OK;
+  CUDA_TRY(c, cudaMemcpy(c->scene_inner.ptr, &all, sizeof all, cudaMemcpyHostToDevice));
+  c->scene_inner_host = all;
+  return ALOHA_OK;
+}
+
 static int upload_brick(aloha_ctx* c, int b, const float* src) {
   const aloha_brick_desc& d = c->descs[b];
   const int nx = d.voxel_hi[0] - d.voxel_lo[0], ny = d.voxel_hi[1] - d.voxel_lo[1], nz = d.voxel_hi[2] - d.voxel_lo[2];
@@ -791,15 +839,17 @@ static int upload_brick(aloha_ctx* c, int b, const float* src) {
     CUDA_TRY(c, cudaMemcpy(c->staging_in.ptr, src, raw * sizeof(float), cudaMemcpyHostToDevice));
     dsrc = static_cast<const float*>(c->staging_in.ptr);
   }
-  const DevBrick& db = c->dev_bricks[b];
+  DevBrick& db = c->dev_bricks[b];
   float4* alloc = static_cast<float4*>(c->voxels.ptr) + c->brick_offset[b];
   CUDA_TRY(c, cudaMemset(c->flag.ptr, 0, sizeof(int)));
   CUDA_TRY(c, launch_pad_brick(dsrc, nx, ny, nz, alloc, db.sy, db.sz, static_cast<int*>(c->flag.ptr), 0));
   CUDA_TRY(c, launch_macrocell_range(db, static_cast<float2*>(c->mc_ranges.ptr) + c->mc_offset[b], 0));
   c->empty_dirty = true;
-  int bad = 0;  // this copy also waits for the two kernels above
-  CUDA_TRY(c, cudaMemcpy(&bad, c->flag.ptr, sizeof(int), cudaMemcpyDeviceToHost));
-  if (bad) return c->fail(ALOHA_ERR_INVALID_ARGUMENT, "brick %d holds a non-finite voxel", b);
+  int flags = 0;  // this copy also waits for the two kernels above
+  CUDA_TRY(c, cudaMemcpy(&flags, c->flag.ptr, sizeof(int), cudaMemcpyDeviceToHost));
+  if (flags & kVoxelNonfinite) return c->fail(ALOHA_ERR_INVALID_ARGUMENT, "brick %d holds a non-finite voxel", b);
+  const int inner = c->brick_inner_box[b] && !(flags & kVoxelWide);
+  db.inner = inner;
   c->brick_present[b] = 1;
   invalidate_training(c);
   return ALOHA_OK;
@@ -812,6 +862,7 @@ int aloha_set_bricks(aloha_ctx* c, const aloha_brick_desc* descs, const float* c
   size_t total = 0;
   std::vector<size_t> offs(n);
   std::vector<DevBrick> db(n);
+  std::vector<char> inner_box(n, 1);
   for (int b = 0; b < n; ++b) {
     const aloha_brick_desc& d = descs[b];
     if (!voxels[b]) return c->fail(ALOHA_ERR_NULL_POINTER, "voxels[%d] is null", b);
@@ -838,7 +889,12 @@ int aloha_set_bricks(aloha_ctx* c, const aloha_brick_desc* descs, const float* c
       db[b].lo[a] = (float)d.voxel_lo[a];
       db[b].space_lo[a] = d.space_lo[a];
       db[b].space_hi[a] = d.space_hi[a];
+      if (!(d.space_lo[a] >= (float)d.voxel_lo[a] && d.space_hi[a] <= (float)d.voxel_hi[a] &&
+            std::fabs(d.space_lo[a]) <= kInnerSpace && std::fabs(d.space_hi[a]) <= kInnerSpace &&
+            std::abs((double)d.voxel_lo[a]) <= kInnerSpace))
+        inner_box[b] = 0;
     }
+    db[b].inner = inner_box[b];  // unless its values are too large (upload_brick)
   }
   size_t free_b = 0, total_b = 0;
   CUDA_TRY(c, cudaMemGetInfo(&free_b, &total_b));
@@ -865,6 +921,7 @@ int aloha_set_bricks(aloha_ctx* c, const aloha_brick_desc* descs, const float* c
   c->dev_bricks = db;
   c->brick_offset = offs;
   c->brick_present.assign(n, 0);
+  c->brick_inner_box = inner_box;
   c->boxes.resize(n);
   for (int a = 0; a < 3; ++a) {
     c->bounds_lo[a] = 1e30f;
@@ -886,6 +943,8 @@ int aloha_set_bricks(aloha_ctx* c, const aloha_brick_desc* descs, const float* c
       return rc;
     }
   }
+  int rc = upload_scene_inner(c);
+  if (rc) return rc;
   c->staging_in.release();
   c->sched_stride = 0;
   return set_partition(c, n, true);
@@ -896,7 +955,8 @@ int aloha_update_brick(aloha_ctx* c, int brick, const float* voxels) {
   if (brick < 0 || brick >= (int)c->descs.size()) return c->fail(ALOHA_ERR_OUT_OF_RANGE, "brick %d", brick);
   CUDA_TRY(c, cudaSetDevice(c->device));
   CUDA_TRY(c, cudaDeviceSynchronize());
-  return upload_brick(c, brick, voxels);
+  const int rc = upload_brick(c, brick, voxels);
+  return rc ? rc : upload_scene_inner(c);
 }
 
 int aloha_drop_brick(aloha_ctx* c, int brick) {
@@ -1247,6 +1307,18 @@ TrainArgs train_args(aloha_ctx* c) {
   return a;
 }
 
+// True when every brick and view of a launch of the differentiable form is
+// InnerCoords (its launches copy host tables, so none can be recorded into a
+// graph and replayed on another scene).
+bool train_inner(const aloha_ctx* c, int n_views, const int* view_ids) {
+  if (!params_inner(c->params)) return false;
+  for (const DevBrick& b : c->dev_bricks)
+    if (!b.inner) return false;
+  for (int i = 0; i < n_views; ++i)
+    if (!view_inner(c->views[view_ids[i]])) return false;
+  return true;
+}
+
 TrainView train_view(const TrainState& t, int view) {
   TrainView tv{};
   tv.ckpt = t.ckpt;
@@ -1387,12 +1459,13 @@ int forward_views(aloha_ctx* c, int n_views, const int* view_ids, float* const* 
   CUDA_TRY(c, cudaMemsetAsync(c->counter.ptr, 0, sizeof(unsigned long long), s));
   // few chunks per resident warp: the launch ends on its longest rays (fewer,
   // faster warps); many: throughput-bound (more warps)
+  const bool inner = train_inner(c, n_views, view_ids);
   const int few_per_sm = forward_train_blocks_per_sm(c->n_tf, false);
   if (few_per_sm <= 0) return c->fail(ALOHA_ERR_CUDA, "forward occupancy query failed");
   const bool many = items >= (unsigned long long)kTrainManyChunksPerWarp * few_per_sm * c->num_sms * 4;
   const int per_sm = many ? forward_train_blocks_per_sm(c->n_tf, true) : few_per_sm;
   if (per_sm <= 0) return c->fail(ALOHA_ERR_CUDA, "forward occupancy query failed");
-  CUDA_TRY(c, launch_forward_train(a, (unsigned)items, per_sm * c->num_sms, many, s));
+  CUDA_TRY(c, launch_forward_train(a, (unsigned)items, per_sm * c->num_sms, many, inner, s));
   c->samples_valid = true;
   bool any_host = false;
   for (int i = 0; i < n_views; ++i) {
@@ -1510,6 +1583,7 @@ int backward_views(aloha_ctx* c, int n_views, const int* view_ids, const float* 
   if (h_grid) CUDA_TRY(c, cudaMemcpyAsync(grid_out, dl_ddensity, g_bytes, cudaMemcpyHostToDevice, s));
   if (with_density)
     CUDA_TRY(c, cudaMemcpyAsync(st + off_org, origin.data(), origin.size() * sizeof(int4), cudaMemcpyHostToDevice, s));
+  const bool inner = train_inner(c, n_views, view_ids);
   const int per_sm = backward_blocks_per_sm(c->n_tf);
   if (per_sm <= 0) return c->fail(ALOHA_ERR_CUDA, "backward occupancy query failed");
   CUDA_TRY(c, cudaMemsetAsync(c->counter.ptr, 0, sizeof(unsigned long long), s));
@@ -1561,14 +1635,14 @@ int backward_views(aloha_ctx* c, int n_views, const int* view_ids, const float* 
         a.one = tvs[i];
         a.one_items = base[i + 1] - base[i];
         a.one_empty = empty_base[i + 1] - empty_base[i];
-        CUDA_TRY(c, launch_backward(a, c->num_sms * per_sm, s));
-        if (dtf && a.one_empty) CUDA_TRY(c, launch_backward_empty(a, c->num_sms, s));
+        CUDA_TRY(c, launch_backward(a, c->num_sms * per_sm, inner, s));
+        if (dtf && a.one_empty) CUDA_TRY(c, launch_backward_empty(a, c->num_sms, inner, s));
       }
     } else {
       a.n_views = (int)tvs.size();
       a.item_base = reinterpret_cast<const unsigned*>(dev[2]);
-      CUDA_TRY(c, launch_backward(a, c->num_sms * per_sm, s));
-      if (dtf && empty_base.back()) CUDA_TRY(c, launch_backward_empty(a, c->num_sms, s));
+      CUDA_TRY(c, launch_backward(a, c->num_sms * per_sm, inner, s));
+      if (dtf && empty_base.back()) CUDA_TRY(c, launch_backward_empty(a, c->num_sms, inner, s));
     }
   }
   if (with_density) {

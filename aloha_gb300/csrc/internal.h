@@ -11,9 +11,10 @@ namespace aloha {
 // Padded brick storage: every brick is stored with an apron of kApron voxels
 // on each side, filled with the clamped edge values (cudaAddressModeClamp of
 // waikikiRenderer.cpp:753-755), so the march loop needs no per-tap clamps.
-// Each stored element is a yz-quad: the float4 (V(x,y,z), V(x,y+1,z),
-// V(x,y,z+1), V(x,y+1,z+1)) (indices clamped), so one 16-byte load fetches a
-// voxel's 2x2 (y, z) neighbourhood and the stencil's core comes from three
+// Each stored element is a yz-quad: the float4 (V(x,y,z), V(x,y,z+1),
+// V(x,y+1,z), V(x,y+1,z+1)) (indices clamped), so one 16-byte load fetches a
+// voxel's 2x2 (y, z) neighbourhood, its halves are (z, z+1) pairs that packed
+// fp32x2 instructions interpolate together, and the stencil's core comes from three
 // neighbouring elements of one row (x-quads, V(x..x+3), took the same bytes
 // from four rows and hit L1 less often).  Quads cut the loads per sample from
 // 20 to 7 at four times the HBM footprint.
@@ -44,7 +45,24 @@ constexpr int kMaxTF = 2048;  // (n + 4) float4 entries stay under 48 KB of shar
 constexpr int kMacroShift = 3;
 constexpr int kMacro = 1 << kMacroShift;
 
-// One brick as the kernels see it (72 bytes).
+// InnerCoords.  When a sample's voxel coordinates provably lie in [-1/4, n +
+// 1/4] along every axis of its brick, the stencil's indices need no clamps (the
+// apron holds every voxel they reach) and floors can be taken with an addition
+// instead of a conversion (|u| < 2^22).  That is so when
+//  - the brick's space range lies inside its voxel range, within kInnerSpace of
+//    the origin, and its values within +-kInnerValue (times at most kMaxTF
+//    entries: below 2^21 for the lookup's floor): DevBrick::inner;
+//  - the eye lies within kInnerEye of the origin and every pixel has a proper
+//    direction: DevView::inner;
+//  - the step is at most kInnerStep and a constant jitter at most kInnerJitter
+//    steps: FrameArgs::inner.
+// Ray parameters then stay below 2^17, and their rounding, the lattice's and
+// the position's add up to less than 1/16 voxel.  Anything else takes the
+// clamped form, which gives the same bits.
+constexpr float kInnerSpace = 16384.0f, kInnerEye = 32768.0f, kInnerValue = 1024.0f, kInnerStep = 1024.0f,
+                kInnerJitter = 16.0f;
+
+// One brick as the kernels see it (80 bytes).
 struct DevBrick {
   const float4* base;    // yz-quad of voxel (0,0,0) of the voxel range inside the padded array
   const uint8_t* empty;  // [mz][my][mx] 1 = every sample there has alpha 0 (null: no skipping)
@@ -52,6 +70,7 @@ struct DevBrick {
   int n[3];              // voxel range size
   float lo[3];           // voxelRange.lower (voxel-unit origin of the brick)
   float space_lo[3], space_hi[3];
+  int inner;             // InnerCoords
 };
 
 // Per-view state read by the kernels.
@@ -65,7 +84,7 @@ struct DevView {
   int pixel_offset;   // offset of the view's first pixel in batched outputs
   int rects;          // offset of the ranks' screen rectangles in the schedule buffer:
                       // per rank [cx0, cy0, cx1, cy1] in 8x4 chunks, inclusive
-  int pad;
+  int inner;          // InnerCoords
 };
 
 // Everything one render launch needs, passed by value.
@@ -81,6 +100,8 @@ struct FrameArgs {
   int crosshair, spp, accum_id, accumulate, heat_map;
   float heat_map_scale;
   int composite_mode, island_id, num_islands;
+  int inner;                    // InnerCoords
+  const int* scene_inner;       // 1 when every brick is InnerCoords
   // outputs
   uint32_t* fb;                 // [H*W] (single view) RGBA8
   float4* rank_images;          // [n_ranks][H*W] or null
@@ -174,9 +195,11 @@ cudaError_t launch_composite_f32(const float4* imgs, const int* order, int n_ran
                                  cudaStream_t s);
 cudaError_t launch_composite_u8(const uint32_t* imgs, const int* order, int n_ranks, int npx, uint32_t* fb,
                                 cudaStream_t s);
-// Fills a brick's padded array (pitches px, sz in quads).
-cudaError_t launch_pad_brick(const float* src, int nx, int ny, int nz, float4* dst_alloc, int px, int sz,
-                             int* nonfinite_flag, cudaStream_t s);
+// Fills a brick's padded array (pitches px, sz in quads).  Sets flag bits:
+// kVoxelNonfinite, kVoxelWide (a value beyond +-kInnerValue).
+constexpr int kVoxelNonfinite = 1, kVoxelWide = 2;
+cudaError_t launch_pad_brick(const float* src, int nx, int ny, int nz, float4* dst_alloc, int px, int sz, int* flags,
+                             cudaStream_t s);
 // Persistent render launch; `batch` selects the instance tuned for batches.
 constexpr int kSingleRenderBlocks = 5, kBatchRenderBlocks = 7;  // CTAs per SM
 // CTAs per SM of the differentiable form's forward (checkpointed march): a

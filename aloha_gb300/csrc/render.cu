@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(kRenderThreads, MINB) render_warps_kernel(Batc
         // the group's lanes share x and y, so they take this branch together
         if (x < v.width && y < v.height) {
           const uint32_t ns =
-              render_pixel<Loads, LG>(b.f, v, tf_s, x, y, fb, (size_t)x + (size_t)v.width * y, loads, g);
+              render_pixel<false, Loads, LG>(b.f, v, tf_s, x, y, fb, (size_t)x + (size_t)v.width * y, loads, g);
           if (gl == 0) n += ns;
         }
         continue;
@@ -89,12 +89,23 @@ __global__ void __launch_bounds__(kRenderThreads, MINB) render_warps_kernel(Batc
       continue;
     }
     const int x0 = ccx * CW, y0 = ccy * CH;
+    // The march with unclamped coordinates (InnerCoords) or the clamped one,
+    // decided per chunk from device memory, so that a recorded launch follows
+    // later scenes and cameras.  Both are inlined: decided per sample, the
+    // branch cost what it saved; the clamped march as an out-of-line call made
+    // the 72-register instances spill around it (uneven batch 10.8 ms, against
+    // 9.7 ms this way and 9.6 ms without a clamped form).
+    const bool inner = Loads::kInner && b.f.inner && v.inner && *b.f.scene_inner;
 #pragma unroll 1
     for (int sub = 0; sub < (CW / 8) * (CH / 4); ++sub) {
       const int x = x0 + (sub % (CW / 8)) * 8 + tile_x(lane);
       const int y = y0 + (sub / (CW / 8)) * 4 + tile_y(lane);
-      if (x < v.width && y < v.height)
-        n += render_pixel(b.f, v, tf_s, x, y, fb, (size_t)x + (size_t)v.width * y, loads);
+      if (x < v.width && y < v.height) {
+        if (inner)
+          n += render_pixel<Loads::kInner>(b.f, v, tf_s, x, y, fb, (size_t)x + (size_t)v.width * y, loads);
+        else
+          n += render_pixel<false>(b.f, v, tf_s, x, y, fb, (size_t)x + (size_t)v.width * y, loads);
+      }
     }
   }
   loads.finish();
@@ -272,6 +283,7 @@ __global__ void __launch_bounds__(kRenderThreads, MINB) render_split_kernel(Spli
   const int cxn = (W + 7) / 8, cyn = (H + 3) / 4;
   const uint32_t n_items = *s.n_items;
   float4* __restrict__ planes = s.f.rank_images;
+  const bool inner = s.f.inner && s.f.views[s.view].inner && *s.f.scene_inner;
   uint32_t n = 0;
   for (;;) {
     uint32_t item = 0;
@@ -298,13 +310,16 @@ __global__ void __launch_bounds__(kRenderThreads, MINB) render_split_kernel(Spli
         if (plain_output_stage(s.f)) {
           // the output stage is the identity: only the plane store is left,
           // so nothing else it needs stays live across the march
-          if (in_island)
-            acc = march_rank(s.f, v, tf_s, generate_ray(v, x, y), rbricks, __ldg(rstart + r), __ldg(rstart + r + 1),
+          if (in_island && inner)
+            acc = march_rank<true>(s.f, v, tf_s, generate_ray(v, x, y), rbricks, __ldg(rstart + r), __ldg(rstart + r + 1),
+                                   pixel, z, ns, direct);
+          else if (in_island)
+            acc = march_rank<false>(s.f, v, tf_s, generate_ray(v, x, y), rbricks, __ldg(rstart + r), __ldg(rstart + r + 1),
                              pixel, z, ns, direct);
           planes[(size_t)r * npx + pixel] = acc;
         } else {
           if (in_island)
-            acc = march_rank(s.f, v, tf_s, generate_ray(v, x, y), rbricks, __ldg(rstart + r), __ldg(rstart + r + 1),
+            acc = march_rank<false>(s.f, v, tf_s, generate_ray(v, x, y), rbricks, __ldg(rstart + r), __ldg(rstart + r + 1),
                              pixel, z, ns, direct);
           rank_output(s.f, W, H, r, x, y, pixel, npx, acc, ns, z, planes, nullptr);
         }
@@ -362,15 +377,16 @@ __global__ void composite_u8_kernel(const uint32_t* __restrict__ imgs, const int
 }
 
 // Copies a brick (x fastest) into its padded yz-quad array: element (x,y,z)
-// holds V(x,y,z), V(x,y+1,z), V(x,y,z+1), V(x,y+1,z+1) with every index
+// holds V(x,y,z), V(x,y,z+1), V(x,y+1,z), V(x,y+1,z+1) with every index
 // clamped to the brick (the apron and the quads' far rows and slices repeat
-// edge values), and flags non-finite voxels.  CTAs take padded rows (y, z),
+// edge values), and flags non-finite voxels and values too large for
+// InnerCoords.  CTAs take padded rows (y, z),
 // their threads the row's elements, so the index arithmetic is one division
 // per row; a row reads four source rows, each coalesced along x.
 __global__ void pad_brick_kernel(const float* __restrict__ src, int nx, int ny, int nz, float4* __restrict__ dst,
-                                 int px, int sz, int* nonfinite) {
+                                 int px, int sz, int* flags) {
   const int py = ny + 2 * kApron, rows = py * (nz + 2 * kApron);
-  bool bad = false;
+  bool bad = false, wide = false;
   for (int r = blockIdx.x; r < rows; r += gridDim.x) {
     const int y = r % py, z = r / py;
     const int y0 = min(max(y - kApron, 0), ny - 1), y1 = min(max(y + 1 - kApron, 0), ny - 1);
@@ -382,12 +398,14 @@ __global__ void pad_brick_kernel(const float* __restrict__ src, int nx, int ny, 
     float4* __restrict__ out = dst + ((size_t)z * sz + (size_t)y * px);
     for (int x = threadIdx.x; x < px; x += blockDim.x) {
       const int sx = min(max(x - kApron, 0), nx - 1);
-      const float4 v = make_float4(__ldg(r00 + sx), __ldg(r10 + sx), __ldg(r01 + sx), __ldg(r11 + sx));
+      const float4 v = make_float4(__ldg(r00 + sx), __ldg(r01 + sx), __ldg(r10 + sx), __ldg(r11 + sx));
+      const float top = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
+      wide |= top > kInnerValue;
       bad |= !isfinite(v.x) || !isfinite(v.y) || !isfinite(v.z) || !isfinite(v.w);
       out[x] = v;
     }
   }
-  if (bad) atomicOr(nonfinite, 1);
+  if (bad || wide) atomicOr(flags, (bad ? kVoxelNonfinite : 0) | (wide ? kVoxelWide : 0));
 }
 
 // Value range each macrocell's samples can read: a sample whose value-tap
@@ -415,11 +433,11 @@ __global__ void macrocell_range_kernel(const float4* __restrict__ base, int sy, 
         const float4 q = __ldg(row + x);
         lo = fminf(lo, q.x);
         hi = fmaxf(hi, q.x);
-        if (y_in) {
+        if (z_in) {
           lo = fminf(lo, q.y);
           hi = fmaxf(hi, q.y);
         }
-        if (z_in) {
+        if (y_in) {
           lo = fminf(lo, q.z);
           hi = fmaxf(hi, q.z);
         }
@@ -579,11 +597,11 @@ cudaError_t launch_composite_u8(const uint32_t* imgs, const int* order, int n_ra
   return cudaGetLastError();
 }
 
-cudaError_t launch_pad_brick(const float* src, int nx, int ny, int nz, float4* dst, int px, int sz, int* nonfinite,
+cudaError_t launch_pad_brick(const float* src, int nx, int ny, int nz, float4* dst, int px, int sz, int* flags,
                              cudaStream_t s) {
   const int rows = (ny + 2 * kApron) * (nz + 2 * kApron);
   const int g = rows < 152 * 32 ? rows : 152 * 32;  // CTAs of 128 threads take rows
-  pad_brick_kernel<<<g < 1 ? 1 : g, 128, 0, s>>>(src, nx, ny, nz, dst, px, sz, nonfinite);
+  pad_brick_kernel<<<g < 1 ? 1 : g, 128, 0, s>>>(src, nx, ny, nz, dst, px, sz, flags);
   return cudaGetLastError();
 }
 
