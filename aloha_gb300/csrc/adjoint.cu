@@ -105,18 +105,11 @@ __device__ __forceinline__ uint32_t walk_samples(const TrainArgs& a, const DevVi
       const float ux = fmaf(t, ray.d[0], ray.o[0]) - b.lo[0];
       const float uy = fmaf(t, ray.d[1], ray.o[1]) - b.lo[1];
       const float uz = fmaf(t, ray.d[2], ray.o[2]) - b.lo[2];
-      if (SKIP && b.empty && !(t < t_cell)) {
-        const int mx = min(max(__float2int_rd(ux), 0), b.n[0] - 1) >> kMacroShift;
-        const int my = min(max(__float2int_rd(uy), 0), b.n[1] - 1) >> kMacroShift;
-        const int mz = min(max(__float2int_rd(uz), 0), b.n[2] - 1) >> kMacroShift;
-        const float bnd[3] = {(float)(mx << kMacroShift), (float)(my << kMacroShift), (float)(mz << kMacroShift)};
-        float tb = t1;
-#pragma unroll
-        for (int ax = 0; ax < 3; ++ax) {
-          const float face = ray.d[ax] > 0.f ? bnd[ax] + (float)kMacro - eps : bnd[ax] + eps;
-          tb = fminf(tb, (face - (ray.o[ax] - b.lo[ax])) * inv_d[ax]);
-        }
-        if (!__ldg(b.empty + (mz * mny + my) * mnx + mx)) {
+      if (SKIP && !(t < t_cell)) {
+        const CellBox cell = cell_box(b.cells, mnx, mny, b.n[0], b.n[1], b.n[2], ux, uy, uz, ray.d, ray.o[0] - b.lo[0],
+                                      ray.o[1] - b.lo[1], ray.o[2] - b.lo[2], inv_d[0], inv_d[1], inv_d[2], eps, t1);
+        const float tb = cell.exit;
+        if (!cell.empty) {
           t_cell = tb;
         } else if (exact) {
           ++n;

@@ -123,7 +123,7 @@ struct aloha_ctx {
   int n_tf = 0;
   // empty-space macrocells: value range per macrocell (per brick) and the
   // per-transfer-function empty mask, refreshed before the next render
-  DeviceBuffer mc_ranges, mc_empty, tf_prefix;
+  DeviceBuffer mc_ranges, mc_codes, tf_prefix;
   std::vector<size_t> mc_offset;
   size_t mc_total = 0;
   bool empty_dirty = true;
@@ -318,9 +318,13 @@ int prepare_view(aloha_ctx* c, int view, cudaStream_t s) {
   for (size_t b = 0; b < c->brick_present.size(); ++b)
     if (!c->brick_present[b]) return c->fail(ALOHA_ERR_MISSING_BRICK, "brick %zu has no data (dropped)", b);
   if (c->empty_dirty) {
-    CUDA_TRY(c, launch_macrocell_empty(static_cast<const float2*>(c->mc_ranges.ptr), (int)c->mc_total,
-                                       static_cast<const int*>(c->tf_prefix.ptr), c->n_tf,
-                                       static_cast<uint8_t*>(c->mc_empty.ptr), s));
+    int most = 0;
+    for (const DevBrick& b : c->dev_bricks) most = std::max(most, macrocells(b));
+    uint8_t* codes = static_cast<uint8_t*>(c->mc_codes.ptr);
+    CUDA_TRY(c, launch_macrocell_codes(static_cast<const DevBrick*>(c->bricks_dev.ptr), (int)c->dev_bricks.size(), most,
+                                       static_cast<const float2*>(c->mc_ranges.ptr),
+                                       static_cast<const int*>(c->tf_prefix.ptr), c->n_tf, codes, codes + c->mc_total,
+                                       s));
     c->empty_dirty = false;
   }
   const int nb = (int)c->descs.size();
@@ -798,7 +802,7 @@ int aloha_destroy(aloha_ctx* c) {
     v.train.release();
   }
   for (DeviceBuffer* b : {&c->voxels, &c->bricks_dev, &c->scene_inner, &c->staging_in, &c->tf, &c->views_dev, &c->sched_dev,
-                          &c->counter, &c->flag, &c->staging_out, &c->mc_ranges, &c->mc_empty, &c->tf_prefix,
+                          &c->counter, &c->flag, &c->staging_out, &c->mc_ranges, &c->mc_codes, &c->tf_prefix,
                           &c->work, &c->grad4, &c->split_images, &c->split_masks, &c->split_items,
                           &c->split_done, &c->chunk_order})
     b->release();
@@ -842,10 +846,10 @@ static int upload_brick(aloha_ctx* c, int b, const float* src) {
   DevBrick& db = c->dev_bricks[b];
   float4* alloc = static_cast<float4*>(c->voxels.ptr) + c->brick_offset[b];
   CUDA_TRY(c, cudaMemset(c->flag.ptr, 0, sizeof(int)));
-  CUDA_TRY(c, launch_pad_brick(dsrc, nx, ny, nz, alloc, db.sy, db.sz, static_cast<int*>(c->flag.ptr), 0));
-  CUDA_TRY(c, launch_macrocell_range(db, static_cast<float2*>(c->mc_ranges.ptr) + c->mc_offset[b], 0));
+  CUDA_TRY(c, launch_fill_brick(db, dsrc, alloc, static_cast<float2*>(c->mc_ranges.ptr) + c->mc_offset[b],
+                                static_cast<int*>(c->flag.ptr), 0));
   c->empty_dirty = true;
-  int flags = 0;  // this copy also waits for the two kernels above
+  int flags = 0;  // this copy also waits for the kernel above
   CUDA_TRY(c, cudaMemcpy(&flags, c->flag.ptr, sizeof(int), cudaMemcpyDeviceToHost));
   if (flags & kVoxelNonfinite) return c->fail(ALOHA_ERR_INVALID_ARGUMENT, "brick %d holds a non-finite voxel", b);
   const int inner = c->brick_inner_box[b] && !(flags & kVoxelWide);
@@ -912,8 +916,8 @@ int aloha_set_bricks(aloha_ctx* c, const aloha_brick_desc* descs, const float* c
     mc_total += (size_t)macrocells(db[b]);
   }
   CUDA_TRY(c, c->mc_ranges.ensure(mc_total * sizeof(float2)));
-  CUDA_TRY(c, c->mc_empty.ensure(mc_total));
-  for (int b = 0; b < n; ++b) db[b].empty = static_cast<const uint8_t*>(c->mc_empty.ptr) + mc_off[b];
+  CUDA_TRY(c, c->mc_codes.ensure(2 * mc_total));  // the codes, then scratch
+  for (int b = 0; b < n; ++b) db[b].cells = static_cast<const uint8_t*>(c->mc_codes.ptr) + mc_off[b];
   c->mc_offset = mc_off;
   c->mc_total = mc_total;
   c->empty_dirty = true;

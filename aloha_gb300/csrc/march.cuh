@@ -435,6 +435,31 @@ __device__ __forceinline__ void composite_step(float4& color, const float4 c, fl
   color.w = fmaf(oma, c.w, color.w);
 }
 
+// A macrocell lookup at voxel coordinate u: whether the cell is empty, and the
+// ray parameter (at most t1) up to which every sample stays in the box of cells
+// of its kind around it, shrunk by eps.
+struct CellBox {
+  bool empty;
+  float exit;
+};
+__device__ __forceinline__ CellBox cell_box(const uint8_t* __restrict__ cells, int mnx, int mny, int nx, int ny, int nz,
+                                            float ux, float uy, float uz, const float d[3], float offx, float offy,
+                                            float offz, float idx, float idy, float idz, float eps, float t1) {
+  const int mx = min(max(__float2int_rd(ux), 0), nx - 1) >> kMacroShift;
+  const int my = min(max(__float2int_rd(uy), 0), ny - 1) >> kMacroShift;
+  const int mz = min(max(__float2int_rd(uz), 0), nz - 1) >> kMacroShift;
+  const int code = __ldg(cells + (mz * mny + my) * mnx + mx);
+  const int reach = code & (kCellFull - 1);
+  auto face = [&](int m, float dir) {
+    return dir > 0.f ? (float)((m + reach) << kMacroShift) - eps : (float)((m + 1 - reach) << kMacroShift) + eps;
+  };
+  CellBox c;
+  c.empty = code < kCellFull;
+  c.exit = fminf(fminf(fminf((face(mx, d[0]) - offx) * idx, (face(my, d[1]) - offy) * idy),
+                       (face(mz, d[2]) - offz) * idz), t1);
+  return c;
+}
+
 // A march hook sees every sample, full or skipped, before it is taken: its
 // t, the samples already taken in the brick and the colour so far.  The
 // render passes NoHook; the differentiable forward stores checkpoints.  An
@@ -457,7 +482,7 @@ __device__ __forceinline__ uint32_t march_brick(const DevBrick& b, const float4*
   const float lox = b.lo[0], loy = b.lo[1], loz = b.lo[2];
   const float nf = (float)n_tf;
   const uint32_t cap = march_cap(t0, t1, dt);
-  const uint8_t* __restrict__ empty = b.empty;
+  const uint8_t* __restrict__ cells = b.cells;
   const int mnx = (nx + kMacro - 1) >> kMacroShift, mny = (ny + kMacro - 1) >> kMacroShift;
   // Brick-local ray origin, inverse direction and the rounding margin (voxel
   // units) that makes the macrocell exit bound below conservative: u = o + t d
@@ -471,9 +496,9 @@ __device__ __forceinline__ uint32_t march_brick(const DevBrick& b, const float4*
   float t = first_sample_t(t0, dt, ils);
   const bool exact = exact_steps(t, t1, dt);
   const float inv_dt = 1.0f / dt;
-  // Samples before t_cell lie in the last macrocell found non-empty, so they
+  // Samples before t_cell lie in the last box of full macrocells, so they
   // need no lookup.  Only the skip below depends on the lookup (a full sample
-  // in an empty macrocell leaves the colour unchanged as well), so the bound
+  // in an empty macrocell leaves the colour unchanged as well), so that bound
   // only has to be right for speed.
   float t_cell = t0;
   loads.begin_brick();
@@ -485,17 +510,11 @@ __device__ __forceinline__ uint32_t march_brick(const DevBrick& b, const float4*
       const float ux = fmaf(t, r.d[0], r.o[0]) - lox;
       const float uy = fmaf(t, r.d[1], r.o[1]) - loy;
       const float uz = fmaf(t, r.d[2], r.o[2]) - loz;
-      if (empty && !(t < t_cell)) {
-        const int mx = min(max(__float2int_rd(ux), 0), nx - 1) >> kMacroShift;
-        const int my = min(max(__float2int_rd(uy), 0), ny - 1) >> kMacroShift;
-        const int mz = min(max(__float2int_rd(uz), 0), nz - 1) >> kMacroShift;
-        const float bx = (float)(mx << kMacroShift), by = (float)(my << kMacroShift),
-                    bz = (float)(mz << kMacroShift);
-        const float ex = ((r.d[0] > 0.f ? bx + (float)kMacro - eps : bx + eps) - offx) * idx_;
-        const float ey = ((r.d[1] > 0.f ? by + (float)kMacro - eps : by + eps) - offy) * idy;
-        const float ez = ((r.d[2] > 0.f ? bz + (float)kMacro - eps : bz + eps) - offz) * idz;
-        const float tb = fminf(fminf(fminf(ex, ey), ez), t1);
-        if (__ldg(empty + (mz * mny + my) * mnx + mx)) {
+      if (!(t < t_cell)) {
+        const CellBox cell = cell_box(cells, mnx, mny, nx, ny, nz, ux, uy, uz, r.d, offx, offy, offz, idx_, idy,
+                                    idz, eps, t1);
+        const float tb = cell.exit;
+        if (cell.empty) {
           ++n;
           t = t + dt;
           if (exact) {
@@ -528,18 +547,11 @@ __device__ __forceinline__ uint32_t march_brick(const DevBrick& b, const float4*
     const float ux = fmaf(t, r.d[0], r.o[0]) - lox;
     const float uy = fmaf(t, r.d[1], r.o[1]) - loy;
     const float uz = fmaf(t, r.d[2], r.o[2]) - loz;
-    if (empty && !(t < t_cell)) {
-      const int mx = min(max(__float2int_rd(ux), 0), nx - 1) >> kMacroShift;
-      const int my = min(max(__float2int_rd(uy), 0), ny - 1) >> kMacroShift;
-      const int mz = min(max(__float2int_rd(uz), 0), nz - 1) >> kMacroShift;
-      // tb: the ray's exit from the macrocell's box shrunk by eps; every
-      // sample before it lies in this macrocell.
-      const float bx = (float)(mx << kMacroShift), by = (float)(my << kMacroShift), bz = (float)(mz << kMacroShift);
-      const float ex = ((r.d[0] > 0.f ? bx + (float)kMacro - eps : bx + eps) - offx) * idx_;
-      const float ey = ((r.d[1] > 0.f ? by + (float)kMacro - eps : by + eps) - offy) * idy;
-      const float ez = ((r.d[2] > 0.f ? bz + (float)kMacro - eps : bz + eps) - offz) * idz;
-      const float tb = fminf(fminf(fminf(ex, ey), ez), t1);
-      if (__ldg(empty + (mz * mny + my) * mnx + mx)) {
+    if (!(t < t_cell)) {
+      const CellBox cell = cell_box(cells, mnx, mny, nx, ny, nz, ux, uy, uz, r.d, offx, offy, offz, idx_, idy,
+                                    idz, eps, t1);
+      const float tb = cell.exit;
+      if (cell.empty) {
         // Empty macrocell: a sample there has alpha exactly 0 and leaves the
         // colour unchanged, so only t and the sample count advance (the same
         // t += dt sequence as full samples) up to tb; the test resumes there.
@@ -651,7 +663,7 @@ __device__ __forceinline__ uint32_t march_brick_group(const DevBrick& b, const f
   const float lox = b.lo[0], loy = b.lo[1], loz = b.lo[2];
   const float nf = (float)n_tf;
   const uint32_t cap = march_cap(t0, t1, dt);
-  const uint8_t* __restrict__ empty = b.empty;
+  const uint8_t* __restrict__ cells = b.cells;
   const int mnx = (nx + kMacro - 1) >> kMacroShift, mny = (ny + kMacro - 1) >> kMacroShift;
   const float offx = r.o[0] - lox, offy = r.o[1] - loy, offz = r.o[2] - loz;
   const float idx_ = 1.0f / r.d[0], idy = 1.0f / r.d[1], idz = 1.0f / r.d[2];
@@ -664,20 +676,14 @@ __device__ __forceinline__ uint32_t march_brick_group(const DevBrick& b, const f
   const float inv_dt = 1.0f / dt;
   float t_cell = t0;
   while (t < t1 && color.w < et && n < cap) {
-    if (empty && !(t < t_cell)) {
-      // the base sample's macrocell, exactly as march_brick
+    if (!(t < t_cell)) {
       const float ux = fmaf(t, r.d[0], r.o[0]) - lox;
       const float uy = fmaf(t, r.d[1], r.o[1]) - loy;
       const float uz = fmaf(t, r.d[2], r.o[2]) - loz;
-      const int mx = min(max(__float2int_rd(ux), 0), nx - 1) >> kMacroShift;
-      const int my = min(max(__float2int_rd(uy), 0), ny - 1) >> kMacroShift;
-      const int mz = min(max(__float2int_rd(uz), 0), nz - 1) >> kMacroShift;
-      const float bx = (float)(mx << kMacroShift), by = (float)(my << kMacroShift), bz = (float)(mz << kMacroShift);
-      const float ex = ((r.d[0] > 0.f ? bx + (float)kMacro - eps : bx + eps) - offx) * idx_;
-      const float ey = ((r.d[1] > 0.f ? by + (float)kMacro - eps : by + eps) - offy) * idy;
-      const float ez = ((r.d[2] > 0.f ? bz + (float)kMacro - eps : bz + eps) - offz) * idz;
-      const float tb = fminf(fminf(fminf(ex, ey), ez), t1);
-      if (__ldg(empty + (mz * mny + my) * mnx + mx)) {
+      const CellBox cell = cell_box(cells, mnx, mny, nx, ny, nz, ux, uy, uz, r.d, offx, offy, offz, idx_, idy,
+                                    idz, eps, t1);
+      const float tb = cell.exit;
+      if (cell.empty) {
         ++n;
         t = t + dt;
         if (exact) {
@@ -703,12 +709,8 @@ __device__ __forceinline__ uint32_t march_brick_group(const DevBrick& b, const f
       const float vx = fmaf(tk, r.d[0], r.o[0]) - lox;
       const float vy = fmaf(tk, r.d[1], r.o[1]) - loy;
       const float vz = fmaf(tk, r.d[2], r.o[2]) - loz;
-      if (empty && !(tk < t_cell)) {
-        const int mx = min(max(__float2int_rd(vx), 0), nx - 1) >> kMacroShift;
-        const int my = min(max(__float2int_rd(vy), 0), ny - 1) >> kMacroShift;
-        const int mz = min(max(__float2int_rd(vz), 0), nz - 1) >> kMacroShift;
-        full = !__ldg(empty + (mz * mny + my) * mnx + mx);
-      }
+      if (!(tk < t_cell))
+        full = !cell_box(cells, mnx, mny, nx, ny, nz, vx, vy, vz, r.d, offx, offy, offz, idx_, idy, idz, eps, t1).empty;
       if (full) {
         const StencilOut s = stencil<false>(base, sy, sz, nx, ny, nz, vx, vy, vz);
         shade = shade_factor(s, r);

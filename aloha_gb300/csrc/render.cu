@@ -376,101 +376,146 @@ __global__ void composite_u8_kernel(const uint32_t* __restrict__ imgs, const int
   }
 }
 
-// Copies a brick (x fastest) into its padded yz-quad array: element (x,y,z)
-// holds V(x,y,z), V(x,y,z+1), V(x,y+1,z), V(x,y+1,z+1) with every index
-// clamped to the brick (the apron and the quads' far rows and slices repeat
-// edge values), and flags non-finite voxels and values too large for
-// InnerCoords.  CTAs take padded rows (y, z),
-// their threads the row's elements, so the index arithmetic is one division
-// per row; a row reads four source rows, each coalesced along x.
-__global__ void pad_brick_kernel(const float* __restrict__ src, int nx, int ny, int nz, float4* __restrict__ dst,
-                                 int px, int sz, int* flags) {
-  const int py = ny + 2 * kApron, rows = py * (nz + 2 * kApron);
+// Fills a brick's padded array: element (x,y,z) holds V(x,y,z), V(x,y,z+1),
+// V(x,y+1,z), V(x,y+1,z+1) with every index clamped to the brick (the apron and
+// the quads' far rows and slices repeat edge values); flags non-finite voxels
+// and values too large for InnerCoords; and takes each macrocell's value range:
+// a sample whose value-tap cell is c (c = clamp(floor(u), 0, n-1)) reads voxels
+// c and c+1 (clamped), so macrocell m covers voxels [m*kMacro, m*kMacro +
+// kMacro] per axis.  A CTA takes kMacro rows of kMacro slices, each thread one
+// column: it loads the (kMacro + 1)^2 voxels of the column once, coalesced
+// along x, and has both the quads of its rows and the column's minimum and
+// maximum in registers; the columns meet in shared memory.
+constexpr int kFillThreads = 128, kFillColumns = kFillThreads - kMacro;
+__global__ void __launch_bounds__(kFillThreads) fill_brick_kernel(const float* __restrict__ src, int nx, int ny,
+                                                                  int nz, float4* __restrict__ dst, int px, int sz,
+                                                                  int blocks_y, float2* __restrict__ ranges,
+                                                                  int* flags) {
+  constexpr int N = kMacro + 1;
+  __shared__ float lo_s[kFillThreads], hi_s[kFillThreads];
+  const int my = (int)(blockIdx.x % (unsigned)blocks_y) - 1, mz = (int)(blockIdx.x / (unsigned)blocks_y) - 1;
+  const int y0 = my * kMacro, z0 = mz * kMacro;
+  const int mnx = (nx + kMacro - 1) >> kMacroShift, mny = (ny + kMacro - 1) >> kMacroShift;
+  const bool in_cells = my >= 0 && my < mny && mz >= 0 && mz * kMacro < nz;
+  const int t = (int)threadIdx.x;
   bool bad = false, wide = false;
-  for (int r = blockIdx.x; r < rows; r += gridDim.x) {
-    const int y = r % py, z = r / py;
-    const int y0 = min(max(y - kApron, 0), ny - 1), y1 = min(max(y + 1 - kApron, 0), ny - 1);
-    const int z0 = min(max(z - kApron, 0), nz - 1), z1 = min(max(z + 1 - kApron, 0), nz - 1);
-    const float* __restrict__ r00 = src + ((size_t)z0 * ny + y0) * nx;
-    const float* __restrict__ r10 = src + ((size_t)z0 * ny + y1) * nx;
-    const float* __restrict__ r01 = src + ((size_t)z1 * ny + y0) * nx;
-    const float* __restrict__ r11 = src + ((size_t)z1 * ny + y1) * nx;
-    float4* __restrict__ out = dst + ((size_t)z * sz + (size_t)y * px);
-    for (int x = threadIdx.x; x < px; x += blockDim.x) {
-      const int sx = min(max(x - kApron, 0), nx - 1);
-      const float4 v = make_float4(__ldg(r00 + sx), __ldg(r01 + sx), __ldg(r10 + sx), __ldg(r11 + sx));
-      const float top = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
-      wide |= top > kInnerValue;
-      bad |= !isfinite(v.x) || !isfinite(v.y) || !isfinite(v.z) || !isfinite(v.w);
-      out[x] = v;
+  for (int x0 = -kMacro; x0 < px - kApron; x0 += kFillColumns) {
+    const int x = x0 + t, xc = min(max(x, 0), nx - 1);
+    float v[N][N];  // [z][y]
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+#pragma unroll
+      for (int j = 0; j < N; ++j)
+        v[k][j] = __ldg(src + ((size_t)min(max(z0 + k, 0), nz - 1) * ny + min(max(y0 + j, 0), ny - 1)) * nx + xc);
+    float lo = v[0][0], hi = lo;
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+#pragma unroll
+      for (int j = 0; j < N; ++j) {
+        lo = fminf(lo, v[k][j]);
+        hi = fmaxf(hi, v[k][j]);
+        bad |= !isfinite(v[k][j]);
+      }
+    wide |= hi > kInnerValue || lo < -kInnerValue;
+    if (t < kFillColumns && x >= -kApron && x < px - kApron) {
+#pragma unroll
+      for (int k = 0; k < kMacro; ++k)
+#pragma unroll
+        for (int j = 0; j < kMacro; ++j) {
+          const int y = y0 + j + kApron, z = z0 + k + kApron;
+          if (y >= 0 && y < ny + 2 * kApron && z >= 0 && z < nz + 2 * kApron)
+            dst[(size_t)z * sz + (size_t)y * px + (x + kApron)] =
+                make_float4(v[k][j], v[k + 1][j], v[k][j + 1], v[k + 1][j + 1]);
+        }
+    }
+    if (in_cells) {
+      __syncthreads();  // the previous chunk's readers
+      lo_s[t] = lo;
+      hi_s[t] = hi;
+      __syncthreads();
+      const int mx = (x0 >> kMacroShift) + t;
+      if (t < kFillColumns / kMacro && mx >= 0 && mx < mnx) {
+        lo = lo_s[t * kMacro];
+        hi = hi_s[t * kMacro];
+#pragma unroll
+        for (int i = 1; i < N; ++i) {
+          lo = fminf(lo, lo_s[t * kMacro + i]);
+          hi = fmaxf(hi, hi_s[t * kMacro + i]);
+        }
+        ranges[((size_t)mz * mny + my) * mnx + mx] = make_float2(lo, hi);
+      }
     }
   }
   if (bad || wide) atomicOr(flags, (bad ? kVoxelNonfinite : 0) | (wide ? kVoxelWide : 0));
 }
 
-// Value range each macrocell's samples can read: a sample whose value-tap
-// cell is c (c = clamp(floor(u), 0, n-1)) reads voxels c and c+1 (clamped), so
-// macrocell m covers voxels [m*kMacro, m*kMacro + kMacro] per axis.  One warp
-// per macrocell: its lanes split the macrocell's pairs of (y, z) rows, read
-// each pair as yz-quads (four voxels per load, the components inside the
-// range used), and combine their minima and maxima with shuffles.
-__global__ void macrocell_range_kernel(const float4* __restrict__ base, int sy, int sz, int nx, int ny, int nz,
-                                       int mnx, int mny, int mnz, float2* __restrict__ out) {
-  const int total = mnx * mny * mnz;
-  const int lane = threadIdx.x & 31;
-  const int warps = (int)((gridDim.x * blockDim.x) >> 5);
-  for (int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); i < total; i += warps) {
-    const int mx = i % mnx, my = (i / mnx) % mny, mz = i / (mnx * mny);
-    const int x0 = mx * kMacro, y0 = my * kMacro, z0 = mz * kMacro;
-    const int x1 = min(x0 + kMacro, nx - 1), y1 = min(y0 + kMacro, ny - 1), z1 = min(z0 + kMacro, nz - 1);
-    const int pairs_y = (y1 - y0 + 2) >> 1, pairs = pairs_y * ((z1 - z0 + 2) >> 1);
-    float lo = __int_as_float(0x7f800000), hi = -lo;
-    for (int r = lane; r < pairs; r += 32) {
-      const int y = y0 + 2 * (r % pairs_y), z = z0 + 2 * (r / pairs_y);
-      const bool y_in = y + 1 <= y1, z_in = z + 1 <= z1;  // the quad's second row / slice inside the range
-      const float4* row = base + (size_t)z * sz + (size_t)y * sy;
-      for (int x = x0; x <= x1; ++x) {
-        const float4 q = __ldg(row + x);
-        lo = fminf(lo, q.x);
-        hi = fmaxf(hi, q.x);
-        if (z_in) {
-          lo = fminf(lo, q.y);
-          hi = fmaxf(hi, q.y);
-        }
-        if (y_in) {
-          lo = fminf(lo, q.z);
-          hi = fmaxf(hi, q.z);
-        }
-        if (y_in && z_in) {
-          lo = fminf(lo, q.w);
-          hi = fmaxf(hi, q.w);
-        }
-      }
+// Macrocell codes.  A macrocell is empty when every transfer-function entry
+// its lookups can touch has alpha 0: indices floor(v*n - 1/2) and +1 for v in
+// [lo, hi], with one index of margin on each side for rounding of the
+// interpolated value.  The Chebyshev distance to the other kind is separable:
+// along x first (here, from the kinds of a row's neighbours in shared memory),
+// then over y, then over z, each the smallest max(step, distance there), where
+// a cell of the other kind has distance 0.
+constexpr int kCodeThreads = 256;
+__global__ void __launch_bounds__(kCodeThreads) macrocell_kinds_kernel(const DevBrick* __restrict__ bricks,
+                                                                       const uint8_t* cells,
+                                                                       const float2* __restrict__ ranges,
+                                                                       const int* __restrict__ prefix, int n,
+                                                                       uint8_t* __restrict__ out) {
+  constexpr int W = kMaxReach - 1;
+  __shared__ uint8_t kind[kCodeThreads + 2 * W];
+  const DevBrick& b = bricks[blockIdx.y];
+  const size_t first = (size_t)(b.cells - cells);
+  const int mnx = (b.n[0] + kMacro - 1) >> kMacroShift;
+  const int count = mnx * ((b.n[1] + kMacro - 1) >> kMacroShift) * ((b.n[2] + kMacro - 1) >> kMacroShift);
+  const float nf = (float)n;
+  for (int i0 = blockIdx.x * kCodeThreads; i0 < count; i0 += gridDim.x * kCodeThreads) {
+    __syncthreads();
+    for (int k = threadIdx.x; k < kCodeThreads + 2 * W; k += kCodeThreads) {
+      const int i = i0 - W + k;
+      if (i < 0 || i >= count) continue;
+      const float2 r = ranges[first + i];
+      const float xl = fminf(fmaxf(r.x * nf - 0.5f, -8.0f), nf + 8.0f);
+      const float xh = fminf(fmaxf(r.y * nf - 0.5f, -8.0f), nf + 8.0f);
+      const int lo = max((int)floorf(xl) - 1, 0);
+      const int hi = min((int)floorf(xh) + 2, n - 1);
+      kind[k] = lo <= hi && __ldg(prefix + hi + 1) != __ldg(prefix + lo) ? kCellFull : 0;
     }
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) {
-      lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, d));
-      hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, d));
-    }
-    if (lane == 0) out[i] = make_float2(lo, hi);
+    __syncthreads();
+    const int i = i0 + (int)threadIdx.x;
+    if (i >= count) continue;
+    const uint8_t* at = kind + W + threadIdx.x;
+    const int x = i % mnx, me = at[0];
+    int reach = 1;
+    while (reach < kMaxReach && (x - reach < 0 || at[-reach] == me) && (x + reach >= mnx || at[reach] == me)) ++reach;
+    out[first + i] = (uint8_t)(me | reach);
   }
 }
 
-// A macrocell is empty when every transfer-function entry its lookups can
-// touch has alpha 0: indices floor(v*n - 1/2) and +1 for v in [lo, hi], with
-// one index of margin on each side for rounding of the interpolated value.
-// prefix[k] = number of entries below k with non-zero alpha.
-__global__ void macrocell_empty_kernel(const float2* __restrict__ ranges, int count, const int* __restrict__ prefix,
-                                       int n, uint8_t* __restrict__ empty) {
-  const float nf = (float)n;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-    const float2 r = ranges[i];
-    const float xl = fminf(fmaxf(r.x * nf - 0.5f, -8.0f), nf + 8.0f);
-    const float xh = fminf(fmaxf(r.y * nf - 0.5f, -8.0f), nf + 8.0f);
-    const int lo = max((int)floorf(xl) - 1, 0);
-    const int hi = min((int)floorf(xh) + 2, n - 1);
-    const int nonzero = lo <= hi ? __ldg(prefix + hi + 1) - __ldg(prefix + lo) : 0;
-    empty[i] = nonzero == 0 ? 1 : 0;
+template <int AXIS>
+__global__ void __launch_bounds__(kCodeThreads) macrocell_reach_kernel(const DevBrick* __restrict__ bricks,
+                                                                       const uint8_t* cells,
+                                                                       const uint8_t* __restrict__ in,
+                                                                       uint8_t* __restrict__ out) {
+  const DevBrick& b = bricks[blockIdx.y];
+  const size_t first = (size_t)(b.cells - cells);
+  const int mnx = (b.n[0] + kMacro - 1) >> kMacroShift, mny = (b.n[1] + kMacro - 1) >> kMacroShift,
+            mnz = (b.n[2] + kMacro - 1) >> kMacroShift;
+  const int count = mnx * mny * mnz, stride = AXIS == 1 ? mnx : mnx * mny, len = AXIS == 1 ? mny : mnz;
+  for (int i = blockIdx.x * kCodeThreads + threadIdx.x; i < count; i += gridDim.x * kCodeThreads) {
+    const int p = (i / stride) % len;
+    const int code = in[first + i], me = code & kCellFull;
+    int reach = code & (kCellFull - 1);
+    auto see = [&](int j, int step) {
+      const int c = in[first + i + j * stride];
+      const int there = (c & kCellFull) == me ? c & (kCellFull - 1) : 0;
+      reach = min(reach, max(step, there));
+    };
+    for (int j = 1; j < reach; ++j) {
+      if (p >= j) see(-j, j);
+      if (p + j < len) see(j, j);
+    }
+    out[first + i] = (uint8_t)(me | reach);
   }
 }
 
@@ -479,20 +524,14 @@ static size_t render_smem(int n_tf, int stage) {
   return tf_smem(n_tf) + (stage == ALOHA_STAGING_NEXT_SAMPLE ? kStageBytes : 0);
 }
 
-cudaError_t launch_macrocell_range(const DevBrick& b, float2* out, cudaStream_t s) {
-  const int mnx = (b.n[0] + kMacro - 1) >> kMacroShift, mny = (b.n[1] + kMacro - 1) >> kMacroShift,
-            mnz = (b.n[2] + kMacro - 1) >> kMacroShift;
-  const int total = mnx * mny * mnz;
-  const int grid = min((total + 3) / 4, 152 * 32);  // 4 warps (macrocells) per CTA
-  macrocell_range_kernel<<<grid, 128, 0, s>>>(b.base, b.sy, b.sz, b.n[0], b.n[1], b.n[2], mnx, mny, mnz, out);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_macrocell_empty(const float2* ranges, int count, const int* prefix, int n, uint8_t* empty,
-                                   cudaStream_t s) {
-  if (count <= 0) return cudaSuccess;
-  const int grid = min((count + 255) / 256, 152 * 16);
-  macrocell_empty_kernel<<<grid, 256, 0, s>>>(ranges, count, prefix, n, empty);
+cudaError_t launch_macrocell_codes(const DevBrick* bricks, int n_bricks, int most_cells, const float2* ranges,
+                                   const int* prefix, int n_tf, uint8_t* cells, uint8_t* tmp, cudaStream_t s) {
+  for (int b0 = 0; b0 < n_bricks; b0 += 65535) {  // a grid's y extent
+    const dim3 grid(min((most_cells + kCodeThreads - 1) / kCodeThreads, 152 * 8), min(n_bricks - b0, 65535));
+    macrocell_kinds_kernel<<<grid, kCodeThreads, 0, s>>>(bricks + b0, cells, ranges, prefix, n_tf, cells);
+    macrocell_reach_kernel<1><<<grid, kCodeThreads, 0, s>>>(bricks + b0, cells, cells, tmp);
+    macrocell_reach_kernel<2><<<grid, kCodeThreads, 0, s>>>(bricks + b0, cells, tmp, cells);
+  }
   return cudaGetLastError();
 }
 
@@ -597,11 +636,12 @@ cudaError_t launch_composite_u8(const uint32_t* imgs, const int* order, int n_ra
   return cudaGetLastError();
 }
 
-cudaError_t launch_pad_brick(const float* src, int nx, int ny, int nz, float4* dst, int px, int sz, int* flags,
-                             cudaStream_t s) {
-  const int rows = (ny + 2 * kApron) * (nz + 2 * kApron);
-  const int g = rows < 152 * 32 ? rows : 152 * 32;  // CTAs of 128 threads take rows
-  pad_brick_kernel<<<g < 1 ? 1 : g, 128, 0, s>>>(src, nx, ny, nz, dst, px, sz, flags);
+cudaError_t launch_fill_brick(const DevBrick& b, const float* src, float4* dst, float2* ranges, int* flags,
+                              cudaStream_t s) {
+  // blocks of kMacro rows and slices from -kMacro to the last apron row
+  const int blocks_y = (b.n[1] + kApron - 1) / kMacro + 2, blocks_z = (b.n[2] + kApron - 1) / kMacro + 2;
+  fill_brick_kernel<<<blocks_y * blocks_z, kFillThreads, 0, s>>>(src, b.n[0], b.n[1], b.n[2], dst, b.sy, b.sz, blocks_y,
+                                                               ranges, flags);
   return cudaGetLastError();
 }
 
