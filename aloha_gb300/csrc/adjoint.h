@@ -82,12 +82,9 @@ struct TrainArgs {
 };
 
 // One persistent training forward over the launch's views (a.tv, a.runs).
-// `many` selects the instance for launches of many chunks per resident warp
-// (kTrainForwardBlocksMany CTAs per SM instead of kTrainForwardBlocks); `inner`
-// (here and below): every brick and view of the launch is InnerCoords.
-cudaError_t launch_forward_train(const TrainArgs& a, unsigned items, int max_grid, bool many, bool inner,
-                                 cudaStream_t s);
-int forward_train_blocks_per_sm(int n_tf, bool many);
+// `inner` (here and below): every brick and view of the launch is InnerCoords.
+cudaError_t launch_forward_train(const TrainArgs& a, unsigned items, int max_grid, bool inner, cudaStream_t s);
+int forward_train_blocks_per_sm(int n_tf);
 // One persistent backward over the launch's views' items (a.tv, a.item_base).
 cudaError_t launch_backward(const TrainArgs& a, int grid, bool inner, cudaStream_t s);
 // The all-empty segments of the same views (a.empty_base): the gradient of

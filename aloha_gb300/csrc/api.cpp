@@ -149,6 +149,7 @@ struct aloha_ctx {
   // the transfer-function size through shared memory)
   int chunk_w = 0, chunk_h = 0;  // 0 = automatic
   int grid_n_tf = -1, grid_blocks = 0, grid_cw = 0, grid_ch = 0;
+  bool grid_few = false;
   // cost-ordered chunks of single-view renders: mode, probe costs | max | order
   int chunk_order_mode = ALOHA_CHUNKS_AUTO;
   DeviceBuffer chunk_order;
@@ -557,14 +558,20 @@ int launch_single(aloha_ctx* c, const FrameArgs& f, int view, cudaStream_t s) {
     cw = 8;
     ch = 4;
   }
-  if (c->grid_n_tf != c->n_tf || c->grid_cw != cw || c->grid_ch != ch || c->grid_stage != c->staging) {
-    const int per_sm = render_blocks_per_sm(cw, ch, c->n_tf, false, c->staging);
+  // few chunks per warp: the instance of fewer, faster warps
+  const long long all_chunks = (long long)((v.width + cw - 1) / cw) * ((v.height + ch - 1) / ch);
+  const bool few = cw == 8 && ch == 4 && c->staging == ALOHA_STAGING_NONE && c->lane_group_permille == 0 &&
+                   all_chunks < (long long)kFewChunksPerWarp * c->num_sms * kSingleRenderBlocks * (kRenderThreads / 32);
+  if (c->grid_n_tf != c->n_tf || c->grid_cw != cw || c->grid_ch != ch || c->grid_stage != c->staging ||
+      c->grid_few != few) {
+    const int per_sm = render_blocks_per_sm(cw, ch, c->n_tf, false, c->staging, false, few);
     if (per_sm <= 0) return c->fail(ALOHA_ERR_CUDA, "render occupancy query failed");
     c->grid_blocks = per_sm * c->num_sms;
     c->grid_n_tf = c->n_tf;
     c->grid_cw = cw;
     c->grid_ch = ch;
     c->grid_stage = c->staging;
+    c->grid_few = few;
   }
   BatchArgs b{};
   b.f = f;
@@ -600,7 +607,7 @@ int launch_single(aloha_ctx* c, const FrameArgs& f, int view, cudaStream_t s) {
   const int warps_per_block = kRenderThreads / 32;
   const int grid = std::max(1, std::min(lane_groups ? c->grid_blocks_lg : c->grid_blocks,
                                         (b.total_tiles + warps_per_block - 1) / warps_per_block));
-  CUDA_TRY(c, launch_render_warps(b, cw, ch, grid, false, s, c->staging, lane_groups));
+  CUDA_TRY(c, launch_render_warps(b, cw, ch, grid, false, s, c->staging, lane_groups, few));
   return ALOHA_OK;
 }
 
@@ -1461,15 +1468,10 @@ int forward_views(aloha_ctx* c, int n_views, const int* view_ids, float* const* 
   a.n_runs = n_runs;
   a.run_views = reinterpret_cast<const int*>(dev[3]);
   CUDA_TRY(c, cudaMemsetAsync(c->counter.ptr, 0, sizeof(unsigned long long), s));
-  // few chunks per resident warp: the launch ends on its longest rays (fewer,
-  // faster warps); many: throughput-bound (more warps)
   const bool inner = train_inner(c, n_views, view_ids);
-  const int few_per_sm = forward_train_blocks_per_sm(c->n_tf, false);
-  if (few_per_sm <= 0) return c->fail(ALOHA_ERR_CUDA, "forward occupancy query failed");
-  const bool many = items >= (unsigned long long)kTrainManyChunksPerWarp * few_per_sm * c->num_sms * 4;
-  const int per_sm = many ? forward_train_blocks_per_sm(c->n_tf, true) : few_per_sm;
+  const int per_sm = forward_train_blocks_per_sm(c->n_tf);
   if (per_sm <= 0) return c->fail(ALOHA_ERR_CUDA, "forward occupancy query failed");
-  CUDA_TRY(c, launch_forward_train(a, (unsigned)items, per_sm * c->num_sms, many, inner, s));
+  CUDA_TRY(c, launch_forward_train(a, (unsigned)items, per_sm * c->num_sms, inner, s));
   c->samples_valid = true;
   bool any_host = false;
   for (int i = 0; i < n_views; ++i) {

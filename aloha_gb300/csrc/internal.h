@@ -215,20 +215,26 @@ cudaError_t launch_fill_brick(const DevBrick& b, const float* src, float4* dst_a
                               cudaStream_t s);
 // Persistent render launch; `batch` selects the instance tuned for batches.
 constexpr int kSingleRenderBlocks = 5, kBatchRenderBlocks = 7;  // CTAs per SM
-// CTAs per SM of the differentiable form's forward (checkpointed march): a
-// launch of few chunks ends on its longest rays and runs faster with fewer,
-// faster warps; one of at least kTrainManyChunksPerWarp chunks per resident
-// warp is throughput-bound and runs faster with more.
-constexpr int kTrainForwardBlocks = 5, kTrainForwardBlocksMany = 7;
-constexpr int kTrainManyChunksPerWarp = 16;
+// A single view of few 8x4 chunks per resident warp ends on its longest rays,
+// which run faster with fewer, less spilling neighbours (4 / 5 CTAs per SM, us:
+// 64^3 at 512^2 81 / 89, 256^3 at 1024x768 257 / 263, 512^3 at 512^2 599 / 633);
+// with many, throughput counts (64^3 at 1024^2 155 / 146, 256^3 at 1280x1024 354
+// / 331, 512^3 at 1920x1080 650 / 630; 512^3 at 1024^2, 10.8 chunks per warp of
+// the 5-CTA instance, 602 / 605).
+constexpr int kFewChunkRenderBlocks = 4, kFewChunksPerWarp = 9;
+// CTAs per SM of the differentiable form's forward (checkpointed march).  Six
+// 512^2 views of 256^3: 785 us at 5, 820 at 6, 875 at 7; one 1024^2 view of
+// 512^3: 900 at 5, 914 at 4.
+constexpr int kTrainForwardBlocks = 5;
 // `stage`: ALOHA_STAGING_NONE or _NEXT_SAMPLE (the stencil loads), or, for
 // batches, kStageUnroll2: direct loads with the march loop written out two
 // steps per trip.
 constexpr int kStageUnroll2 = 2;
 // `lane_groups`: the instance that renders the first a.group_chunks chunks of
 // the cost order with lane groups (single view, 8x4 chunks, direct loads).
+// `few`: the 8x4 instance for few chunks per warp (single view, direct loads).
 cudaError_t launch_render_warps(const BatchArgs& a, int chunk_w, int chunk_h, int grid, bool batch, cudaStream_t s,
-                                int stage = ALOHA_STAGING_NONE, bool lane_groups = false);
+                                int stage = ALOHA_STAGING_NONE, bool lane_groups = false, bool few = false);
 // The macrocell codes of all bricks from their value ranges; prefix[k] = number
 // of transfer-function entries below k with non-zero alpha.  Cells of brick b
 // start at bricks[b].cells - cells in each array; tmp is scratch of their size.
@@ -240,7 +246,7 @@ inline int macrocells(const DevBrick& b) {
 }
 // CTAs of the render kernel that fit on one SM for a chunk shape (0 if the shape is unknown).
 int render_blocks_per_sm(int chunk_w, int chunk_h, int n_tf, bool batch, int stage = ALOHA_STAGING_NONE,
-                         bool lane_groups = false);
+                         bool lane_groups = false, bool few = false);
 // `many_ranks` selects the instance tuned for many short (chunk, rank) items.
 constexpr int kManyRankSplitBlocks = 7;  // CTAs per SM
 cudaError_t launch_render_split(const SplitArgs& a, int grid, bool many_ranks, cudaStream_t s);

@@ -435,29 +435,30 @@ __device__ __forceinline__ void composite_step(float4& color, const float4 c, fl
   color.w = fmaf(oma, c.w, color.w);
 }
 
-// A macrocell lookup at voxel coordinate u: whether the cell is empty, and the
-// ray parameter (at most t1) up to which every sample stays in the box of cells
-// of its kind around it, shrunk by eps.
-struct CellBox {
-  bool empty;
-  float exit;
+// A macrocell at voxel coordinate u: its code, and the ray parameter (at most
+// t1) up to which every sample stays in the box of cells of its kind around it
+// (its reach), shrunk by eps.
+struct Cell {
+  int x, y, z, code;
+  __device__ __forceinline__ bool empty() const { return code < kCellFull; }
 };
-__device__ __forceinline__ CellBox cell_box(const uint8_t* __restrict__ cells, int mnx, int mny, int nx, int ny, int nz,
-                                            float ux, float uy, float uz, const float d[3], float offx, float offy,
-                                            float offz, float idx, float idy, float idz, float eps, float t1) {
-  const int mx = min(max(__float2int_rd(ux), 0), nx - 1) >> kMacroShift;
-  const int my = min(max(__float2int_rd(uy), 0), ny - 1) >> kMacroShift;
-  const int mz = min(max(__float2int_rd(uz), 0), nz - 1) >> kMacroShift;
-  const int code = __ldg(cells + (mz * mny + my) * mnx + mx);
-  const int reach = code & (kCellFull - 1);
+__device__ __forceinline__ Cell cell_at(const uint8_t* __restrict__ cells, int mnx, int mny, int nx, int ny, int nz,
+                                        float ux, float uy, float uz) {
+  Cell c;
+  c.x = min(max(__float2int_rd(ux), 0), nx - 1) >> kMacroShift;
+  c.y = min(max(__float2int_rd(uy), 0), ny - 1) >> kMacroShift;
+  c.z = min(max(__float2int_rd(uz), 0), nz - 1) >> kMacroShift;
+  c.code = __ldg(cells + (c.z * mny + c.y) * mnx + c.x);
+  return c;
+}
+__device__ __forceinline__ float cell_exit(const Cell& c, const float d[3], float offx, float offy, float offz,
+                                           float idx, float idy, float idz, float eps, float t1) {
+  const int reach = c.code & (kCellFull - 1);
   auto face = [&](int m, float dir) {
     return dir > 0.f ? (float)((m + reach) << kMacroShift) - eps : (float)((m + 1 - reach) << kMacroShift) + eps;
   };
-  CellBox c;
-  c.empty = code < kCellFull;
-  c.exit = fminf(fminf(fminf((face(mx, d[0]) - offx) * idx, (face(my, d[1]) - offy) * idy),
-                       (face(mz, d[2]) - offz) * idz), t1);
-  return c;
+  return fminf(fminf(fminf((face(c.x, d[0]) - offx) * idx, (face(c.y, d[1]) - offy) * idy),
+                     (face(c.z, d[2]) - offz) * idz), t1);
 }
 
 // A march hook sees every sample, full or skipped, before it is taken: its
@@ -473,6 +474,19 @@ struct NoHook {
 
 // integrateBrick (deviceCode.cpp:256-298) over [t0, t1); returns the number
 // of samples taken.
+//
+// The lanes of a warp reach empty space at different samples, and the warp
+// pays for a lookup and a jump whenever one of them does.  So the march
+// alternates: lookups and jumps, at most kMarchJumps of them, then kMarchRun
+// samples that need none; the lanes meet at both.
+// With a lookup before every sample that leaves a box, a 64^3 frame at 512^2
+// executed 313 instructions per warp and sample, which at 16 to 20 warps per SM
+// its longest rays wait for one after the other.  512^3 frame / 64^3 frame /
+// 24-view batch: 752 us / 90.7 us / 7.66 ms with boxes, 689 / 75 / 7.47 with 2
+// jumps and 6 samples (4 CTAs per SM for the frames); 1 and 6: 707 / 78 / 7.83;
+// 3 and 6: 697 / 76 / 7.35; 2 and 5: 692 / 75 / 7.45; 2 and 8: 688 / 76 / 7.52;
+// as many jumps as it takes and 4: 935 / 90 / 7.97.
+constexpr int kMarchJumps = 2, kMarchRun = 6;
 template <bool INNER, class Hook, class Loads = DirectLoads>
 __device__ __forceinline__ uint32_t march_brick(const DevBrick& b, const float4* __restrict__ tf_s, int n_tf,
                                                 const Ray& r, float t0, float t1, float ils, float dt, float et,
@@ -496,125 +510,91 @@ __device__ __forceinline__ uint32_t march_brick(const DevBrick& b, const float4*
   float t = first_sample_t(t0, dt, ils);
   const bool exact = exact_steps(t, t1, dt);
   const float inv_dt = 1.0f / dt;
-  // Samples before t_cell lie in the last box of full macrocells, so they
-  // need no lookup.  Only the skip below depends on the lookup (a full sample
-  // in an empty macrocell leaves the colour unchanged as well), so that bound
-  // only has to be right for speed.
-  float t_cell = t0;
   loads.begin_brick();
-  if constexpr (Loads::kSteps > 1 && !Hook::kActive && !Loads::kStaged) {
-    // The loop below for the render (no hook, direct loads), written out
-    // Loads::kSteps steps per trip.
-    auto step = [&]() -> bool {
-      if (!(t < t1 && color.w < et && n < cap)) return false;
+  while (t < t1 && color.w < et && n < cap) {
+    // Up to kMarchJumps steps over empty boxes, until the ray is at a sample in
+    // a full macrocell.  A sample in an empty one has alpha exactly 0 and leaves
+    // the colour unchanged, so only t and the sample count advance (the same t
+    // += dt sequence as full samples) up to the box's end.  The first is always
+    // taken.  With exact steps the rest of the run is one jump (one more per
+    // power of two it crosses, and one per checkpoint the hook needs).
+    int jumps = 0;
+    for (; jumps < kMarchJumps && t < t1 && n < cap; ++jumps) {
+      const Cell cell = cell_at(cells, mnx, mny, nx, ny, nz, fmaf(t, r.d[0], r.o[0]) - lox,
+                                fmaf(t, r.d[1], r.o[1]) - loy, fmaf(t, r.d[2], r.o[2]) - loz);
+      if (!cell.empty()) break;
+      const float tb = cell_exit(cell, r.d, offx, offy, offz, idx_, idy, idz, eps, t1);
+      hook(t, n, color);
+      ++n;
+      t = t + dt;
+      if constexpr (!Hook::kActive) {
+        if (exact) {
+          run_steps(t, n, tb, cap, dt, inv_dt, 0xffffffffu);
+        } else {
+          while (t < tb && n < cap) {
+            ++n;
+            t = t + dt;
+          }
+        }
+      } else if (exact) {
+        for (;;) {
+          hook.left -= run_steps(t, n, tb, cap, dt, inv_dt, hook.left);
+          if (!(t < tb && n < cap)) break;
+          hook(t, n, color);  // a checkpoint falls due here (hook.left == 0)
+          ++n;
+          t = t + dt;
+        }
+      } else {
+        while (t < tb && n < cap) {
+          uint32_t k = hook.left;
+          while (k > 0 && t < tb && n < cap) {
+            ++n;
+            t = t + dt;
+            --k;
+          }
+          hook.left = k;
+          if (k == 0 && t < tb && n < cap) {
+            hook(t, n, color);
+            ++n;
+            t = t + dt;
+          }
+        }
+      }
+    }
+    if (jumps == kMarchJumps) continue;
+    // Up to kMarchRun samples without another lookup (a full sample in an empty
+    // macrocell leaves the colour unchanged as well).
+    int k = 0;
+    auto step = [&]() {
+      if (!(k < kMarchRun && t < t1 && color.w < et && n < cap)) return false;
       const float ux = fmaf(t, r.d[0], r.o[0]) - lox;
       const float uy = fmaf(t, r.d[1], r.o[1]) - loy;
       const float uz = fmaf(t, r.d[2], r.o[2]) - loz;
-      if (!(t < t_cell)) {
-        const CellBox cell = cell_box(cells, mnx, mny, nx, ny, nz, ux, uy, uz, r.d, offx, offy, offz, idx_, idy,
-                                    idz, eps, t1);
-        const float tb = cell.exit;
-        if (cell.empty) {
-          ++n;
-          t = t + dt;
-          if (exact) {
-            run_steps(t, n, tb, cap, dt, inv_dt, 0xffffffffu);
-          } else {
-            while (t < tb && n < cap) {
-              ++n;
-              t = t + dt;
-            }
-          }
-          return true;
-        }
-        t_cell = tb;
-      }
+      hook(t, n, color);
+      if constexpr (Hook::kActive) hook.full_segment = true;
       ++n;
-      const StencilOut s = stencil<INNER>(base, sy, sz, nx, ny, nz, ux, uy, uz);
+      ++k;
+      StencilOut s;
+      if constexpr (Loads::kStaged)
+        s = loads.sample(base, sy, sz, nx, ny, nz, ux, uy, uz, t, t1, dt, r.o, r.d, lox, loy, loz);
+      else
+        s = stencil<INNER>(base, sy, sz, nx, ny, nz, ux, uy, uz);
       const float shade = shade_factor(s, r);
       const float4 c = tf_lookup<INNER>(tf_s, n_tf, nf, s.value);
       composite_step(color, c, shade);
       t = t + dt;
       return true;
     };
-    for (bool go = true; go;) {
+    if constexpr (Loads::kSteps > 1) {
+      for (bool go = true; go;) {
 #pragma unroll
-      for (int k = 0; k < Loads::kSteps; ++k) go = go && step();
-    }
-    return n;
-  }
-  while (t < t1 && color.w < et && n < cap) {
-    const float ux = fmaf(t, r.d[0], r.o[0]) - lox;
-    const float uy = fmaf(t, r.d[1], r.o[1]) - loy;
-    const float uz = fmaf(t, r.d[2], r.o[2]) - loz;
-    if (!(t < t_cell)) {
-      const CellBox cell = cell_box(cells, mnx, mny, nx, ny, nz, ux, uy, uz, r.d, offx, offy, offz, idx_, idy,
-                                    idz, eps, t1);
-      const float tb = cell.exit;
-      if (cell.empty) {
-        // Empty macrocell: a sample there has alpha exactly 0 and leaves the
-        // colour unchanged, so only t and the sample count advance (the same
-        // t += dt sequence as full samples) up to tb; the test resumes there.
-        // The first is always taken.  With exact steps the rest of the run is
-        // one jump (one more per power of two it crosses, and one per
-        // checkpoint the hook needs).
-        if constexpr (!Hook::kActive) {
-          ++n;
-          t = t + dt;
-          if (exact) {
-            run_steps(t, n, tb, cap, dt, inv_dt, 0xffffffffu);
-            continue;
-          }
-          while (t < tb && n < cap) {
-            ++n;
-            t = t + dt;
-          }
-        } else if (exact) {
-          hook(t, n, color);
-          ++n;
-          t = t + dt;
-          for (;;) {
-            hook.left -= run_steps(t, n, tb, cap, dt, inv_dt, hook.left);
-            if (!(t < tb && n < cap)) break;
-            hook(t, n, color);  // a checkpoint falls due here (hook.left == 0)
-            ++n;
-            t = t + dt;
-          }
-        } else {
-          hook(t, n, color);
-          ++n;
-          t = t + dt;
-          while (t < tb && n < cap) {
-            uint32_t k = hook.left;
-            while (k > 0 && t < tb && n < cap) {
-              ++n;
-              t = t + dt;
-              --k;
-            }
-            hook.left = k;
-            if (k == 0 && t < tb && n < cap) {
-              hook(t, n, color);
-              ++n;
-              t = t + dt;
-            }
-          }
-        }
-        continue;
+        for (int i = 0; i < Loads::kSteps; ++i) go = go && step();
       }
-      t_cell = tb;
+    } else {
+#pragma unroll 1
+      while (step()) {
+      }
     }
-    hook(t, n, color);
-    if constexpr (Hook::kActive) hook.full_segment = true;
-    ++n;
-    StencilOut s;
-    if constexpr (Loads::kStaged)
-      s = loads.sample(base, sy, sz, nx, ny, nz, ux, uy, uz, t, t1, dt, r.o, r.d, lox, loy, loz);
-    else
-      s = stencil<INNER>(base, sy, sz, nx, ny, nz, ux, uy, uz);
-    const float shade = shade_factor(s, r);
-    const float4 c = tf_lookup<INNER>(tf_s, n_tf, nf, s.value);
-    composite_step(color, c, shade);
-    t = t + dt;
   }
   return n;
 }
@@ -680,10 +660,9 @@ __device__ __forceinline__ uint32_t march_brick_group(const DevBrick& b, const f
       const float ux = fmaf(t, r.d[0], r.o[0]) - lox;
       const float uy = fmaf(t, r.d[1], r.o[1]) - loy;
       const float uz = fmaf(t, r.d[2], r.o[2]) - loz;
-      const CellBox cell = cell_box(cells, mnx, mny, nx, ny, nz, ux, uy, uz, r.d, offx, offy, offz, idx_, idy,
-                                    idz, eps, t1);
-      const float tb = cell.exit;
-      if (cell.empty) {
+      const Cell cell = cell_at(cells, mnx, mny, nx, ny, nz, ux, uy, uz);
+      const float tb = cell_exit(cell, r.d, offx, offy, offz, idx_, idy, idz, eps, t1);
+      if (cell.empty()) {
         ++n;
         t = t + dt;
         if (exact) {
@@ -709,8 +688,7 @@ __device__ __forceinline__ uint32_t march_brick_group(const DevBrick& b, const f
       const float vx = fmaf(tk, r.d[0], r.o[0]) - lox;
       const float vy = fmaf(tk, r.d[1], r.o[1]) - loy;
       const float vz = fmaf(tk, r.d[2], r.o[2]) - loz;
-      if (!(tk < t_cell))
-        full = !cell_box(cells, mnx, mny, nx, ny, nz, vx, vy, vz, r.d, offx, offy, offz, idx_, idy, idz, eps, t1).empty;
+      if (!(tk < t_cell)) full = !cell_at(cells, mnx, mny, nx, ny, nz, vx, vy, vz).empty();
       if (full) {
         const StencilOut s = stencil<false>(base, sy, sz, nx, ny, nz, vx, vy, vz);
         shade = shade_factor(s, r);

@@ -20,8 +20,9 @@ namespace aloha {
 // on other warps or CTAs.
 // MINB CTAs of 128 threads per SM: a single view ends with its slowest
 // chunks, which run faster with more registers per thread (5 CTAs, 96
-// registers); a batch of views is throughput-bound and runs faster with more
-// resident warps (7 CTAs, 72 registers).
+// registers, or 4 when there are few chunks); a batch of views is
+// throughput-bound and runs faster with more resident warps (7 CTAs, 72
+// registers).
 // STAGE selects the stencil loads: 0 direct, 1 the next sample's rows staged
 // in shared memory with cp.async (StagedLoads; shared memory after the
 // transfer function), kStageUnroll2 (batches) direct with the march loop
@@ -548,7 +549,7 @@ RenderKernel render_kernel_for(int chunk_w, int chunk_h) {
   return nullptr;
 }
 
-RenderKernel render_kernel(int chunk_w, int chunk_h, bool batch, int stage, bool lane_groups) {
+RenderKernel render_kernel(int chunk_w, int chunk_h, bool batch, int stage, bool lane_groups, bool few) {
   if (lane_groups)
     return (!batch && stage == ALOHA_STAGING_NONE && chunk_w == 8 && chunk_h == 4)
                ? render_warps_kernel<8, 4, kSingleRenderBlocks, 0, kLaneGroup>
@@ -559,6 +560,7 @@ RenderKernel render_kernel(int chunk_w, int chunk_h, bool batch, int stage, bool
   if (stage == kStageUnroll2) return batch ? render_kernel_for<kBatchRenderBlocks, kStageUnroll2>(chunk_w, chunk_h)
                                            : nullptr;
   if (stage != ALOHA_STAGING_NONE) return nullptr;
+  if (few && !batch && chunk_w == 8 && chunk_h == 4) return render_warps_kernel<8, 4, kFewChunkRenderBlocks, 0>;
   return batch ? render_kernel_for<kBatchRenderBlocks, 0>(chunk_w, chunk_h)
                : render_kernel_for<kSingleRenderBlocks, 0>(chunk_w, chunk_h);
 }
@@ -566,16 +568,16 @@ RenderKernel render_kernel(int chunk_w, int chunk_h, bool batch, int stage, bool
 }  // namespace
 
 cudaError_t launch_render_warps(const BatchArgs& b, int chunk_w, int chunk_h, int grid, bool batch, cudaStream_t s,
-                                int stage, bool lane_groups) {
+                                int stage, bool lane_groups, bool few) {
   if (lane_groups && (!b.chunk_order || b.f.rank_images || b.f.rank_depth || b.f.accum)) return cudaErrorInvalidValue;
-  const RenderKernel k = render_kernel(chunk_w, chunk_h, batch, stage, lane_groups);
+  const RenderKernel k = render_kernel(chunk_w, chunk_h, batch, stage, lane_groups, few);
   if (!k) return cudaErrorInvalidValue;
   k<<<grid, kRenderThreads, render_smem(b.f.n_tf, stage), s>>>(b);
   return cudaGetLastError();
 }
 
-int render_blocks_per_sm(int chunk_w, int chunk_h, int n_tf, bool batch, int stage, bool lane_groups) {
-  const RenderKernel k = render_kernel(chunk_w, chunk_h, batch, stage, lane_groups);
+int render_blocks_per_sm(int chunk_w, int chunk_h, int n_tf, bool batch, int stage, bool lane_groups, bool few) {
+  const RenderKernel k = render_kernel(chunk_w, chunk_h, batch, stage, lane_groups, few);
   int n = 0;
   if (!k || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, kRenderThreads, render_smem(n_tf, stage)) !=
                 cudaSuccess) {
