@@ -413,6 +413,16 @@ class Batch:
             pass
 
 
+def _wait_elsewhere(stream, *buffers):
+    """Waits for `stream` if it is not torch's current one and a buffer is a CUDA
+    tensor: the library's call has only been enqueued there, and the tensor's
+    memory may be given to work on the current stream once it is freed."""
+    if any(getattr(b, "is_cuda", False) for b in buffers):
+        import torch
+        if _stream(stream) != torch.cuda.current_stream().cuda_stream:
+            torch.cuda.ExternalStream(_stream(stream)).synchronize()
+
+
 def composite_over(rank_images, order, width: int, height: int, mode: int = COMPOSITE_FP32, fb=None, stream=None):
     """IceT stand-in: ordered over of float rank images [n][H][W][4] -> RGBA8."""
     L = lib()
@@ -423,6 +433,7 @@ def composite_over(rank_images, order, width: int, height: int, mode: int = COMP
                                 _stream(stream))
     if rc != OK:
         raise AlohaError(rc, L.aloha_status_string(rc).decode())
+    _wait_elsewhere(stream, rank_images, fb)
     return fb
 
 
@@ -434,4 +445,5 @@ def composite_over_rgba8(rank_fbs, order, width: int, height: int, fb=None, stre
     rc = L.aloha_composite_over_rgba8(_addr(rank_fbs), _addr(o), o.size, width, height, _addr(fb), _stream(stream))
     if rc != OK:
         raise AlohaError(rc, L.aloha_status_string(rc).decode())
+    _wait_elsewhere(stream, rank_fbs, fb)
     return fb

@@ -32,14 +32,12 @@ struct TrainState {
   Checkpoint* ckpt = nullptr;
   float4* final_rgba = nullptr;
   uint2* work = nullptr;
-  unsigned* work_count = nullptr;
-  int* overflow = nullptr;
   size_t bytes = 0;
   unsigned k = 0, cap = 0;
   size_t npx = 0;
   bool valid = false;
   void release() {
-    for (void* p : {(void*)ckpt, (void*)final_rgba, (void*)work, (void*)work_count, (void*)overflow})
+    for (void* p : {(void*)ckpt, (void*)final_rgba, (void*)work})
       if (p) cudaFree(p);
     *this = TrainState();
   }
@@ -74,6 +72,29 @@ struct DeviceBuffer {
   }
 };
 
+// Page-locked host memory, mapped into the device.
+struct PinnedBuffer {
+  void* ptr = nullptr;
+  size_t bytes = 0;
+  cudaError_t ensure(size_t want) {
+    if (want <= bytes) return cudaSuccess;
+    release();
+    cudaError_t e = cudaHostAlloc(&ptr, want, cudaHostAllocMapped);
+    if (e == cudaSuccess) bytes = want;
+    return e;
+  }
+  void* device() const {
+    void* d = nullptr;
+    if (cudaHostGetDevicePointer(&d, ptr, 0) != cudaSuccess) cudaGetLastError();
+    return d;
+  }
+  void release() {
+    if (ptr) cudaFreeHost(ptr);
+    ptr = nullptr;
+    bytes = 0;
+  }
+};
+
 bool finite3(const float* v) { return std::isfinite(v[0]) && std::isfinite(v[1]) && std::isfinite(v[2]); }
 
 bool is_device_pointer(const void* p) {
@@ -103,6 +124,13 @@ bool classify_output(void* p, void** pinned_alias) {
 
 }  // namespace
 
+// A view's counters on the device: its two segment lists' lengths, the samples
+// of the all-empty segments (64 bits), and the overflow flag.
+struct TrainCounts {
+  unsigned segments[2], samples[2];
+  int overflow, pad[3];
+};
+
 struct aloha_ctx {
   int device = 0;
   int num_sms = 0;
@@ -116,6 +144,8 @@ struct aloha_ctx {
   std::vector<size_t> brick_offset;  // quad offset of each padded brick in `voxels`
   DeviceBuffer voxels, bricks_dev, staging_in;
   DeviceBuffer scene_inner;  // int: every brick is InnerCoords
+  PinnedBuffer upload_flags;  // int the upload kernel sets (kVoxel*)
+  int* upload_flags_dev = nullptr;
   int scene_inner_host = 0;
   float bounds_lo[3] = {0, 0, 0}, bounds_hi[3] = {0, 0, 0};
   // transfer function
@@ -123,7 +153,7 @@ struct aloha_ctx {
   int n_tf = 0;
   // empty-space macrocells: value range per macrocell (per brick) and the
   // per-transfer-function empty mask, refreshed before the next render
-  DeviceBuffer mc_ranges, mc_codes, tf_prefix;
+  DeviceBuffer mc_ranges, mc_codes;
   std::vector<size_t> mc_offset;
   size_t mc_total = 0;
   bool empty_dirty = true;
@@ -139,8 +169,12 @@ struct aloha_ctx {
   int sched_stride = 0;  // ints per view slot
   // params, scratch
   aloha_render_params params;
-  DeviceBuffer counter, flag, staging_out, work, grad4;
+  DeviceBuffer counter, staging_out, work, grad4;
   DeviceBuffer train_tables;  // per launch of the differentiable form: item counter, views, runs
+  // Counters of every view's last training forward (TrainCounts), in one array
+  // so that a call clears and reads its views' in one operation each.
+  DeviceBuffer train_counts;
+  PinnedBuffer counts_host;
   // every byte of grad4 is zero once the stream reaches the last fold (the
   // fold clears the quads it reads); false after a reallocation or a backward
   // that returned before its fold was enqueued
@@ -309,7 +343,9 @@ bool view_inner(const ViewState& v) {
 }
 
 // Upload dirty view state (camera, size, schedule) for `view` on `s`.
-int prepare_view(aloha_ctx* c, int view, cudaStream_t s) {
+// *enqueued (if given) tells whether anything was put on the stream.
+int prepare_view(aloha_ctx* c, int view, cudaStream_t s, bool* enqueued = nullptr) {
+  if (enqueued) *enqueued = false;
   if (c->descs.empty()) return c->fail(ALOHA_ERR_NOT_READY, "no bricks uploaded");
   if (c->n_tf == 0) return c->fail(ALOHA_ERR_NOT_READY, "no transfer function set");
   if (view < 0 || view >= (int)c->views.size()) return c->fail(ALOHA_ERR_OUT_OF_RANGE, "view %d has no state", view);
@@ -319,12 +355,13 @@ int prepare_view(aloha_ctx* c, int view, cudaStream_t s) {
   for (size_t b = 0; b < c->brick_present.size(); ++b)
     if (!c->brick_present[b]) return c->fail(ALOHA_ERR_MISSING_BRICK, "brick %zu has no data (dropped)", b);
   if (c->empty_dirty) {
+    if (enqueued) *enqueued = true;
     int most = 0;
     for (const DevBrick& b : c->dev_bricks) most = std::max(most, macrocells(b));
     uint8_t* codes = static_cast<uint8_t*>(c->mc_codes.ptr);
     CUDA_TRY(c, launch_macrocell_codes(static_cast<const DevBrick*>(c->bricks_dev.ptr), (int)c->dev_bricks.size(), most,
                                        static_cast<const float2*>(c->mc_ranges.ptr),
-                                       static_cast<const int*>(c->tf_prefix.ptr), c->n_tf, codes, codes + c->mc_total,
+                                       reinterpret_cast<const int*>(static_cast<const float*>(c->tf.ptr) + 4 * (size_t)c->n_tf), c->n_tf, codes, codes + c->mc_total,
                                        s));
     c->empty_dirty = false;
   }
@@ -336,6 +373,7 @@ int prepare_view(aloha_ctx* c, int view, cudaStream_t s) {
     for (auto& vv : c->views) vv.dirty = true;
   }
   if (!v.dirty) return ALOHA_OK;
+  if (enqueued) *enqueued = true;
   if (!c->order_cache_valid) {
     c->order_cache = build_order_cache(c->boxes, c->brick_rank, c->n_ranks);
     c->order_cache_valid = true;
@@ -790,7 +828,8 @@ int aloha_create(int device, aloha_ctx** out) {
   c->num_sms = prop.multiProcessorCount;
   aloha_default_render_params(&c->params);
   if (c->views_dev.ensure(sizeof(DevView) * kMaxViews) != cudaSuccess ||
-      c->counter.ensure(sizeof(unsigned long long)) != cudaSuccess || c->flag.ensure(sizeof(int)) != cudaSuccess ||
+      c->counter.ensure(sizeof(unsigned long long)) != cudaSuccess || c->upload_flags.ensure(sizeof(int)) != cudaSuccess ||
+      !(c->upload_flags_dev = static_cast<int*>(c->upload_flags.device())) ||
       c->work.ensure(sizeof(unsigned int)) != cudaSuccess || c->scene_inner.ensure(sizeof(int)) != cudaSuccess ||
       cudaMemset(c->scene_inner.ptr, 0, sizeof(int)) != cudaSuccess) {
     delete c;
@@ -809,10 +848,12 @@ int aloha_destroy(aloha_ctx* c) {
     v.train.release();
   }
   for (DeviceBuffer* b : {&c->voxels, &c->bricks_dev, &c->scene_inner, &c->staging_in, &c->tf, &c->views_dev, &c->sched_dev,
-                          &c->counter, &c->flag, &c->staging_out, &c->mc_ranges, &c->mc_codes, &c->tf_prefix,
+                          &c->counter, &c->staging_out, &c->mc_ranges, &c->mc_codes,
                           &c->work, &c->grad4, &c->split_images, &c->split_masks, &c->split_items,
-                          &c->split_done, &c->chunk_order})
+                          &c->split_done, &c->chunk_order, &c->train_tables, &c->train_counts})
     b->release();
+  c->counts_host.release();
+  c->upload_flags.release();
   delete c;
   return ALOHA_OK;
 }
@@ -852,12 +893,15 @@ static int upload_brick(aloha_ctx* c, int b, const float* src) {
   }
   DevBrick& db = c->dev_bricks[b];
   float4* alloc = static_cast<float4*>(c->voxels.ptr) + c->brick_offset[b];
-  CUDA_TRY(c, cudaMemset(c->flag.ptr, 0, sizeof(int)));
+  // The kernel sets flags in page-locked memory: nothing to clear or copy back
+  // on the device, one wait.
+  volatile int* flags_host = static_cast<volatile int*>(c->upload_flags.ptr);
+  *flags_host = 0;
   CUDA_TRY(c, launch_fill_brick(db, dsrc, alloc, static_cast<float2*>(c->mc_ranges.ptr) + c->mc_offset[b],
-                                static_cast<int*>(c->flag.ptr), 0));
+                                c->upload_flags_dev, 0));
   c->empty_dirty = true;
-  int flags = 0;  // this copy also waits for the kernel above
-  CUDA_TRY(c, cudaMemcpy(&flags, c->flag.ptr, sizeof(int), cudaMemcpyDeviceToHost));
+  CUDA_TRY(c, cudaStreamSynchronize(0));
+  const int flags = *flags_host;
   if (flags & kVoxelNonfinite) return c->fail(ALOHA_ERR_INVALID_ARGUMENT, "brick %d holds a non-finite voxel", b);
   const int inner = c->brick_inner_box[b] && !(flags & kVoxelWide);
   db.inner = inner;
@@ -989,13 +1033,17 @@ int aloha_set_transfer_function(aloha_ctx* c, const float* rgba, int n) {
   for (float v : h)
     if (!std::isfinite(v)) return c->fail(ALOHA_ERR_INVALID_ARGUMENT, "transfer function holds a non-finite value");
   CUDA_TRY(c, cudaDeviceSynchronize());
+  // the table, then the prefix counts of its entries with non-zero alpha (for
+  // the macrocell codes), in one copy
+  const size_t entries = h.size();
+  h.resize(entries + n + 1);
+  int count = 0;
+  for (int i = 0; i <= n; ++i) {
+    std::memcpy(&h[entries + i], &count, sizeof count);
+    if (i < n && h[(size_t)i * 4 + 3] != 0.0f) ++count;
+  }
   CUDA_TRY(c, c->tf.ensure(h.size() * sizeof(float)));
   CUDA_TRY(c, cudaMemcpy(c->tf.ptr, h.data(), h.size() * sizeof(float), cudaMemcpyHostToDevice));
-  // prefix counts of entries with non-zero alpha, for the empty-space masks
-  std::vector<int> prefix(n + 1, 0);
-  for (int i = 0; i < n; ++i) prefix[i + 1] = prefix[i] + (h[(size_t)i * 4 + 3] != 0.0f ? 1 : 0);
-  CUDA_TRY(c, c->tf_prefix.ensure(prefix.size() * sizeof(int)));
-  CUDA_TRY(c, cudaMemcpy(c->tf_prefix.ptr, prefix.data(), prefix.size() * sizeof(int), cudaMemcpyHostToDevice));
   c->empty_dirty = true;
   c->n_tf = n;
   invalidate_training(c);
@@ -1068,9 +1116,11 @@ int aloha_resize(aloha_ctx* c, int view, int width, int height) {
 int aloha_get_composite_order(aloha_ctx* c, int view, int* rank_order, int max_ranks, int* n_ranks) {
   if (!c || !rank_order || !n_ranks) return ALOHA_ERR_NULL_POINTER;
   CUDA_TRY(c, cudaSetDevice(c->device));
-  int rc = prepare_view(c, view, 0);
+  bool enqueued = false;
+  int rc = prepare_view(c, view, 0, &enqueued);
   if (rc) return rc;
-  CUDA_TRY(c, cudaStreamSynchronize(0));
+  // what was put on the default stream has to be there for launches on any other
+  if (enqueued) CUDA_TRY(c, cudaStreamSynchronize(0));
   const std::vector<int>& o = c->views[view].sched.rank_order;
   if ((int)o.size() > max_ranks) return c->fail(ALOHA_ERR_INVALID_ARGUMENT, "order needs %zu entries", o.size());
   std::copy(o.begin(), o.end(), rank_order);
@@ -1220,6 +1270,23 @@ static int composite_common(const void* imgs, size_t img_bytes, const int* order
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const size_t npx = (size_t)width * height;
   const bool host_in = !is_device_pointer(imgs), host_out = !is_device_pointer(fb);
+  if (!host_in && !host_out && n_ranks <= kParamRanks) {
+    // device images and frame buffer: the order goes in the launch parameters,
+    // nothing is allocated and nothing waits (a stream under capture is refused
+    // below, as the allocation has always done)
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
+      cudaGetLastError();
+      cs = cudaStreamCaptureStatusActive;
+    }
+    if (cs == cudaStreamCaptureStatusNone) {
+      const cudaError_t e =
+          u8 ? launch_composite_u8(static_cast<const uint32_t*>(imgs), nullptr, h_order.data(), n_ranks, (int)npx, fb, s)
+             : launch_composite_f32(static_cast<const float4*>(imgs), nullptr, h_order.data(), n_ranks, (int)npx, mode, fb,
+                                    s);
+      return e == cudaSuccess ? ALOHA_OK : ALOHA_ERR_CUDA;
+    }
+  }
   void* d_in = nullptr;
   uint32_t* d_out = nullptr;
   int* d_order = nullptr;
@@ -1245,8 +1312,8 @@ static int composite_common(const void* imgs, size_t img_bytes, const int* order
       if (cudaMalloc(&d_out, npx * sizeof(uint32_t)) != cudaSuccess) { fail(ALOHA_ERR_OUT_OF_MEMORY); break; }
       out = d_out;
     }
-    cudaError_t e = u8 ? launch_composite_u8(static_cast<const uint32_t*>(in), d_order, n_ranks, (int)npx, out, s)
-                       : launch_composite_f32(static_cast<const float4*>(in), d_order, n_ranks, (int)npx, mode, out, s);
+    cudaError_t e = u8 ? launch_composite_u8(static_cast<const uint32_t*>(in), d_order, nullptr, n_ranks, (int)npx, out, s)
+                       : launch_composite_f32(static_cast<const float4*>(in), d_order, nullptr, n_ranks, (int)npx, mode, out, s);
     if (e != cudaSuccess) { fail(ALOHA_ERR_CUDA); break; }
     if (host_out && cudaMemcpyAsync(fb, out, npx * sizeof(uint32_t), cudaMemcpyDeviceToHost, s) != cudaSuccess) {
       fail(ALOHA_ERR_CUDA);
@@ -1330,13 +1397,28 @@ bool train_inner(const aloha_ctx* c, int n_views, const int* view_ids) {
   return true;
 }
 
-TrainView train_view(const TrainState& t, int view) {
+// Runs [first, last] of consecutive views among `views`.
+std::vector<std::pair<int, int>> view_runs(int n_views, const int* views) {
+  std::vector<int> v(views, views + n_views);
+  std::sort(v.begin(), v.end());
+  std::vector<std::pair<int, int>> runs;
+  for (int x : v) {
+    if (!runs.empty() && x <= runs.back().second + 1)
+      runs.back().second = x;
+    else
+      runs.push_back({x, x});
+  }
+  return runs;
+}
+
+TrainView train_view(const aloha_ctx* c, const TrainState& t, int view) {
   TrainView tv{};
   tv.ckpt = t.ckpt;
   tv.final_rgba = t.final_rgba;
   tv.work = t.work;
-  tv.work_count = t.work_count;
-  tv.overflow = t.overflow;
+  TrainCounts* counts = static_cast<TrainCounts*>(c->train_counts.ptr) + view;
+  tv.work_count = counts->segments;
+  tv.overflow = &counts->overflow;
   tv.ckpt_cap = t.cap;
   tv.work_cap = (unsigned)std::min<size_t>(t.npx * t.cap, 0xffffffffu);
   tv.view = view;
@@ -1391,6 +1473,7 @@ int forward_views(aloha_ctx* c, int n_views, const int* view_ids, float* const* 
   const unsigned cap = checkpoint_capacity(c, k);
   std::vector<TrainView> tvs(n_views);
   std::vector<char> host_out(n_views, 0);
+  CUDA_TRY(c, c->train_counts.ensure(sizeof(TrainCounts) * kMaxViews));
   for (int i = 0; i < n_views; ++i) {
     const int view = view_ids[i];
     rc = prepare_view(c, view, s);
@@ -1412,20 +1495,19 @@ int forward_views(aloha_ctx* c, int n_views, const int* view_ids, float* const* 
       CUDA_TRY(c, cudaMalloc(&t.ckpt, npx * cap * sizeof(Checkpoint)));
       CUDA_TRY(c, cudaMalloc(&t.work, npx * cap * sizeof(uint2)));
       CUDA_TRY(c, cudaMalloc(&t.final_rgba, npx * sizeof(float4)));
-      CUDA_TRY(c, cudaMalloc(&t.work_count, 4 * sizeof(unsigned)));
-      CUDA_TRY(c, cudaMalloc(&t.overflow, sizeof(int)));
       t.npx = npx;
       t.cap = cap;
       t.bytes = need;
     }
     t.k = k;
-    tvs[i] = train_view(t, view);
+    tvs[i] = train_view(c, t, view);
     host_out[i] = !is_device_pointer(rgba[i]);
     tvs[i].out_rgba = host_out[i] ? nullptr : reinterpret_cast<float4*>(rgba[i]);
-    CUDA_TRY(c, cudaMemsetAsync(t.work_count, 0, 4 * sizeof(unsigned), s));
-    CUDA_TRY(c, cudaMemsetAsync(t.overflow, 0, sizeof(int), s));
     tvs[i].n_chunks = ring_slots(v.width, v.height, 8, 4);
   }
+  for (const auto& run : view_runs(n_views, view_ids))
+    CUDA_TRY(c, cudaMemsetAsync(static_cast<TrainCounts*>(c->train_counts.ptr) + run.first, 0,
+                                sizeof(TrainCounts) * (run.second - run.first + 1), s));
   if (n_views == 1) {
     const int* order = nullptr;
     int chunks = 0;
@@ -1533,22 +1615,20 @@ int backward_views(aloha_ctx* c, int n_views, const int* view_ids, const float* 
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   CUDA_TRY(c, cudaSetDevice(c->device));
-  // every view's overflow flag and segment count, read with one wait
-  std::vector<int> overflow(n_views, 0);
-  std::vector<unsigned> segments(2 * (size_t)n_views, 0);  // per view: with full samples, all-empty
-  for (int i = 0; i < n_views; ++i) {
-    const TrainState& t = c->views[view_ids[i]].train;
-    CUDA_TRY(c, cudaMemcpyAsync(&overflow[i], t.overflow, sizeof(int), cudaMemcpyDeviceToHost, s));
-    CUDA_TRY(c, cudaMemcpyAsync(&segments[2 * (size_t)i], t.work_count, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost,
-                                s));
-  }
+  // every view's overflow flag and segment counts, read with one wait
+  CUDA_TRY(c, c->counts_host.ensure(sizeof(TrainCounts) * kMaxViews));
+  TrainCounts* counts = static_cast<TrainCounts*>(c->counts_host.ptr);
+  for (const auto& run : view_runs(n_views, view_ids))
+    CUDA_TRY(c, cudaMemcpyAsync(counts + run.first, static_cast<TrainCounts*>(c->train_counts.ptr) + run.first,
+                                sizeof(TrainCounts) * (run.second - run.first + 1), cudaMemcpyDeviceToHost, s));
   CUDA_TRY(c, cudaStreamSynchronize(s));
   unsigned long long all_segments = 0;
   for (int i = 0; i < n_views; ++i) {
-    if (overflow[i])
+    const TrainCounts& n = counts[view_ids[i]];
+    if (n.overflow)
       return c->fail(ALOHA_ERR_OUT_OF_RANGE, "a ray of view %d needed more checkpoints than reserved", view_ids[i]);
     // the two lists share t.npx * t.cap entries
-    all_segments += (unsigned long long)segments[2 * (size_t)i] + segments[2 * (size_t)i + 1];
+    all_segments += (unsigned long long)n.segments[0] + n.segments[1];
     if (all_segments >= 0xffffffffull)
       return c->fail(ALOHA_ERR_UNSUPPORTED, "too many checkpoint segments in one backward");
   }
@@ -1604,12 +1684,12 @@ int backward_views(aloha_ctx* c, int n_views, const int* view_ids, const float* 
     for (int i = first; i < n_views; ++i) {
       if (done[i] || c->views[view_ids[i]].train.k != k) continue;
       done[i] = 1;
-      TrainView tv = train_view(c->views[view_ids[i]].train, view_ids[i]);
+      TrainView tv = train_view(c, c->views[view_ids[i]].train, view_ids[i]);
       tv.dl_drgba = off_dl[i] != SIZE_MAX ? reinterpret_cast<const float4*>(st + off_dl[i])
                                           : reinterpret_cast<const float4*>(dl_drgba[i]);
       tvs.push_back(tv);
-      base.push_back(base.back() + segments[2 * (size_t)i]);
-      empty_base.push_back(empty_base.back() + segments[2 * (size_t)i + 1]);
+      base.push_back(base.back() + counts[view_ids[i]].segments[0]);
+      empty_base.push_back(empty_base.back() + counts[view_ids[i]].segments[1]);
     }
     std::vector<char*> dev;
     rc = upload_train_tables(c, {{tvs.data(), tvs.size() * sizeof(TrainView)},

@@ -203,10 +203,13 @@ __host__ __device__ inline int ring_slots(int width, int height, int cw, int ch)
   return (2 * r + 1) * (2 * r + 1);
 }
 constexpr int kRenderThreads = 128;
-cudaError_t launch_composite_f32(const float4* imgs, const int* order, int n_ranks, int npx, int mode, uint32_t* fb,
-                                 cudaStream_t s);
-cudaError_t launch_composite_u8(const uint32_t* imgs, const int* order, int n_ranks, int npx, uint32_t* fb,
-                                cudaStream_t s);
+// Ordered composite; the order is in device memory, or, up to kParamRanks
+// ranks, in host memory and passed with the launch.
+constexpr int kParamRanks = 1024;
+cudaError_t launch_composite_f32(const float4* imgs, const int* order, const int* host_order, int n_ranks, int npx,
+                                 int mode, uint32_t* fb, cudaStream_t s);
+cudaError_t launch_composite_u8(const uint32_t* imgs, const int* order, const int* host_order, int n_ranks, int npx,
+                                uint32_t* fb, cudaStream_t s);
 // Fills a brick's padded array from its voxels (x fastest) and the value range
 // of each macrocell.  Sets flag bits: kVoxelNonfinite, kVoxelWide (a value
 // beyond +-kInnerValue).

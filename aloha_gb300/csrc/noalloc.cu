@@ -103,7 +103,7 @@ extern "C" int aloha_composite_over_noalloc(const float* rank_images, const int*
   // pageable source: staged by the runtime before the call returns
   if (cudaMemcpyAsync(d_order, snapshot, sizeof(int) * (size_t)n_ranks, cudaMemcpyHostToDevice, s) != cudaSuccess)
     return ALOHA_ERR_CUDA;
-  if (launch_composite_f32(reinterpret_cast<const float4*>(rank_images), d_order, n_ranks, width * height, mode, fb,
+  if (launch_composite_f32(reinterpret_cast<const float4*>(rank_images), d_order, nullptr, n_ranks, width * height, mode, fb,
                            s) != cudaSuccess)
     return ALOHA_ERR_CUDA;
   return ALOHA_OK;

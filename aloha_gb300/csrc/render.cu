@@ -351,24 +351,38 @@ __global__ void __launch_bounds__(kRenderThreads, MINB) render_split_kernel(Spli
   count_samples(s.f.counter, n);
 }
 
+// The order of a composite: from device memory, or from the launch parameters.
+struct MemoryOrder {
+  const int* r;
+  __device__ __forceinline__ int operator[](int k) const { return __ldg(r + k); }
+};
+struct ParamOrder {
+  uint16_t r[kParamRanks];
+  __device__ __forceinline__ int operator[](int k) const { return r[k]; }
+};
+
 // Ordered "over" of per-rank float images (IceT BLEND with ORDERED_COMPOSITE,
 // waikikiRenderer.cpp:910-917,1042-1079), front to back.
-__global__ void composite_f32_kernel(const float4* __restrict__ imgs, const int* __restrict__ order, int n_ranks,
+template <class Order>
+__global__ void composite_f32_kernel(const float4* __restrict__ imgs, const __grid_constant__ Order order, int n_ranks,
                                      int npx, int mode, uint32_t* __restrict__ fb) {
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npx; p += gridDim.x * blockDim.x) {
     OverBlend blend;
-    for (int k = 0; k < n_ranks; ++k) blend.add(mode, __ldg(imgs + (size_t)__ldg(order + k) * npx + p));
+#pragma unroll 4
+    for (int k = 0; k < n_ranks; ++k) blend.add(mode, __ldg(imgs + (size_t)order[k] * npx + p));
     fb[p] = blend.pack(mode);
   }
 }
 
 // 8-bit ordered over of external RGBA8 rank images.
-__global__ void composite_u8_kernel(const uint32_t* __restrict__ imgs, const int* __restrict__ order, int n_ranks,
-                                    int npx, uint32_t* __restrict__ fb) {
+template <class Order>
+__global__ void composite_u8_kernel(const uint32_t* __restrict__ imgs, const __grid_constant__ Order order,
+                                    int n_ranks, int npx, uint32_t* __restrict__ fb) {
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npx; p += gridDim.x * blockDim.x) {
     uint32_t c8[4] = {0u, 0u, 0u, 0u};
+#pragma unroll 4
     for (int k = 0; k < n_ranks; ++k) {
-      const uint32_t q = __ldg(imgs + (size_t)__ldg(order + k) * npx + p);
+      const uint32_t q = __ldg(imgs + (size_t)order[k] * npx + p);
       const uint32_t f = 255u - c8[3];
 #pragma unroll
       for (int ch = 0; ch < 4; ++ch) c8[ch] = min(255u, c8[ch] + (((q >> (8 * ch)) & 255u) * f + 127u) / 255u);
@@ -380,7 +394,7 @@ __global__ void composite_u8_kernel(const uint32_t* __restrict__ imgs, const int
 // Fills a brick's padded array: element (x,y,z) holds V(x,y,z), V(x,y,z+1),
 // V(x,y+1,z), V(x,y+1,z+1) with every index clamped to the brick (the apron and
 // the quads' far rows and slices repeat edge values); flags non-finite voxels
-// and values too large for InnerCoords; and takes each macrocell's value range:
+// and values too large for InnerCoords (in page-locked host memory); and takes each macrocell's value range:
 // a sample whose value-tap cell is c (c = clamp(floor(u), 0, n-1)) reads voxels
 // c and c+1 (clamped), so macrocell m covers voxels [m*kMacro, m*kMacro +
 // kMacro] per axis.  A CTA takes kMacro rows of kMacro slices, each thread one
@@ -447,7 +461,7 @@ __global__ void __launch_bounds__(kFillThreads) fill_brick_kernel(const float* _
       }
     }
   }
-  if (bad || wide) atomicOr(flags, (bad ? kVoxelNonfinite : 0) | (wide ? kVoxelWide : 0));
+  if (bad || wide) atomicOr_system(flags, (bad ? kVoxelNonfinite : 0) | (wide ? kVoxelWide : 0));
 }
 
 // Macrocell codes.  A macrocell is empty when every transfer-function entry
@@ -626,15 +640,33 @@ static int composite_grid(int npx) {
   return g < 1 ? 1 : (g > 152 * 16 ? 152 * 16 : g);
 }
 
-cudaError_t launch_composite_f32(const float4* imgs, const int* order, int n_ranks, int npx, int mode, uint32_t* fb,
-                                 cudaStream_t s) {
-  composite_f32_kernel<<<composite_grid(npx), 256, 0, s>>>(imgs, order, n_ranks, npx, mode, fb);
+static bool param_order(const int* host_order, int n_ranks, ParamOrder& o) {
+  if (!host_order || n_ranks > kParamRanks) return false;
+  for (int k = 0; k < n_ranks; ++k) o.r[k] = (uint16_t)host_order[k];
+  return true;
+}
+
+cudaError_t launch_composite_f32(const float4* imgs, const int* order, const int* host_order, int n_ranks, int npx,
+                                 int mode, uint32_t* fb, cudaStream_t s) {
+  ParamOrder o;
+  if (order)
+    composite_f32_kernel<<<composite_grid(npx), 256, 0, s>>>(imgs, MemoryOrder{order}, n_ranks, npx, mode, fb);
+  else if (param_order(host_order, n_ranks, o))
+    composite_f32_kernel<<<composite_grid(npx), 256, 0, s>>>(imgs, o, n_ranks, npx, mode, fb);
+  else
+    return cudaErrorInvalidValue;
   return cudaGetLastError();
 }
 
-cudaError_t launch_composite_u8(const uint32_t* imgs, const int* order, int n_ranks, int npx, uint32_t* fb,
-                                cudaStream_t s) {
-  composite_u8_kernel<<<composite_grid(npx), 256, 0, s>>>(imgs, order, n_ranks, npx, fb);
+cudaError_t launch_composite_u8(const uint32_t* imgs, const int* order, const int* host_order, int n_ranks, int npx,
+                                uint32_t* fb, cudaStream_t s) {
+  ParamOrder o;
+  if (order)
+    composite_u8_kernel<<<composite_grid(npx), 256, 0, s>>>(imgs, MemoryOrder{order}, n_ranks, npx, fb);
+  else if (param_order(host_order, n_ranks, o))
+    composite_u8_kernel<<<composite_grid(npx), 256, 0, s>>>(imgs, o, n_ranks, npx, fb);
+  else
+    return cudaErrorInvalidValue;
   return cudaGetLastError();
 }
 
