@@ -114,18 +114,12 @@ __device__ __forceinline__ uint32_t walk_samples(const TrainArgs& a, const DevVi
                                    inv_d[1], inv_d[2], eps, t1);
         if (!cell.empty()) {
           t_cell = tb;
-        } else if (exact) {
+        } else {
           ++n;
           ++nb;
           t = t + dt;
-          n += run_steps(t, nb, tb, cap, dt, inv_dt, max_samples - n);
-          continue;
-        } else {
-          do {
-            ++n;
-            ++nb;
-            t = t + dt;
-          } while (t < tb && nb < cap && n != max_samples);
+          n += exact ? run_steps(t, nb, tb, cap, dt, inv_dt, max_samples - n)
+                     : run_steps_any(t, nb, tb, cap, dt, max_samples - n);
           continue;
         }
       }

@@ -516,8 +516,8 @@ __device__ __forceinline__ uint32_t march_brick(const DevBrick& b, const float4*
     // a full macrocell.  A sample in an empty one has alpha exactly 0 and leaves
     // the colour unchanged, so only t and the sample count advance (the same t
     // += dt sequence as full samples) up to the box's end.  The first is always
-    // taken.  With exact steps the rest of the run is one jump (one more per
-    // power of two it crosses, and one per checkpoint the hook needs).
+    // taken.  The rest of the run is one jump (one more per power of two it
+    // crosses, and one per checkpoint the hook needs).
     int jumps = 0;
     for (; jumps < kMarchJumps && t < t1 && n < cap; ++jumps) {
       const Cell cell = cell_at(cells, mnx, mny, nx, ny, nz, fmaf(t, r.d[0], r.o[0]) - lox,
@@ -528,14 +528,10 @@ __device__ __forceinline__ uint32_t march_brick(const DevBrick& b, const float4*
       ++n;
       t = t + dt;
       if constexpr (!Hook::kActive) {
-        if (exact) {
+        if (exact)
           run_steps(t, n, tb, cap, dt, inv_dt, 0xffffffffu);
-        } else {
-          while (t < tb && n < cap) {
-            ++n;
-            t = t + dt;
-          }
-        }
+        else
+          run_steps_any(t, n, tb, cap, dt, 0xffffffffu);
       } else if (exact) {
         for (;;) {
           hook.left -= run_steps(t, n, tb, cap, dt, inv_dt, hook.left);
@@ -545,6 +541,8 @@ __device__ __forceinline__ uint32_t march_brick(const DevBrick& b, const float4*
           t = t + dt;
         }
       } else {
+        // step by step: a second jump form in here cost the training forward
+        // of the exact steps 4 % (16 views of 128^3 at 256^2)
         while (t < tb && n < cap) {
           uint32_t k = hook.left;
           while (k > 0 && t < tb && n < cap) {
@@ -665,14 +663,10 @@ __device__ __forceinline__ uint32_t march_brick_group(const DevBrick& b, const f
       if (cell.empty()) {
         ++n;
         t = t + dt;
-        if (exact) {
+        if (exact)
           run_steps(t, n, tb, cap, dt, inv_dt, 0xffffffffu);
-          continue;
-        }
-        while (t < tb && n < cap) {
-          ++n;
-          t = t + dt;
-        }
+        else
+          run_steps_any(t, n, tb, cap, dt, 0xffffffffu);
         continue;
       }
       t_cell = tb;

@@ -122,4 +122,59 @@ ALOHA_HD uint32_t run_steps(float& t, uint32_t& n, float tb, uint32_t cap, float
   return k;
 }
 
+// Quotient that only estimates a step count.
+ALOHA_HD float estimate_div(float a, float b) {
+#ifdef __CUDA_ARCH__
+  return __fdividef(a, b);
+#else
+  return a / b;
+#endif
+}
+
+// run_steps for any dt.  Within a binade of spacing u every t is a multiple of
+// u, so t + dt rounds to t plus one fixed multiple of u, unless dt lies halfway
+// between two multiples: then the sum rounds to an even one, and from an even t
+// on the step is fixed again.  Two equal steps in a row (t to t1, t1 to t1 +
+// dt) therefore stay equal up to the binade's end; otherwise, and across the
+// end, single steps are taken as the loop takes them.  A 200^3 volume at
+// 700x400 and dt 0.3: 300 us with the loop, 276 this way, 267 at dt 0.3125
+// (run_steps).
+ALOHA_HD uint32_t run_steps_any(float& t, uint32_t& n, float tb, uint32_t cap, float dt, uint32_t max_steps) {
+  uint32_t k = 0;
+  while (k < max_steps && t < tb && n < cap) {
+    const uint32_t lim = (max_steps - k) < (cap - n) ? (max_steps - k) : (cap - n);
+    const float t1 = t + dt;
+    const float step = t1 - t;
+    if (step > 0.0f && (t1 + dt) - t1 == step) {
+      const float d = t - bits_float((float_bits(t) & 0x7f800000u) + 0x00800000u);  // t - B, exact, < 0
+      const float kf = fminf(fmaxf(ceilf(estimate_div(tb - t, step)), 1.0f), 4194304.0f);
+      uint32_t j = (uint32_t)kf < lim ? (uint32_t)kf : lim;
+      while (j > 1u && !(fmaf((float)(j - 1u), step, t) < tb)) --j;
+      while (j < lim && j < 4194304u && fmaf((float)j, step, t) < tb) ++j;
+      if (fmaf((float)j, step, d) <= 0.0f) {  // up to B, the steps and their sums are exact
+        t = fmaf((float)j, step, t);
+        n += j;
+        k += j;
+        continue;
+      }
+      const float jf = fminf(fmaxf(floorf(estimate_div(-d, step)), 0.0f), 4194304.0f);
+      uint32_t jb = (uint32_t)jf < lim ? (uint32_t)jf : lim;
+      while (jb > 0u && fmaf((float)jb, step, d) > 0.0f) --jb;
+      while (jb < lim && fmaf((float)(jb + 1u), step, d) <= 0.0f) ++jb;
+      t = fmaf((float)jb, step, t);
+      n += jb;
+      k += jb;
+      if (jb == lim) break;
+      t = t + dt;  // the crossing step
+      ++n;
+      ++k;
+      continue;
+    }
+    t = t1;
+    ++n;
+    ++k;
+  }
+  return k;
+}
+
 }  // namespace aloha
