@@ -549,7 +549,7 @@ int plan_chunk_order(aloha_ctx* c, const FrameArgs& f, int view, int cw, int ch,
   o.ch = ch;
   o.n_slots = ring_slots(v.width, v.height, cw, ch);
   const size_t n_chunks = (size_t)((v.width + cw - 1) / cw) * ((v.height + ch - 1) / ch);
-  const size_t slots = (size_t)o.n_slots, hist = (size_t)kOrderClasses * chunk_order_blocks(o.n_slots);
+  const size_t slots = (size_t)o.n_slots, hist = (size_t)kOrderClasses * chunk_order_blocks(o.n_slots) + 1;
   const size_t key_words = (slots + 3) / 4;  // uint8 keys, padded to whole words
   const size_t before = c->chunk_order.bytes;
   CUDA_TRY(c, c->chunk_order.ensure((key_words + slots + hist + n_chunks) * sizeof(uint32_t)));
@@ -557,6 +557,7 @@ int plan_chunk_order(aloha_ctx* c, const FrameArgs& f, int view, int cw, int ch,
   o.key = reinterpret_cast<uint8_t*>(w);
   o.cid = reinterpret_cast<int*>(w + key_words);
   o.hist = w + key_words + slots;
+  o.readers = o.hist + hist - 1;
   o.order = reinterpret_cast<int*>(w + key_words + slots + hist);
   o.n_chunks = (int)n_chunks;
   // the histogram is zero between launches of one layout (the scatter clears
@@ -645,7 +646,7 @@ int launch_single(aloha_ctx* c, const FrameArgs& f, int view, cudaStream_t s) {
   const int warps_per_block = kRenderThreads / 32;
   const int grid = std::max(1, std::min(lane_groups ? c->grid_blocks_lg : c->grid_blocks,
                                         (b.total_tiles + warps_per_block - 1) / warps_per_block));
-  CUDA_TRY(c, launch_render_warps(b, cw, ch, grid, false, s, c->staging, lane_groups, few));
+  CUDA_TRY(c, launch_render_warps(b, cw, ch, grid, false, s, c->staging, lane_groups, few, order != nullptr));
   return ALOHA_OK;
 }
 

@@ -153,7 +153,8 @@ struct ChunkOrderArgs {
   int n_slots;       // ring slots of the chunk grid (the probe's input order)
   uint8_t* key;      // [n_slots] cost class per slot (0xff off the grid)
   int* cid;          // [n_slots] chunk id per slot
-  uint32_t* hist;    // [kOrderClasses][chunk_order_blocks(n_slots)] counts, then offsets; zero between launches
+  uint32_t* hist;    // [kOrderClasses][chunk_order_blocks(n_slots)] counts; zero between launches
+  uint32_t* readers; // the word after hist: scatter CTAs that have read it; zero between launches
   int* order;        // [chunks] chunk ids, most expensive first
   int n_chunks;      // chunks of the grid (entries of `order`)
   // counters of the render launch that follows, zeroed by the probe (or null)
@@ -161,6 +162,26 @@ struct ChunkOrderArgs {
   unsigned long long* zero_samples;
 };
 int chunk_order_blocks(int n_slots);
+
+// Programmatic dependent launch: `beside` lets the kernel start before the
+// stream's previous kernel has finished (once all its CTAs have called
+// launch_dependents or ended); it waits for that kernel's results with
+// wait_for_primary (at once when launched in the ordinary way).
+template <class... Args>
+cudaError_t launch_beside(void (*kernel)(Args...), int grid, int threads, size_t smem, cudaStream_t s, bool beside,
+                          Args... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = beside ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
 cudaError_t launch_chunk_order(const ChunkOrderArgs& a, cudaStream_t s);
 
 // Rank-split render of one view into f.fb: work items are (8x4 chunk, rank)
@@ -236,8 +257,9 @@ constexpr int kStageUnroll2 = 2;
 // `lane_groups`: the instance that renders the first a.group_chunks chunks of
 // the cost order with lane groups (single view, 8x4 chunks, direct loads).
 // `few`: the 8x4 instance for few chunks per warp (single view, direct loads).
+// `beside`: the launch before it in the stream is launch_chunk_order's.
 cudaError_t launch_render_warps(const BatchArgs& a, int chunk_w, int chunk_h, int grid, bool batch, cudaStream_t s,
-                                int stage = ALOHA_STAGING_NONE, bool lane_groups = false, bool few = false);
+                                int stage = ALOHA_STAGING_NONE, bool lane_groups = false, bool few = false, bool beside = false);
 // The macrocell codes of all bricks from their value ranges; prefix[k] = number
 // of transfer-function entries below k with non-zero alpha.  Cells of brick b
 // start at bricks[b].cells - cells in each array; tmp is scratch of their size.

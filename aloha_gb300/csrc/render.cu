@@ -41,6 +41,7 @@ __global__ void __launch_bounds__(kRenderThreads, MINB) render_warps_kernel(Batc
       typename std::conditional<STAGE == kStageUnroll2, UnrolledDirectLoads<2>, DirectLoads>::type>::type;
   Loads loads;
   if constexpr (STAGE == 1) loads.init(tf_s + (b.f.n_tf + 4));
+  wait_for_primary();  // the chunk order and the cleared counters
   const int lane = threadIdx.x & 31;
   uint32_t n = 0;
   for (;;) {
@@ -582,12 +583,11 @@ RenderKernel render_kernel(int chunk_w, int chunk_h, bool batch, int stage, bool
 }  // namespace
 
 cudaError_t launch_render_warps(const BatchArgs& b, int chunk_w, int chunk_h, int grid, bool batch, cudaStream_t s,
-                                int stage, bool lane_groups, bool few) {
+                                int stage, bool lane_groups, bool few, bool beside) {
   if (lane_groups && (!b.chunk_order || b.f.rank_images || b.f.rank_depth || b.f.accum)) return cudaErrorInvalidValue;
   const RenderKernel k = render_kernel(chunk_w, chunk_h, batch, stage, lane_groups, few);
   if (!k) return cudaErrorInvalidValue;
-  k<<<grid, kRenderThreads, render_smem(b.f.n_tf, stage), s>>>(b);
-  return cudaGetLastError();
+  return launch_beside(k, grid, kRenderThreads, render_smem(b.f.n_tf, stage), s, beside, b);
 }
 
 int render_blocks_per_sm(int chunk_w, int chunk_h, int n_tf, bool batch, int stage, bool lane_groups, bool few) {

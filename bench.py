@@ -418,7 +418,7 @@ def main():
     # counts the classes), scan and scatter of the cost order, and for the
     # rank split its mask, three scan kernels and emit
     probed = chunks == abi.CHUNKS_PROBED or (chunks == abi.CHUNKS_AUTO and W * H >= 512 * 512)
-    launches_per_frame = (6 if split == abi.SPLIT_RANKS else 1) + (3 if probed else 0)
+    launches_per_frame = (6 if split == abi.SPLIT_RANKS else 1) + (2 if probed else 0)  # probe and scatter
 
     steps = [mine[k % len(mine)] for k in range(args.steps)]
     for k in range(args.warmup):
