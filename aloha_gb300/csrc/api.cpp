@@ -483,7 +483,7 @@ bool use_rank_split(const aloha_ctx* c, const FrameArgs& f, const ViewState& v) 
 
 int plan_chunk_order(aloha_ctx* c, const FrameArgs& f, int view, int cw, int ch, cudaStream_t s, const int** order,
                      int* chunks, bool auto_order = true, unsigned int* zero_work = nullptr,
-                     unsigned long long* zero_samples = nullptr);
+                     unsigned long long* zero_samples = nullptr, const int** pairs = nullptr);
 
 // Rank-split launch of a single view (mask, plan and render kernels).
 int launch_split(aloha_ctx* c, const FrameArgs& f, int view, cudaStream_t s) {
@@ -533,9 +533,11 @@ int launch_split(aloha_ctx* c, const FrameArgs& f, int view, cudaStream_t s) {
 // The cost-ordered chunk list of a single view when the chunk-order mode asks
 // for one (probe and sort kernels on `s`); *order stays null for ring order.
 // Automatic mode orders frames of 512^2 pixels or more when auto_order is set.
-// The probe also zeroes the given counters (only when *order is set).
+// The probe also zeroes the given counters (only when *order is set).  *pairs:
+// where the order's kernels put BatchArgs::pair_chunks.
 int plan_chunk_order(aloha_ctx* c, const FrameArgs& f, int view, int cw, int ch, cudaStream_t s, const int** order,
-                     int* chunks, bool auto_order, unsigned int* zero_work, unsigned long long* zero_samples) {
+                     int* chunks, bool auto_order, unsigned int* zero_work, unsigned long long* zero_samples,
+                     const int** pairs) {
   const ViewState& v = c->views[view];
   *order = nullptr;
   const bool probed = c->chunk_order_mode == ALOHA_CHUNKS_PROBED ||
@@ -549,7 +551,7 @@ int plan_chunk_order(aloha_ctx* c, const FrameArgs& f, int view, int cw, int ch,
   o.ch = ch;
   o.n_slots = ring_slots(v.width, v.height, cw, ch);
   const size_t n_chunks = (size_t)((v.width + cw - 1) / cw) * ((v.height + ch - 1) / ch);
-  const size_t slots = (size_t)o.n_slots, hist = (size_t)kOrderClasses * chunk_order_blocks(o.n_slots) + 1;
+  const size_t slots = (size_t)o.n_slots, hist = (size_t)kOrderClasses * chunk_order_blocks(o.n_slots) + 2;
   const size_t key_words = (slots + 3) / 4;  // uint8 keys, padded to whole words
   const size_t before = c->chunk_order.bytes;
   CUDA_TRY(c, c->chunk_order.ensure((key_words + slots + hist + n_chunks) * sizeof(uint32_t)));
@@ -557,7 +559,10 @@ int plan_chunk_order(aloha_ctx* c, const FrameArgs& f, int view, int cw, int ch,
   o.key = reinterpret_cast<uint8_t*>(w);
   o.cid = reinterpret_cast<int*>(w + key_words);
   o.hist = w + key_words + slots;
-  o.readers = o.hist + hist - 1;
+  o.readers = o.hist + hist - 2;
+  o.pairs = reinterpret_cast<int*>(o.hist + hist - 1);
+  o.warps = c->num_sms * kFewChunkRenderBlocks * (kRenderThreads / 32);
+  if (pairs) *pairs = o.pairs;
   o.order = reinterpret_cast<int*>(w + key_words + slots + hist);
   o.n_chunks = (int)n_chunks;
   // the histogram is zero between launches of one layout (the scatter clears
@@ -620,12 +625,14 @@ int launch_single(aloha_ctx* c, const FrameArgs& f, int view, cudaStream_t s) {
   b.work_counter = static_cast<unsigned int*>(c->work.ptr);
   int chunks = 0;
   const int* order = nullptr;
-  int rc = plan_chunk_order(c, f, view, cw, ch, s, &order, &chunks, true, b.work_counter, f.counter);
+  int rc = plan_chunk_order(c, f, view, cw, ch, s, &order, &chunks, true, b.work_counter, f.counter,
+                            few ? &b.pair_chunks : nullptr);
   if (rc) return rc;
   if (order) {
     b.chunk_order = order;
     b.total_tiles = chunks;
   } else {
+    b.ring_pairs = few && all_chunks <= kPairRingChunks;
     CUDA_TRY(c, cudaMemsetAsync(c->work.ptr, 0, sizeof(unsigned int), s));
     CUDA_TRY(c, cudaMemsetAsync(f.counter, 0, sizeof(unsigned long long), s));
   }
@@ -644,8 +651,9 @@ int launch_single(aloha_ctx* c, const FrameArgs& f, int view, cudaStream_t s) {
     }
   }
   const int warps_per_block = kRenderThreads / 32;
-  const int grid = std::max(1, std::min(lane_groups ? c->grid_blocks_lg : c->grid_blocks,
-                                        (b.total_tiles + warps_per_block - 1) / warps_per_block));
+  const long long items = (long long)b.total_tiles * (few ? 2 : 1);  // a chunk in pairs is two
+  const int grid = (int)std::max(1ll, std::min((long long)(lane_groups ? c->grid_blocks_lg : c->grid_blocks),
+                                               (items + warps_per_block - 1) / warps_per_block));
   CUDA_TRY(c, launch_render_warps(b, cw, ch, grid, false, s, c->staging, lane_groups, few, order != nullptr));
   return ALOHA_OK;
 }

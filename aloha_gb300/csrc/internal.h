@@ -135,6 +135,9 @@ struct BatchArgs {
   int total_tiles;           // chunks in the launch
   unsigned int* work_counter;
   const int* chunk_order;    // single view: chunk ids in the order to render them, or null (ring order)
+  const int* pair_chunks;    // the instance of few chunks, single view in cost order (or null): so many first
+                             // positions are rendered with two lanes per ray, as two items each
+  bool ring_pairs;           // ... in ring order: every position is
   int group_chunks;          // single view in cost order: the first group_chunks chunks of chunk_order are
                              // rendered by lane groups (kLaneGroup lanes per ray), as kLaneGroup items each
 };
@@ -154,6 +157,8 @@ struct ChunkOrderArgs {
   uint8_t* key;      // [n_slots] cost class per slot (0xff off the grid)
   int* cid;          // [n_slots] chunk id per slot
   uint32_t* hist;    // [kOrderClasses][chunk_order_blocks(n_slots)] counts; zero between launches
+  int warps;         // resident warps of the render
+  int* pairs;        // set: chunks at the head of the order that two lanes per ray render sooner
   uint32_t* readers; // the word after hist: scatter CTAs that have read it; zero between launches
   int* order;        // [chunks] chunk ids, most expensive first
   int n_chunks;      // chunks of the grid (entries of `order`)
@@ -245,7 +250,12 @@ constexpr int kSingleRenderBlocks = 5, kBatchRenderBlocks = 7;  // CTAs per SM
 // with many, throughput counts (64^3 at 1024^2 155 / 146, 256^3 at 1280x1024 354
 // / 331, 512^3 at 1920x1080 650 / 630; 512^3 at 1024^2, 10.8 chunks per warp of
 // the 5-CTA instance, 602 / 605).
-constexpr int kFewChunkRenderBlocks = 4, kFewChunksPerWarp = 9;
+// Without a cost order, frames of at most kPairRingChunks chunks are rendered
+// with two lanes per ray throughout (one / two, us: 64^3 at 256^2 69 / 53, at
+// 480^2, 7200 chunks, 69 / 69; 512^3 at 64^2 420 / 281, at 480^2 487 / 336; a
+// GPU's warps are 2432 at a time).
+constexpr int kFewChunkRenderBlocks = 4, kFewChunksPerWarp = 9, kPairRingChunks = 8192;
+constexpr int kRingPairs = -2;  // the kernel's LG for ring_pairs
 // CTAs per SM of the differentiable form's forward (checkpointed march).  Six
 // 512^2 views of 256^3: 785 us at 5, 820 at 6, 875 at 7; one 1024^2 view of
 // 512^3: 900 at 5, 914 at 4.

@@ -708,6 +708,82 @@ __device__ __forceinline__ uint32_t march_brick_group(const DevBrick& b, const f
   return n;
 }
 
+// Two lanes per ray: march_brick with the ray's state (t, n, colour) in both
+// lanes and its samples two at a time, the first lane taking the sample at t,
+// the second the one after it; both composite the two in order from exchanged
+// values, so the state leaves a step as march_brick leaves it after the same
+// samples, bit for bit.  A ray's chain of dependent steps is half as long and a
+// warp waits for the longest of 16 rays, not of 32; the lookups, jumps and the
+// composite are done twice, so all chunks of a full GPU are slower this way
+// (512^3 at 1024^2 678 -> 711 us, 24-view batch 7.5 -> 9.4 ms) and those of a
+// GPU with idle warps faster (512^3 at 512^2 576 -> 371 us, 256^3 235 -> 185).
+// kPairRun 6 / 8 / 12: 256^3 at 512^2 with an upload 430 / 425 / 432 us.
+constexpr int kPairRun = 8;
+template <bool INNER>
+__device__ __forceinline__ uint32_t march_brick_pair(const DevBrick& b, const float4* __restrict__ tf_s, int n_tf,
+                                                     const Ray& r, float t0, float t1, float ils, float dt, float et,
+                                                     float4& color, const LaneGroup& g) {
+  const float4* __restrict__ base = b.base;
+  const int sy = b.sy, sz = b.sz, nx = b.n[0], ny = b.n[1], nz = b.n[2];
+  const float lox = b.lo[0], loy = b.lo[1], loz = b.lo[2];
+  const float nf = (float)n_tf;
+  const uint32_t cap = march_cap(t0, t1, dt);
+  const uint8_t* __restrict__ cells = b.cells;
+  const int mnx = (nx + kMacro - 1) >> kMacroShift, mny = (ny + kMacro - 1) >> kMacroShift;
+  const float offx = r.o[0] - lox, offy = r.o[1] - loy, offz = r.o[2] - loz;
+  const float idx_ = 1.0f / r.d[0], idy = 1.0f / r.d[1], idz = 1.0f / r.d[2];
+  const float mag = fmaxf(fmaxf(fabsf(r.o[0]) + fabsf(lox), fabsf(r.o[1]) + fabsf(loy)),
+                          fabsf(r.o[2]) + fabsf(loz)) + fabsf(t1);
+  const float eps = 2e-6f * mag + 1e-4f;
+  const bool first = g.lane == 0;
+  uint32_t n = 0;
+  float t = first_sample_t(t0, dt, ils);
+  const bool exact = exact_steps(t, t1, dt);
+  const float inv_dt = 1.0f / dt;
+  while (t < t1 && color.w < et && n < cap) {
+    int jumps = 0;  // as in march_brick, by both lanes
+    for (; jumps < kMarchJumps && t < t1 && n < cap; ++jumps) {
+      const Cell cell = cell_at(cells, mnx, mny, nx, ny, nz, fmaf(t, r.d[0], r.o[0]) - lox,
+                                fmaf(t, r.d[1], r.o[1]) - loy, fmaf(t, r.d[2], r.o[2]) - loz);
+      if (!cell.empty()) break;
+      const float tb = cell_exit(cell, r.d, offx, offy, offz, idx_, idy, idz, eps, t1);
+      ++n;
+      t = t + dt;
+      if (exact)
+        run_steps(t, n, tb, cap, dt, inv_dt, 0xffffffffu);
+      else
+        run_steps_any(t, n, tb, cap, dt, 0xffffffffu);
+    }
+    if (jumps == kMarchJumps) continue;
+#pragma unroll 1
+    for (int k = 0; k < kPairRun && t < t1 && color.w < et && n < cap; k += 2) {
+      // past the ray's end the second lane takes the first one's sample again
+      // (its coordinates are known to be the brick's) and drops it
+      const float t2 = t + dt;
+      const bool two = t2 < t1 && n + 1 < cap;
+      const float tk = !first && two ? t2 : t;
+      const StencilOut s =
+          stencil<INNER>(base, sy, sz, nx, ny, nz, fmaf(tk, r.d[0], r.o[0]) - lox, fmaf(tk, r.d[1], r.o[1]) - loy,
+                         fmaf(tk, r.d[2], r.o[2]) - loz);
+      const float shade = shade_factor(s, r);
+      const float4 c = tf_lookup<INNER>(tf_s, n_tf, nf, s.value);
+      const float os = __shfl_xor_sync(g.mask, shade, 1);
+      const float ox = __shfl_xor_sync(g.mask, c.x, 1), oy = __shfl_xor_sync(g.mask, c.y, 1);
+      const float oz = __shfl_xor_sync(g.mask, c.z, 1), ow = __shfl_xor_sync(g.mask, c.w, 1);
+      composite_step(color, make_float4(first ? c.x : ox, first ? c.y : oy, first ? c.z : oz, first ? c.w : ow),
+                     first ? shade : os);
+      ++n;
+      t = t2;
+      if (two && color.w < et) {
+        composite_step(color, make_float4(first ? ox : c.x, first ? oy : c.y, first ? oz : c.z, first ? ow : c.w),
+                       first ? os : shade);
+        ++n;
+        t = t + dt;
+      }
+    }
+  }
+  return n;
+}
 
 __device__ __forceinline__ float saturatef_(float x) { return fminf(fmaxf(x, 0.0f), 1.0f); }
 
@@ -742,9 +818,10 @@ __device__ __forceinline__ void load_tf(float4* tf_s, const float4* __restrict__
 
 // One virtual rank's march for one pixel (deviceCode.cpp:378-399): the
 // rank's bricks [j0, j1) of the view schedule front to back, spp draws, early
-// termination on the rank's own alpha.  Returns the spp sum of the colours;
+// termination on the rank's own alpha.  ONE: spp is known to be 1; ROLLED: one
+// copy of the march for all passes.  Returns the spp sum of the colours;
 // z = nearest brick entry / max depth, ns = samples taken.
-template <bool INNER, class Loads = DirectLoads, int G = 1>
+template <bool INNER, class Loads = DirectLoads, int G = 1, bool ONE = false, bool ROLLED = false>
 __device__ __forceinline__ float4 march_rank(const FrameArgs& a, const DevView& v, const float4* tf_s, const Ray& ray,
                                              const int* __restrict__ rbricks, int j0, int j1, int pixel, float& z,
                                              uint32_t& ns, Loads& loads, const LaneGroup& g = LaneGroup{0, 0u, 0}) {
@@ -761,7 +838,9 @@ __device__ __forceinline__ float4 march_rank(const FrameArgs& a, const DevView& 
       const float tnear = (t0 > tmin ? t0 : 0.0f) + tmin;
       z = fminf(z, tnear / v.max_depth);
       NoHook none;
-      if constexpr (G > 1) {
+      if constexpr (G == 2) {
+        ns += march_brick_pair<INNER>(b, tf_s, a.n_tf, ray, t0, t1, ils, a.dt, a.et_alpha, color, g);
+      } else if constexpr (G > 1) {
         ns += march_brick_group<G>(b, tf_s, a.n_tf, ray, t0, t1, ils, a.dt, a.et_alpha, color, g);
       } else {
         ns += march_brick<INNER>(b, tf_s, a.n_tf, ray, t0, t1, ils, a.dt, a.et_alpha, color, none, loads);
@@ -775,6 +854,19 @@ __device__ __forceinline__ float4 march_rank(const FrameArgs& a, const DevView& 
   // march colour is never -0 (it starts at +0 and every update is an fmaf
   // onto it, and an exact zero sum rounds to +0).  With one pass no sum is
   // then live across the march.
+  if constexpr (ONE) return pass();
+  if constexpr (ROLLED) {
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+    for (int s = 0; s < a.spp; ++s) {
+      const float4 color = pass();
+      sum.x = sum.x + color.x;
+      sum.y = sum.y + color.y;
+      sum.z = sum.z + color.z;
+      sum.w = sum.w + color.w;
+    }
+    return sum;
+  }
   float4 acc = pass();
   for (int s = 1; s < a.spp; ++s) {
     const float4 color = pass();
@@ -885,9 +977,15 @@ __device__ __forceinline__ bool pixel_in_island(const FrameArgs& a, int W, int x
 // renderFrame's output stage; the rank images are blended front to back.
 // Returns the number of samples.
 // With G > 1 the G lanes of `g` render the pixel together (a lane group);
-// only the group's first lane writes the frame buffer.  The group form has no
-// accumulation buffer and no rank planes (the caller ensures it).
-template <bool INNER, class Loads = DirectLoads, int G = 1>
+// only the group's first lane runs the output stage and writes.  Groups of
+// more than two have no accumulation buffer and no rank planes (the caller
+// ensures it).
+// ONE: one copy of the march for plain InnerCoords frames of one pass and one for
+// everything else, for kernels that hold several marches and are short of
+// instruction cache rather than registers (2 spp frame with two lanes per ray
+// 335 -> 299 us, 512^3 at 1024^2 678 -> 673; the 72-register instances spill
+// more with it, 7.47 -> 7.67 ms for a 24-view batch).
+template <bool INNER, class Loads = DirectLoads, int G = 1, bool ONE = false>
 __device__ __forceinline__ uint32_t render_pixel(const FrameArgs& a, const DevView& v, const float4* tf_s, int x,
                                                  int y, uint32_t* fb_out, size_t fb_index, Loads& loads,
                                                  const LaneGroup& g = LaneGroup{0, 0u, 0}) {
@@ -902,7 +1000,7 @@ __device__ __forceinline__ uint32_t render_pixel(const FrameArgs& a, const DevVi
   const Ray ray = generate_ray(v, x, y);
   OverBlend blend;
   uint32_t total = 0;
-  if (plain_output(a)) {
+  if ((INNER || !ONE) && plain_output(a)) {
     // the output stage is the identity (acc * 1 * 1): nothing it needs stays
     // live across the march
     for (int k = 0; k < R; ++k) {
@@ -911,8 +1009,8 @@ __device__ __forceinline__ uint32_t render_pixel(const FrameArgs& a, const DevVi
       uint32_t ns = 0;
       float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
       if (in_island)
-        acc = march_rank<INNER, Loads, G>(a, v, tf_s, ray, rbricks, __ldg(rstart + r), __ldg(rstart + r + 1), pixel, z, ns,
-                                   loads, g);
+        acc = march_rank<INNER, Loads, G, ONE>(a, v, tf_s, ray, rbricks, __ldg(rstart + r), __ldg(rstart + r + 1),
+                                               pixel, z, ns, loads, g);
       blend.add(a.composite_mode, acc);
       total += ns;
     }
@@ -923,9 +1021,10 @@ __device__ __forceinline__ uint32_t render_pixel(const FrameArgs& a, const DevVi
       uint32_t ns = 0;
       float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
       if (in_island)
-        acc = march_rank<INNER, Loads, G>(a, v, tf_s, ray, rbricks, __ldg(rstart + r), __ldg(rstart + r + 1), pixel, z, ns,
-                                   loads, g);
-      blend.add(a.composite_mode, rank_output(a, W, H, r, x, y, pixel, npx, acc, ns, z, a.rank_images, a.rank_depth));
+        acc = march_rank<INNER, Loads, G, false, ONE>(a, v, tf_s, ray, rbricks, __ldg(rstart + r),
+                                                      __ldg(rstart + r + 1), pixel, z, ns, loads, g);
+      if (G == 1 || g.lane == 0)
+        blend.add(a.composite_mode, rank_output(a, W, H, r, x, y, pixel, npx, acc, ns, z, a.rank_images, a.rank_depth));
       total += ns;
     }
   }
@@ -938,6 +1037,10 @@ __device__ __forceinline__ uint32_t render_pixel(const FrameArgs& a, const DevVi
 // quads than a row of eight does.
 __device__ __forceinline__ int tile_x(int lane) { return (lane & 1) | ((lane >> 2) & 6); }
 __device__ __forceinline__ int tile_y(int lane) { return (lane >> 1) & 3; }
+
+// The same for pixel p of a 4x4 tile whose rays have two lanes each.
+__device__ __forceinline__ int pair_x(int p) { return (p & 1) | ((p >> 1) & 2); }
+__device__ __forceinline__ int pair_y(int p) { return ((p >> 1) & 1) | ((p >> 2) & 2); }
 
 // Work slot k of a view -> chunk (cx, cy) in centre-out square rings; false
 // for slots outside the chunk grid.  Ring r >= 1 holds slots

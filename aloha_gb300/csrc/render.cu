@@ -10,6 +10,24 @@
 
 namespace aloha {
 
+// Half `half` (4x4 pixels) of an 8x4 chunk, two lanes per ray (march_brick_pair).
+// INNER: the view and scene are InnerCoords.  Returns the samples, counted in
+// the rays' first lanes.
+template <bool INNER, class Loads>
+__device__ __forceinline__ uint32_t render_half_chunk(const BatchArgs& b, const DevView& v, const float4* tf_s, int ccx,
+                                                      int ccy, int half, int lane, uint32_t* fb, Loads& loads) {
+  const int p = lane >> 1, x = ccx * 8 + 4 * half + pair_x(p), y = ccy * 4 + pair_y(p);
+  if (x >= v.width || y >= v.height) return 0;  // both lanes of the ray
+  const LaneGroup g{lane & 1, 3u << (lane & 30), lane & 30};
+  const size_t at = (size_t)x + (size_t)v.width * y;
+  uint32_t ns;
+  if (INNER || (b.f.inner && v.inner && *b.f.scene_inner))
+    ns = render_pixel<true, Loads, 2, true>(b.f, v, tf_s, x, y, fb, at, loads, g);
+  else
+    ns = render_pixel<false, Loads, 2, true>(b.f, v, tf_s, x, y, fb, at, loads, g);
+  return g.lane == 0 ? ns : 0;
+}
+
 // Persistent render: every warp pulls CW x CH pixel chunks of the launch's
 // items (views) from one atomic counter -- a single view in cost order when
 // b.chunk_order is set (schedule.cu), else centre-out per view -- and renders
@@ -26,8 +44,11 @@ namespace aloha {
 // STAGE selects the stencil loads: 0 direct, 1 the next sample's rows staged
 // in shared memory with cp.async (StagedLoads; shared memory after the
 // transfer function), kStageUnroll2 (batches) direct with the march loop
-// written out two steps per trip.  LG > 1 (single view in cost order, 8x4 chunks, frame
-// buffer only): work positions [0, LG * group_chunks) are the costliest
+// written out two steps per trip.  LG == 2 (single view in cost order, 8x4
+// chunks): the first *pair_chunks positions of an InnerCoords scene are two
+// items each, the chunk's 4x4 halves with two lanes per ray.  LG == kRingPairs:
+// the same for all positions of the ring order of any scene.  LG > 2 (single view in
+// cost order, 8x4 chunks, frame buffer only): work positions [0, LG * group_chunks) are the costliest
 // group_chunks chunks, each as LG items of 32 / LG pixels rendered by lane
 // groups of LG lanes per ray; the remaining positions are the other chunks of
 // the cost order, rendered as usual.
@@ -39,16 +60,21 @@ __global__ void __launch_bounds__(kRenderThreads, MINB) render_warps_kernel(Batc
   using Loads = typename std::conditional<
       STAGE == 1, StagedLoads,
       typename std::conditional<STAGE == kStageUnroll2, UnrolledDirectLoads<2>, DirectLoads>::type>::type;
+  constexpr bool kOne = MINB < kBatchRenderBlocks;  // render_pixel's ONE
   Loads loads;
   if constexpr (STAGE == 1) loads.init(tf_s + (b.f.n_tf + 4));
+  // pairs are for InnerCoords scenes alone here (fewer copies of the march)
+  const bool may_pair =
+      LG == 2 && b.pair_chunks && b.f.inner && b.f.views[b.single_view].inner && *b.f.scene_inner;
   wait_for_primary();  // the chunk order and the cleared counters
   const int lane = threadIdx.x & 31;
+  const int pairs = LG == kRingPairs ? b.total_tiles : (may_pair ? __ldcg(b.pair_chunks) : 0);
   uint32_t n = 0;
   for (;;) {
     int chunk = 0;
     if (lane == 0) chunk = (int)atomicAdd(b.work_counter, 1u);
     chunk = __shfl_sync(0xffffffffu, chunk, 0);
-    if (chunk >= b.total_tiles) break;
+    if (chunk >= b.total_tiles + pairs) break;
     int item = 0, first = 0;
     if (b.tile_prefix) {
       // item = last index with tile_prefix[item] <= chunk
@@ -67,7 +93,20 @@ __global__ void __launch_bounds__(kRenderThreads, MINB) render_warps_kernel(Batc
     uint32_t* fb = b.fbs ? b.fbs[item] : b.f.fb;
     int ccx, ccy;
     const int cxn = (v.width + CW - 1) / CW;
-    if constexpr (LG > 1) {
+    if constexpr (LG == 2) {
+      if (chunk < 2 * pairs) {
+        const int id = __ldg(b.chunk_order + (chunk >> 1));
+        n += render_half_chunk<true>(b, v, tf_s, id % cxn, id / cxn, chunk & 1, lane, fb, loads);
+        continue;
+      }
+      chunk -= pairs;
+    }
+    if constexpr (LG == kRingPairs) {
+      if (ring_chunk(chunk >> 1, cxn, (v.height + CH - 1) / CH, ccx, ccy))
+        n += render_half_chunk<false>(b, v, tf_s, ccx, ccy, chunk & 1, lane, fb, loads);
+      continue;
+    }
+    if constexpr (LG > 2) {
       if (chunk < b.group_chunks * LG) {
         const int id = __ldg(b.chunk_order + chunk / LG), part = chunk % LG;
         const int gl = lane % LG, p = part * (32 / LG) + lane / LG;
@@ -104,9 +143,10 @@ __global__ void __launch_bounds__(kRenderThreads, MINB) render_warps_kernel(Batc
       const int y = y0 + (sub / (CW / 8)) * 4 + tile_y(lane);
       if (x < v.width && y < v.height) {
         if (inner)
-          n += render_pixel<Loads::kInner>(b.f, v, tf_s, x, y, fb, (size_t)x + (size_t)v.width * y, loads);
+          n += render_pixel<Loads::kInner, Loads, 1, kOne>(b.f, v, tf_s, x, y, fb, (size_t)x + (size_t)v.width * y,
+                                                           loads);
         else
-          n += render_pixel<false>(b.f, v, tf_s, x, y, fb, (size_t)x + (size_t)v.width * y, loads);
+          n += render_pixel<false, Loads, 1, kOne>(b.f, v, tf_s, x, y, fb, (size_t)x + (size_t)v.width * y, loads);
       }
     }
   }
@@ -564,7 +604,7 @@ RenderKernel render_kernel_for(int chunk_w, int chunk_h) {
   return nullptr;
 }
 
-RenderKernel render_kernel(int chunk_w, int chunk_h, bool batch, int stage, bool lane_groups, bool few) {
+RenderKernel render_kernel(int chunk_w, int chunk_h, bool batch, int stage, bool lane_groups, bool few, bool ring_pairs) {
   if (lane_groups)
     return (!batch && stage == ALOHA_STAGING_NONE && chunk_w == 8 && chunk_h == 4)
                ? render_warps_kernel<8, 4, kSingleRenderBlocks, 0, kLaneGroup>
@@ -575,7 +615,9 @@ RenderKernel render_kernel(int chunk_w, int chunk_h, bool batch, int stage, bool
   if (stage == kStageUnroll2) return batch ? render_kernel_for<kBatchRenderBlocks, kStageUnroll2>(chunk_w, chunk_h)
                                            : nullptr;
   if (stage != ALOHA_STAGING_NONE) return nullptr;
-  if (few && !batch && chunk_w == 8 && chunk_h == 4) return render_warps_kernel<8, 4, kFewChunkRenderBlocks, 0>;
+  if (few && !batch && chunk_w == 8 && chunk_h == 4)
+    return ring_pairs ? render_warps_kernel<8, 4, kFewChunkRenderBlocks, 0, kRingPairs>
+                      : render_warps_kernel<8, 4, kFewChunkRenderBlocks, 0, 2>;
   return batch ? render_kernel_for<kBatchRenderBlocks, 0>(chunk_w, chunk_h)
                : render_kernel_for<kSingleRenderBlocks, 0>(chunk_w, chunk_h);
 }
@@ -585,13 +627,13 @@ RenderKernel render_kernel(int chunk_w, int chunk_h, bool batch, int stage, bool
 cudaError_t launch_render_warps(const BatchArgs& b, int chunk_w, int chunk_h, int grid, bool batch, cudaStream_t s,
                                 int stage, bool lane_groups, bool few, bool beside) {
   if (lane_groups && (!b.chunk_order || b.f.rank_images || b.f.rank_depth || b.f.accum)) return cudaErrorInvalidValue;
-  const RenderKernel k = render_kernel(chunk_w, chunk_h, batch, stage, lane_groups, few);
+  const RenderKernel k = render_kernel(chunk_w, chunk_h, batch, stage, lane_groups, few, few && b.ring_pairs);
   if (!k) return cudaErrorInvalidValue;
   return launch_beside(k, grid, kRenderThreads, render_smem(b.f.n_tf, stage), s, beside, b);
 }
 
 int render_blocks_per_sm(int chunk_w, int chunk_h, int n_tf, bool batch, int stage, bool lane_groups, bool few) {
-  const RenderKernel k = render_kernel(chunk_w, chunk_h, batch, stage, lane_groups, few);
+  const RenderKernel k = render_kernel(chunk_w, chunk_h, batch, stage, lane_groups, few, false);
   int n = 0;
   if (!k || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, kRenderThreads, render_smem(n_tf, stage)) !=
                 cudaSuccess) {

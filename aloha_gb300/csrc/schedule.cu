@@ -131,6 +131,7 @@ __global__ void probe_chunks_kernel(ChunkOrderArgs a) {
 // Exclusive scan of the histogram table in place (one CTA; each thread scans
 // a contiguous range).
 __global__ void __launch_bounds__(kScanThreads) class_scan_kernel(ChunkOrderArgs a, int n) {
+  if (threadIdx.x == 0) *a.pairs = 0;  // large frames fill the GPU
   __shared__ uint32_t warp_sum[kScanThreads / 32];
   const int per = (n + kScanThreads - 1) / kScanThreads;
   const int lo = min(n, (int)threadIdx.x * per), hi = min(n, lo + per);
@@ -161,6 +162,31 @@ __global__ void __launch_bounds__(kScanThreads) class_scan_kernel(ChunkOrderArgs
     a.hist[i] = at;
     at += c;
   }
+}
+
+// How many chunks at the head of the order two lanes per ray render sooner
+// than one: all that the probe found samples in, or none.  `waves` is the
+// frame's work against what the resident warps do while the costliest chunk
+// runs: the fewer, the more warps only wait for that chunk, which two lanes per
+// ray shorten, the more so the longer its rays (each lane also repeats a ray's
+// set-up).  One / two lanes, us, over (waves, strides of the costliest chunk):
+//   wins:   (.23, 18) 148 / 115   (.34, 37) 352 / 298   (.36, 53) 579 / 371
+//           (.38, 26) 199 / 157   (.43, 15) 111 / 99    (.45, 31) 239 / 209   (.50, 53) 561 / 394
+//   losses: (.47, 7) 224 / 252    (.49, 18) 261 / 287   (.51, 7) 68 / 74      (.74, 31) 249 / 254
+// One warp: classes 2 lane and 2 lane + 1 hold t0 and t1 chunks.
+__device__ __forceinline__ void pair_rule(const ChunkOrderArgs& a, int lane, uint32_t t0, uint32_t t1) {
+  const float c0 = exp2f(0.25f * (float)(kOrderClasses - 1 - 2 * lane)) - 1.0f;
+  const float c1 = exp2f(0.25f * (float)(kOrderClasses - 2 - 2 * lane)) - 1.0f;
+  float sum = fmaf((float)t0, c0, (float)t1 * c1), most = t0 ? c0 : (t1 ? c1 : 0.f);
+  int active = (int)t0 + (lane == 31 ? 0 : (int)t1);
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    sum += __shfl_xor_sync(0xffffffffu, sum, d);
+    most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, d));
+    active += __shfl_xor_sync(0xffffffffu, active, d);
+  }
+  const float waves = 0.22f + most * (1.0f / 70.0f);
+  if (lane == 0) *a.pairs = sum < waves * most * (float)a.warps ? active : 0;
 }
 
 // Stable scatter: a slot's position is its class's base for this CTA plus the
@@ -212,6 +238,7 @@ __global__ void __launch_bounds__(kSortThreads) class_scatter_kernel(ChunkOrderA
         const uint32_t o = __shfl_up_sync(0xffffffffu, incl, d);
         if (lane >= d) incl += o;
       }
+      if (blockIdx.x == 0) pair_rule(a, lane, t0, t1);
       class_base[2 * lane] += incl - t0 - t1;
       class_base[2 * lane + 1] += incl - t1;
     }
