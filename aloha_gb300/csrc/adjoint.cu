@@ -706,28 +706,36 @@ __global__ void __launch_bounds__(128, 5) backward_kernel(TrainArgs a) {
 //     dL/d(alpha of the sample) = (1 - a)(s g.c + gA),
 // with the colour of the segment's checkpoint for all its samples.  No sample
 // waits for the one before it and nothing here has to round as the forward
-// does, so one segment per thread costs little more than the stencil's loads:
-// no composite, an approximate reciprocal square root in the shading, two
-// pending sums instead of eight.  Bound by the L1 data pipe (82 % of its
-// wavefronts; 30 per 32 samples, of which 24 are the stencil's 96 bytes per
-// sample), so occupancy hardly matters: 6.51 ms per pass of a 512^3 1024^2
-// transfer-function step at 6 CTAs/SM, 6.65 at 5, 6.54 at 8.  One 512^3 view's
-// transfer-function backward: 5.82 ms with every segment replayed, 1.20 ms for
-// the replayed ones and 3.34 ms here; the density-only replay of 6 views of
-// 256^3, which only loses the empty rows between its lanes, went from 2.2 to
-// 1.3 ms.
-template <bool INNER, bool MULTI>
+// does: no composite, an approximate reciprocal square root in the shading, two
+// pending sums instead of eight.  Bound by the L1 data pipe (83 % busy), mostly
+// with the stencil's 112 bytes per sample: so two lanes take a segment's samples
+// in turn, and a quarter warp, the unit of 16-byte loads, covers 2x2 rays by two
+// samples, whose quads collide in fewer banks than those of 2x4 rays (a model of
+// the pipe, confirmed for the first: 55 -> 41 cycles for a warp's seven loads at
+// 0.83 voxels per pixel).  The two lanes want the same bins, and adding to a
+// float in shared memory is a loop until no other lane interferes, so the bins
+// are kept in COPIES, interleaved so that a lane's copy has banks of its own.
+// Per pass of a 512^3 1024^2 transfer-function step, ms: one lane and one copy
+// 5.95, two lanes 6.51, two lanes and 2 / 4 / 8 / 16 / 32 copies 5.95 / 5.78 /
+// 5.67 / 5.62 / 6.09, one lane and 2 / 16 copies 5.83 / 5.89; at 5 / 7 / 8 CTAs
+// per SM 1.7 / 1.8 / 7.4 % slower.  One 512^3 view's transfer-function backward
+// with every segment replayed: 5.82 ms; 1.20 ms for the replayed ones and 3.08
+// here.  The density-only replay of 6 views of 256^3, which only loses the empty
+// rows between its lanes, went from 2.2 to 1.3 ms with the split.
+template <bool INNER, bool MULTI, int COPIES>
 __global__ void __launch_bounds__(128, kBackwardEmptyBlocks) backward_empty_kernel(TrainArgs a) {
   extern __shared__ float4 smem[];
   float4* tf_s = smem;                                         // n_tf + 4 entries
   float* dalpha_s = reinterpret_cast<float*>(smem + a.n_tf + 4);  // n_tf + 4: alpha entries, two unused on each side
   load_tf(tf_s, a.tf, a.n_tf);
-  for (int i = threadIdx.x; i < a.n_tf + 4; i += blockDim.x) dalpha_s[i] = 0.f;
+  for (int i = threadIdx.x; i < (a.n_tf + 4) * COPIES; i += blockDim.x) dalpha_s[i] = 0.f;
+  float* const bins = dalpha_s + threadIdx.x % COPIES;
   __syncthreads();
   const unsigned count = MULTI ? __ldg(a.empty_base + a.n_views) : a.one_empty;
   const float nf = (float)a.n_tf, dt = a.dt;
   uint32_t nsamp = 0;
   const unsigned lane = threadIdx.x & 31u;
+  const bool second = lane & 1u;  // two lanes per item: the samples at even and odd places
   const unsigned warps = gridDim.x * (blockDim.x / 32u);
   const unsigned take = max(32u, min(kBackwardGrab, (count / (warps * 8u)) & ~31u));
   for (;;) {
@@ -736,7 +744,7 @@ __global__ void __launch_bounds__(128, kBackwardEmptyBlocks) backward_empty_kern
     grab = __shfl_sync(0xffffffffu, grab, 0);
     if (grab >= count) break;
     const unsigned end = min(grab + take, count);
-    for (unsigned item = grab + lane; item < end; item += 32u) {
+    for (unsigned item = grab + (lane >> 1); item < end; item += 16u) {
       int slot = 0;
       unsigned first = 0;
       if constexpr (MULTI) {
@@ -781,9 +789,13 @@ __global__ void __launch_bounds__(128, kBackwardEmptyBlocks) backward_empty_kern
         const int sy = b.sy, sz = b.sz, nx = b.n[0], ny = b.n[1], nz = b.n[2];
         const float lox = b.lo[0], loy = b.lo[1], loz = b.lo[2];
         while (t < t1 && nb < cap && n < a.k) {
+          // two samples at a time; without a second one its lane adds nothing
+          const float t2 = t + dt;
+          const bool two = t2 < t1 && nb + 1 < cap && n + 1 < a.k;
+          const float tk = second && two ? t2 : t;
           const StencilOut s =
-              stencil<INNER, true>(base, sy, sz, nx, ny, nz, fmaf(t, ray.d[0], ray.o[0]) - lox,
-                            fmaf(t, ray.d[1], ray.o[1]) - loy, fmaf(t, ray.d[2], ray.o[2]) - loz);
+              stencil<INNER, true>(base, sy, sz, nx, ny, nz, fmaf(tk, ray.d[0], ray.o[0]) - lox,
+                                   fmaf(tk, ray.d[1], ray.o[1]) - loy, fmaf(tk, ray.d[2], ray.o[2]) - loz);
           const float ex = s.gx + 1e-4f, ey = s.gy + 1e-4f, ez = s.gz + 1e-4f;
           const float inv = rsqrtf(fmaf(ex, ex, fmaf(ey, ey, ez * ez)));
           const float gd = fmaf(s.gx, ray.d[0], fmaf(s.gy, ray.d[1], s.gz * ray.d[2]));
@@ -797,8 +809,8 @@ __global__ void __launch_bounds__(128, kBackwardEmptyBlocks) backward_empty_kern
           const int step = ic - pend_i;
           if (step != 0) {
             const bool down = step == -1;
-            atomicAdd(dalpha_s + pend_i + (down ? 3 : 2), down ? pend1 : pend0);
-            if (step != 1 && !down) atomicAdd(dalpha_s + pend_i + 3, pend1);
+            atomicAdd(bins + (pend_i + (down ? 3 : 2)) * COPIES, down ? pend1 : pend0);
+            if (step != 1 && !down) atomicAdd(bins + (pend_i + 3) * COPIES, pend1);
             const float next0 = step == 1 ? pend1 : 0.f;
             pend1 = down ? pend0 : 0.f;
             pend0 = next0;
@@ -807,23 +819,27 @@ __global__ void __launch_bounds__(128, kBackwardEmptyBlocks) backward_empty_kern
             gc0 = fmaf(g.x, e0.x, fmaf(g.y, e0.y, g.z * e0.z));
             gcd = fmaf(g.x, e1.x, fmaf(g.y, e1.y, g.z * e1.z)) - gc0;
           }
-          const float dA = oma * fmaf(shade, fmaf(wt, gcd, gc0), gA);
+          const float dA = second && !two ? 0.f : oma * fmaf(shade, fmaf(wt, gcd, gc0), gA);
           pend0 = fmaf(1.f - wt, dA, pend0);
           pend1 = fmaf(wt, dA, pend1);
-          ++n;
-          ++nb;
-          t = t + dt;
+          n += two ? 2 : 1;
+          nb += two ? 2 : 1;
+          t = two ? t2 + dt : t2;
         }
         tmin = t1 + 1e-20f;
       }
-      atomicAdd(dalpha_s + pend_i + 2, pend0);
-      atomicAdd(dalpha_s + pend_i + 3, pend1);
-      nsamp += n;
+      atomicAdd(bins + (pend_i + 2) * COPIES, pend0);
+      atomicAdd(bins + (pend_i + 3) * COPIES, pend1);
+      nsamp += second ? 0u : n;
     }
   }
   count_samples(a.counter, nsamp);
   __syncthreads();
-  for (int i = threadIdx.x; i < a.n_tf; i += blockDim.x) red_add(a.dtf + 4 * i + 3, dalpha_s[i + 2]);
+  for (int i = threadIdx.x; i < a.n_tf; i += blockDim.x) {
+    float v = 0.f;
+    for (int c = 0; c < COPIES; ++c) v += dalpha_s[(i + 2) * COPIES + c];
+    red_add(a.dtf + 4 * i + 3, v);
+  }
 }
 
 size_t backward_smem(int n_tf, bool with_tf) {
@@ -877,12 +893,26 @@ cudaError_t launch_backward(const TrainArgs& a, int grid, bool inner, cudaStream
   return cudaGetLastError();
 }
 
+template <int COPIES>
+static BackwardKernel backward_empty(bool inner, bool multi) {
+  if (inner) return multi ? backward_empty_kernel<true, true, COPIES> : backward_empty_kernel<true, false, COPIES>;
+  return multi ? backward_empty_kernel<false, true, COPIES> : backward_empty_kernel<false, false, COPIES>;
+}
+
 cudaError_t launch_backward_empty(const TrainArgs& a, int sms, bool inner, cudaStream_t s) {
-  const size_t smem = (size_t)(a.n_tf + 4) * (sizeof(float4) + sizeof(float));
+  // As many copies of the bins as leave most of an SM's memory to the L1 (six
+  // CTAs), at least two where they fit.  A 1024^2 backward of 512^3, us, by
+  // entries, one thread per segment and one copy first: 16: 4807 / 4451 (16
+  // copies), 256: 5267 / 4881 (16), 512: 5611 / 5237 (4), 1024: 5811 / 5789 (2;
+  // 9260 with 4), 2044: 10476 / 7476 (2).
+  auto bytes = [&](int copies) { return (size_t)(a.n_tf + 4) * (sizeof(float4) + copies * sizeof(float)); };
+  const int copies = bytes(16) <= 23 * 1024 ? 16 : (bytes(4) <= 23 * 1024 ? 4 : (bytes(2) <= 48 * 1024 ? 2 : 1));
   const bool multi = a.n_views > 1;
-  const BackwardKernel k = inner ? (multi ? backward_empty_kernel<true, true> : backward_empty_kernel<true, false>)
-                                 : (multi ? backward_empty_kernel<false, true> : backward_empty_kernel<false, false>);
-  k<<<sms * kBackwardEmptyBlocks, 128, smem, s>>>(a);
+  const BackwardKernel k = copies == 16  ? backward_empty<16>(inner, multi)
+                           : copies == 4 ? backward_empty<4>(inner, multi)
+                           : copies == 2 ? backward_empty<2>(inner, multi)
+                                         : backward_empty<1>(inner, multi);
+  k<<<sms * kBackwardEmptyBlocks, 128, bytes(copies), s>>>(a);
   return cudaGetLastError();
 }
 
