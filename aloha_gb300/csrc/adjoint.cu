@@ -425,20 +425,20 @@ __global__ void fold_quads_kernel(float4* __restrict__ q, float* __restrict__ ou
   }
 }
 
-// Adds a pending transfer-function gradient (entries i and i+1, four
-// channels each) to the CTA's shared copy and clears it.
-__device__ __forceinline__ void flush_tf(float* dtf_s, int n, int i, float pend[8]) {
+// Adds a pending transfer-function gradient (four channels of entry e) to this
+// lane's copy in shared memory.
+__device__ __forceinline__ void add_tf_entry(float* dtf_s, int copies, int n, int e, const float* pend) {
+  if (e < 0 || e >= n) return;
+  float* p = dtf_s + e * 4 * copies;
 #pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    const int e = i + k;
-    if (e >= 0 && e < n) {
-#pragma unroll
-      for (int ch = 0; ch < 4; ++ch)
-        if (pend[4 * k + ch] != 0.f) atomicAdd(dtf_s + e * 4 + ch, pend[4 * k + ch]);
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < 8; ++k) pend[k] = 0.f;
+  for (int ch = 0; ch < 4; ++ch)
+    if (pend[ch] != 0.f) atomicAdd(p + ch * copies, pend[ch]);
+}
+
+// Adds the pending gradient of entries i and i + 1.
+__device__ __forceinline__ void flush_tf(float* dtf_s, int copies, int n, int i, const float pend[8]) {
+  add_tf_entry(dtf_s, copies, n, i, pend);
+  add_tf_entry(dtf_s, copies, n, i + 1, pend + 4);
 }
 
 // Near-opaque samples.  The closed form for the adjoint of the accumulated
@@ -497,6 +497,16 @@ __device__ __forceinline__ float4 suffix_composite(const TrainArgs& a, const Dev
   return make_float4(r0, r1, r2, tp);
 }
 
+// Copies of the transfer-function gradient in a replaying CTA's shared memory,
+// interleaved (a lane's copy has banks of its own): adding to a float there is a
+// loop until no other lane interferes.  As many as fit kTfCopyBytes, which at 5
+// CTAs per SM leaves the L1 its share.  With one copy / 2 / 4 / 8, ms: one 512^3
+// view's transfer-function step 5.64 / 5.46 / 5.35 / 5.34, 16 views of 128^3, both
+// gradients, 2.39 / 2.31 / 2.27 / 2.27, 2 views of 512^3 13.4 / 13.2 / 13.05 / 13.2;
+// moving a sum along with the lookup index (backward_item) then 5.25, 2.27, 12.9.
+// Bytes, 512 entries, 512^3 backward: 23 KB (1 copy) 5.04, 36 (2) 4.96, 64 (4) 5.09.
+constexpr int kTfCopies = 4;
+constexpr size_t kTfCopyBytes = 36 * 1024;
 constexpr int kBackwardEmptyBlocks = 6;   // CTAs per SM of the all-empty segments' kernel
 constexpr unsigned kBackwardGrab = 256;  // most items a backward warp takes per grab (8 rows of 32)
 
@@ -556,7 +566,16 @@ __device__ __forceinline__ uint32_t backward_item(const TrainArgs& a, const DevV
         const int ic = min(max(i0, -2), a.n_tf);
         const float4 e0 = tf_s[ic + 2], e1 = tf_s[ic + 3];
         if (WITH_TF && i0 != pend_i) {
-          flush_tf(dtf_s, a.n_tf, pend_i, pend);
+          // moved by one entry: one sum is complete, the other moves along
+          const bool up = i0 == pend_i + 1, down = i0 == pend_i - 1;
+          if (!down) add_tf_entry(dtf_s, a.tf_copies, a.n_tf, pend_i, pend);
+          if (!up) add_tf_entry(dtf_s, a.tf_copies, a.n_tf, pend_i + 1, pend + 4);
+#pragma unroll
+          for (int ch = 0; ch < 4; ++ch) {
+            const float lo = pend[ch];
+            pend[ch] = up ? pend[4 + ch] : 0.f;
+            pend[4 + ch] = down ? lo : 0.f;
+          }
           pend_i = i0;
         }
         if (e0.w == 0.f && e1.w == 0.f) {
@@ -596,7 +615,7 @@ __device__ __forceinline__ uint32_t backward_item(const TrainArgs& a, const DevV
         stencil_backward(b, a, __ldg(rb + wcur.j), ux, uy, uz, dv, fmaf(ki, ray.d[0], -kc3 * ex),
                          fmaf(ki, ray.d[1], -kc3 * ey), fmaf(ki, ray.d[2], -kc3 * ez));
       });
-  if (WITH_TF) flush_tf(dtf_s, a.n_tf, pend_i, pend);
+  if (WITH_TF) flush_tf(dtf_s, a.tf_copies, a.n_tf, pend_i, pend);
   // near-opaque samples: correct the alpha adjoint by the true one
   for (int k = 0; k < n_events; ++k) {
     const OpaqueEvent& e = events[k];
@@ -608,8 +627,8 @@ __device__ __forceinline__ uint32_t backward_item(const TrainArgs& a, const DevV
     const int i0 = __float2int_rd(xb);
     const float wt = xb - (float)i0;
     if (WITH_TF) {
-      if (i0 >= 0 && i0 < a.n_tf) atomicAdd(dtf_s + i0 * 4 + 3, (1.f - wt) * dd);
-      if (i0 + 1 >= 0 && i0 + 1 < a.n_tf) atomicAdd(dtf_s + (i0 + 1) * 4 + 3, wt * dd);
+      if (i0 >= 0 && i0 < a.n_tf) atomicAdd(dtf_s + (i0 * 4 + 3) * a.tf_copies, (1.f - wt) * dd);
+      if (i0 + 1 >= 0 && i0 + 1 < a.n_tf) atomicAdd(dtf_s + ((i0 + 1) * 4 + 3) * a.tf_copies, wt * dd);
     }
     if (WITH_DENSITY) {
       const int ic = min(max(i0, -2), a.n_tf);
@@ -637,10 +656,11 @@ template <bool INNER, bool WITH_TF, bool WITH_DENSITY, bool MULTI>
 __global__ void __launch_bounds__(128, 5) backward_kernel(TrainArgs a) {
   extern __shared__ float4 smem[];
   float4* tf_s = smem;                                         // n_tf + 4 entries
-  float* dtf_s = reinterpret_cast<float*>(smem + a.n_tf + 4);  // n_tf * 4 (WITH_TF)
+  float* dtf_all = reinterpret_cast<float*>(smem + a.n_tf + 4);  // n_tf * 4 * tf_copies (WITH_TF)
+  float* dtf_s = WITH_TF ? dtf_all + (threadIdx.x & (a.tf_copies - 1)) : nullptr;
   load_tf(tf_s, a.tf, a.n_tf);
   if (WITH_TF)
-    for (int i = threadIdx.x; i < a.n_tf * 4; i += blockDim.x) dtf_s[i] = 0.f;
+    for (int i = threadIdx.x; i < a.n_tf * 4 * a.tf_copies; i += blockDim.x) dtf_all[i] = 0.f;
   __syncthreads();
   const unsigned count = MULTI ? __ldg(a.item_base + a.n_views) : a.one_items;
   const float nf = (float)a.n_tf;
@@ -693,7 +713,11 @@ __global__ void __launch_bounds__(128, 5) backward_kernel(TrainArgs a) {
   count_samples(a.counter, nsamp);
   if (WITH_TF) {
     __syncthreads();
-    for (int i = threadIdx.x; i < a.n_tf * 4; i += blockDim.x) red_add(a.dtf + i, dtf_s[i]);
+    for (int i = threadIdx.x; i < a.n_tf * 4; i += blockDim.x) {
+      float v = 0.f;
+      for (int c = 0; c < a.tf_copies; ++c) v += dtf_all[i * a.tf_copies + c];
+      red_add(a.dtf + i, v);
+    }
   } else if (a.counter && blockIdx.x == 0) {
     // the samples of all-empty segments, which nothing replays
     for (int i = threadIdx.x; i < a.n_views; i += blockDim.x)
@@ -842,8 +866,14 @@ __global__ void __launch_bounds__(128, kBackwardEmptyBlocks) backward_empty_kern
   }
 }
 
-size_t backward_smem(int n_tf, bool with_tf) {
-  return (size_t)(n_tf + 4) * sizeof(float4) + (with_tf ? (size_t)n_tf * 4 * sizeof(float) : 0);
+size_t backward_smem(int n_tf, int tf_copies) {
+  return (size_t)(n_tf + 4) * sizeof(float4) + (size_t)n_tf * 4 * sizeof(float) * tf_copies;
+}
+
+int backward_tf_copies(int n_tf) {
+  for (int copies = kTfCopies; copies > 1; copies /= 2)
+    if (backward_smem(n_tf, copies) <= kTfCopyBytes) return copies;
+  return 1;
 }
 
 }  // namespace
@@ -879,10 +909,12 @@ static BackwardKernel backward(bool with_tf, bool with_density, bool multi) {
                   : (with_density ? backward_kernel<INNER, true, true, false> : backward_kernel<INNER, true, false, false>);
 }
 
-cudaError_t launch_backward(const TrainArgs& a, int grid, bool inner, cudaStream_t s) {
+cudaError_t launch_backward(const TrainArgs& args, int grid, bool inner, cudaStream_t s) {
+  TrainArgs a = args;
   const bool with_tf = a.dtf != nullptr, with_density = a.dgrid4 != nullptr;
+  a.tf_copies = with_tf ? backward_tf_copies(a.n_tf) : 0;
   if (!with_tf && !with_density) return cudaErrorInvalidValue;
-  const size_t smem = backward_smem(a.n_tf, with_tf);
+  const size_t smem = backward_smem(a.n_tf, a.tf_copies);
   const bool multi = a.n_views > 1;
   const BackwardKernel k = inner ? backward<true>(with_tf, with_density, multi) : backward<false>(with_tf, with_density, multi);
   if (smem > 48 * 1024) {
@@ -927,7 +959,7 @@ cudaError_t launch_fold_quads(float4* quads, float* out, const int dims[3], cuda
 
 int backward_blocks_per_sm(int n_tf) {
   // the instance with the transfer-function gradient needs more shared memory
-  const size_t smem = backward_smem(n_tf, true);
+  const size_t smem = backward_smem(n_tf, backward_tf_copies(n_tf));
   if (smem > 48 * 1024 &&
       cudaFuncSetAttribute(backward_kernel<true, true, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
           cudaSuccess) {

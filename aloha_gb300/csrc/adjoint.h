@@ -74,6 +74,7 @@ struct TrainArgs {
   TrainView one;
   unsigned one_items, one_empty;
   float* dtf;                 // [n_tf*4] accumulated
+  int tf_copies;              // copies of it in a CTA's shared memory, interleaved (launch_backward)
   float4* dgrid4;             // density gradient in x-quads: element (x,y,z) holds the
                               // contributions to voxels x, x+1, x+2 (w unused)
   const int4* brick_grid_origin;  // per brick: voxelRange.lower - grid_lo
