@@ -732,7 +732,7 @@ __global__ void __launch_bounds__(128, 5) backward_kernel(TrainArgs a) {
 // waits for the one before it and nothing here has to round as the forward
 // does: no composite, an approximate reciprocal square root in the shading, two
 // pending sums instead of eight.  Bound by the L1 data pipe (83 % busy), mostly
-// with the stencil's 112 bytes per sample: so two lanes take a segment's samples
+// with the stencil's 96 bytes per sample: so two lanes take a segment's samples
 // in turn, and a quarter warp, the unit of 16-byte loads, covers 2x2 rays by two
 // samples, whose quads collide in fewer banks than those of 2x4 rays (a model of
 // the pipe, confirmed for the first: 55 -> 41 cycles for a warp's seven loads at

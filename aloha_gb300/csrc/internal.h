@@ -11,7 +11,7 @@ namespace aloha {
 // Padded brick storage: every brick is stored with an apron of kApron voxels
 // on each side, filled with the clamped edge values (cudaAddressModeClamp of
 // waikikiRenderer.cpp:753-755), so the march loop needs no per-tap clamps.
-// Each stored element is a yz-quad: the float4 (V(x,y,z), V(x,y,z+1),
+// Each stored element is a zy-quad: the float4 (V(x,y,z), V(x,y,z+1),
 // V(x,y+1,z), V(x,y+1,z+1)) (indices clamped), so one 16-byte load fetches a
 // voxel's 2x2 (y, z) neighbourhood, its halves are (z, z+1) pairs that packed
 // fp32x2 instructions interpolate together, and the stencil's core comes from three
@@ -76,7 +76,7 @@ constexpr float kInnerSpace = 16384.0f, kInnerEye = 32768.0f, kInnerValue = 1024
 
 // One brick as the kernels see it (80 bytes).
 struct DevBrick {
-  const float4* base;    // yz-quad of voxel (0,0,0) of the voxel range inside the padded array
+  const float4* base;    // quad of voxel (0,0,0) of the voxel range inside the padded array
   const uint8_t* cells;  // [mz][my][mx] macrocell codes
   int sy, sz;            // padded row and slice pitch, in quads
   int n[3];              // voxel range size

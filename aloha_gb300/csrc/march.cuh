@@ -10,7 +10,7 @@
 // tap is the trilinear interpolation at u, the six gradient taps sit at
 // u +- 1/2 (the reference's tc +- 0.5/N, deviceCode.cpp:278-284).  u - 1/2 and
 // u + 1/2 differ by exactly 1, so all seven taps read one 20-voxel cross
-// around the cell and share their fractional weights.  With the yz-quad brick
+// around the cell and share their fractional weights.  With the zy-quad brick
 // layout (each element holds a voxel's 2x2 (y, z) neighbourhood) the cross is
 // five 16-byte and two 8-byte loads per sample (56 texel fetches in the
 // reference).
@@ -317,7 +317,7 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 
 // Shared memory of the staged loads: [2 slots][7 rows][kRenderThreads] float4
 // (each thread's rows strided by the CTA size, so a warp's row reads are
-// contiguous): the seven yz-quads of stencil(), in its order.
+// contiguous): the seven zy-quads of stencil(), in its order.
 constexpr int kStageRows = 7;
 constexpr size_t kStageBytes = (size_t)2 * kStageRows * kRenderThreads * sizeof(float4);
 

@@ -415,10 +415,10 @@ def main():
     kernel = ("render_split_kernel" if split == abi.SPLIT_RANKS else
               f"render_warps_kernel<{tw},{th},5,{stage}{',4' if lg else ''}>")
     # our kernels per frame: the render, plus the chunk probe (which also
-    # counts the classes), scan and scatter of the cost order, and for the
+    # counts the classes) and scatter of the cost order, and for the
     # rank split its mask, three scan kernels and emit
     probed = chunks == abi.CHUNKS_PROBED or (chunks == abi.CHUNKS_AUTO and W * H >= 512 * 512)
-    launches_per_frame = (6 if split == abi.SPLIT_RANKS else 1) + (2 if probed else 0)  # probe and scatter
+    launches_per_frame = (6 if split == abi.SPLIT_RANKS else 1) + (2 if probed else 0)
 
     steps = [mine[k % len(mine)] for k in range(args.steps)]
     for k in range(args.warmup):
