@@ -245,7 +245,8 @@ cudaError_t launch_fill_brick(const DevBrick& b, const float* src, float4* dst_a
 // Persistent render launch; `batch` selects the instance tuned for batches.
 constexpr int kSingleRenderBlocks = 5, kBatchRenderBlocks = 7;  // CTAs per SM
 // A single view of few 8x4 chunks per resident warp ends on its longest rays,
-// which run faster with fewer, less spilling neighbours (4 / 5 CTAs per SM, us:
+// which run faster with fewer, less spilling neighbours (4 / 5 CTAs per SM, us,
+// one lane per ray:
 // 64^3 at 512^2 81 / 89, 256^3 at 1024x768 257 / 263, 512^3 at 512^2 599 / 633);
 // with many, throughput counts (64^3 at 1024^2 155 / 146, 256^3 at 1280x1024 354
 // / 331, 512^3 at 1920x1080 650 / 630; 512^3 at 1024^2, 10.8 chunks per warp of
