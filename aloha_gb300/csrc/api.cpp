@@ -880,16 +880,21 @@ int aloha_set_render_params(aloha_ctx* c, const aloha_render_params* p) {
   return ALOHA_OK;
 }
 
-// Uploads one brick's voxels into its padded slot.
+// Brings the device's scene_inner up to date.  The kernels drop their clamps on
+// its word, so it has to be there when the call returns: a copy from pageable
+// memory returns before it has landed, and streams that do not wait for the
+// default stream would still read the old value.
 static int upload_scene_inner(aloha_ctx* c) {
   int all = 1;
   for (const DevBrick& b : c->dev_bricks) all &= b.inner;
   if (all == c->scene_inner_host) return ALOHA_OK;
   CUDA_TRY(c, cudaMemcpy(c->scene_inner.ptr, &all, sizeof all, cudaMemcpyHostToDevice));
+  CUDA_TRY(c, cudaStreamSynchronize(0));
   c->scene_inner_host = all;
   return ALOHA_OK;
 }
 
+// Uploads one brick's voxels into its padded slot.
 static int upload_brick(aloha_ctx* c, int b, const float* src) {
   const aloha_brick_desc& d = c->descs[b];
   const int nx = d.voxel_hi[0] - d.voxel_lo[0], ny = d.voxel_hi[1] - d.voxel_lo[1], nz = d.voxel_hi[2] - d.voxel_lo[2];
@@ -1000,14 +1005,18 @@ int aloha_set_bricks(aloha_ctx* c, const aloha_brick_desc* descs, const float* c
     }
   CUDA_TRY(c, c->bricks_dev.ensure(sizeof(DevBrick) * n));
   CUDA_TRY(c, cudaMemcpy(c->bricks_dev.ptr, db.data(), sizeof(DevBrick) * n, cudaMemcpyHostToDevice));
+  // what the boxes say goes first: a launch recorded earlier may be replayed
+  // even if a brick below is refused
+  int rc = upload_scene_inner(c);
+  if (rc) return rc;
   for (int b = 0; b < n; ++b) {
-    int rc = upload_brick(c, b, voxels[b]);
+    rc = upload_brick(c, b, voxels[b]);
     if (rc) {
       c->descs.clear();
       return rc;
     }
   }
-  int rc = upload_scene_inner(c);
+  rc = upload_scene_inner(c);
   if (rc) return rc;
   c->staging_in.release();
   c->sched_stride = 0;

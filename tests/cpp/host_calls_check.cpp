@@ -1,0 +1,93 @@
+// Checks of what the host side of the C ABI (api.cpp) leaves done when a call
+// returns, on a stand-in for the CUDA runtime.  Arguments: the checks to run.
+// Prints one line per failure; status 1 if there was any.
+#include <string>
+
+#include "aloha.h"
+#include "fake_cuda.h"
+
+namespace {
+
+int failures = 0;
+#define CHECK(cond)                                                        \
+  do {                                                                     \
+    if (!(cond)) {                                                         \
+      std::printf("%s:%d: %s\n", __FILE__, __LINE__, #cond);               \
+      ++failures;                                                          \
+    }                                                                      \
+  } while (0)
+
+const cudaStream_t kSide = reinterpret_cast<cudaStream_t>(0x1000);
+
+aloha_brick_desc brick(int nx, int ny, int nz, float grow = 0.0f) {
+  aloha_brick_desc d{};
+  const int n[3] = {nx, ny, nz};
+  for (int a = 0; a < 3; ++a) {
+    d.voxel_hi[a] = d.cell_hi[a] = n[a];
+    d.space_lo[a] = -grow;
+    d.space_hi[a] = (float)n[a] + grow;
+  }
+  return d;
+}
+
+void* device(size_t bytes) {
+  void* p = nullptr;
+  cudaMalloc(&p, bytes);
+  return p;
+}
+
+// A context with a camera, a size and a table, ready to render.
+aloha_ctx* context(const aloha_brick_desc& d, const float* voxels) {
+  aloha_ctx* c = nullptr;
+  CHECK(aloha_create(0, &c) == ALOHA_OK);
+  const float tf[8] = {0, 0, 0, 0, 1, 1, 1, 1};
+  CHECK(aloha_set_bricks(c, &d, &voxels, 1) == ALOHA_OK);
+  CHECK(aloha_set_transfer_function(c, tf, 2) == ALOHA_OK);
+  const float org[3] = {4, 4, -20}, d00[3] = {-0.4f, -0.4f, 1}, du[3] = {0.1f, 0, 0}, dv[3] = {0, 0.1f, 0};
+  CHECK(aloha_set_camera(c, 0, org, d00, du, dv) == ALOHA_OK);
+  CHECK(aloha_resize(c, 0, 8, 8) == ALOHA_OK);
+  return c;
+}
+
+// The flag that lets kernels drop their clamps is the scene's when a render is
+// launched on any stream, also one that does not wait for the default stream.
+void scene_flag() {
+  const float* voxels = static_cast<const float*>(device(8 * 8 * 8 * 4));
+  uint32_t* fb = static_cast<uint32_t*>(device(8 * 8 * 4));
+  const aloha_brick_desc inside = brick(8, 8, 8), beyond = brick(8, 8, 8, 1.0f);
+  aloha_ctx* c = context(inside, voxels);
+  auto inner = [&] {
+    CHECK(aloha_render(c, 0, fb, kSide) == ALOHA_OK);
+    return fake::rendered_inner.back();
+  };
+  CHECK(inner() == 1);
+  CHECK(aloha_set_bricks(c, &beyond, &voxels, 1) == ALOHA_OK);
+  CHECK(inner() == 0);
+  CHECK(aloha_set_bricks(c, &inside, &voxels, 1) == ALOHA_OK);
+  CHECK(inner() == 1);
+  fake::fill_flags = aloha::kVoxelWide;
+  CHECK(aloha_update_brick(c, 0, voxels) == ALOHA_OK);
+  CHECK(inner() == 0);
+  fake::fill_flags = 0;
+  CHECK(aloha_update_brick(c, 0, voxels) == ALOHA_OK);
+  CHECK(inner() == 1);
+  // bricks that are refused half-way: a recorded launch may still be replayed
+  fake::fill_flags = aloha::kVoxelNonfinite;
+  const int* flag = fake::renders.back().f.scene_inner;
+  CHECK(aloha_set_bricks(c, &beyond, &voxels, 1) == ALOHA_ERR_INVALID_ARGUMENT);
+  CHECK(*flag == 0);
+  fake::fill_flags = 0;
+  aloha_destroy(c);
+}
+
+}  // namespace
+
+int main(int argc, char** argv) {
+  for (int i = 1; i < argc; ++i) {
+    const std::string a = argv[i];
+    if (a == "scene_flag") scene_flag();
+    else ++failures;
+  }
+  std::printf("failures %d\n", failures);
+  return failures == 0 ? 0 : 1;
+}
