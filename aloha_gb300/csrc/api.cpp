@@ -1062,6 +1062,7 @@ int aloha_set_transfer_function(aloha_ctx* c, const float* rgba, int n) {
   }
   CUDA_TRY(c, c->tf.ensure(h.size() * sizeof(float)));
   CUDA_TRY(c, cudaMemcpy(c->tf.ptr, h.data(), h.size() * sizeof(float), cudaMemcpyHostToDevice));
+  CUDA_TRY(c, cudaStreamSynchronize(0));  // landed, for renders on streams that do not wait for this one
   c->empty_dirty = true;
   c->n_tf = n;
   invalidate_training(c);

@@ -80,12 +80,30 @@ void scene_flag() {
   aloha_destroy(c);
 }
 
+// The table is on the device when the call returns.
+void table() {
+  const float* voxels = static_cast<const float*>(device(8 * 8 * 8 * 4));
+  uint32_t* fb = static_cast<uint32_t*>(device(8 * 8 * 4));
+  aloha_ctx* c = context(brick(8, 8, 8), voxels);
+  CHECK(aloha_render(c, 0, fb, kSide) == ALOHA_OK);
+  const float4* tf = fake::renders.back().f.tf;
+  for (int k = 0; k < 3; ++k) {
+    const float rgba[8] = {0.25f * k, 0, 0, 0, 1, 1, 0.5f * k, 1};
+    CHECK(aloha_set_transfer_function(c, rgba, 2) == ALOHA_OK);
+    CHECK(std::memcmp(tf, rgba, sizeof rgba) == 0);
+    const int want[3] = {0, 0, 1};  // entries of non-zero alpha before each
+    CHECK(std::memcmp(tf + 2, want, sizeof want) == 0);
+  }
+  aloha_destroy(c);
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
   for (int i = 1; i < argc; ++i) {
     const std::string a = argv[i];
     if (a == "scene_flag") scene_flag();
+    else if (a == "table") table();
     else ++failures;
   }
   std::printf("failures %d\n", failures);

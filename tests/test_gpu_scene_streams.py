@@ -58,3 +58,12 @@ def test_bricks_that_change_the_form_of_the_march(scene):
         expect(plain, wide, tf)
         ctx.update_brick(0, dev)
         expect(plain, vol, tf)
+
+
+def test_tables(scene):
+    ctx, torch, plain, tf, expect = scene
+    vol = volume(83)
+    for n in (16, 2048, 100, 256):
+        table = S.seeded_tf(n, n)
+        ctx.set_transfer_function(table)
+        expect(plain, vol, table)
