@@ -136,16 +136,18 @@ ALOHA_HD float estimate_div(float a, float b) {
 // between two multiples: then the sum rounds to an even one, and from an even t
 // on the step is fixed again.  Two equal steps in a row (t to t1, t1 to t1 +
 // dt) therefore stay equal up to the binade's end; otherwise, and across the
-// end, single steps are taken as the loop takes them.  A 200^3 volume at
-// 700x400 and dt 0.3: 300 us with the loop, 276 this way, 267 at dt 0.3125
-// (run_steps).
+// end, single steps are taken as the loop takes them.  So are all steps from a
+// negative t, whose binade ends towards zero, with finer ones after it: a march
+// starts there when a constant jitter of 10^7 steps or more rounds its first
+// sample to before the eye.  A 200^3 volume at 700x400 and dt 0.3: 300 us with
+// the loop, 276 this way, 267 at dt 0.3125 (run_steps).
 ALOHA_HD uint32_t run_steps_any(float& t, uint32_t& n, float tb, uint32_t cap, float dt, uint32_t max_steps) {
   uint32_t k = 0;
   while (k < max_steps && t < tb && n < cap) {
     const uint32_t lim = (max_steps - k) < (cap - n) ? (max_steps - k) : (cap - n);
     const float t1 = t + dt;
     const float step = t1 - t;
-    if (step > 0.0f && (t1 + dt) - t1 == step) {
+    if (t >= 0.0f && step > 0.0f && (t1 + dt) - t1 == step) {
       const float d = t - bits_float((float_bits(t) & 0x7f800000u) + 0x00800000u);  // t - B, exact, < 0
       const float kf = fminf(fmaxf(ceilf(estimate_div(tb - t, step)), 1.0f), 4194304.0f);
       uint32_t j = (uint32_t)kf < lim ? (uint32_t)kf : lim;
