@@ -97,14 +97,17 @@ struct PinnedBuffer {
 
 bool finite3(const float* v) { return std::isfinite(v[0]) && std::isfinite(v[1]) && std::isfinite(v[2]); }
 
-bool is_device_pointer(const void* p) {
+cudaMemoryType memory_of(const void* p) {
   cudaPointerAttributes attr;
   if (cudaPointerGetAttributes(&attr, p) != cudaSuccess) {
     cudaGetLastError();
-    return false;
+    return cudaMemoryTypeUnregistered;
   }
-  return attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged;
+  return attr.type;
 }
+
+bool is_device_memory(cudaMemoryType t) { return t == cudaMemoryTypeDevice || t == cudaMemoryTypeManaged; }
+bool is_device_pointer(const void* p) { return is_device_memory(memory_of(p)); }
 
 // Where an output buffer lives, from one pointer query: device memory, or
 // host memory with the device address of page-locked memory registered with
@@ -1288,21 +1291,25 @@ static int composite_common(const void* imgs, size_t img_bytes, const int* order
     if (r < 0 || r >= n_ranks) return ALOHA_ERR_OUT_OF_RANGE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const size_t npx = (size_t)width * height;
-  const bool host_in = !is_device_pointer(imgs), host_out = !is_device_pointer(fb);
+  const cudaMemoryType in_memory = memory_of(imgs), out_memory = memory_of(fb);
+  const bool host_in = !is_device_memory(in_memory), host_out = !is_device_memory(out_memory);
   if (!host_in && !host_out && n_ranks <= kParamRanks) {
     // device images and frame buffer: the order goes in the launch parameters,
-    // nothing is allocated and nothing waits (a stream under capture is refused
-    // below, as the allocation has always done)
+    // nothing is allocated, and only managed memory, which the host reads and
+    // writes as well, is waited for (a stream under capture is refused below, as
+    // the allocation has always done)
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
       cudaGetLastError();
       cs = cudaStreamCaptureStatusActive;
     }
     if (cs == cudaStreamCaptureStatusNone) {
-      const cudaError_t e =
+      cudaError_t e =
           u8 ? launch_composite_u8(static_cast<const uint32_t*>(imgs), nullptr, h_order.data(), n_ranks, (int)npx, fb, s)
              : launch_composite_f32(static_cast<const float4*>(imgs), nullptr, h_order.data(), n_ranks, (int)npx, mode, fb,
                                     s);
+      if (e == cudaSuccess && (in_memory == cudaMemoryTypeManaged || out_memory == cudaMemoryTypeManaged))
+        e = cudaStreamSynchronize(s);
       return e == cudaSuccess ? ALOHA_OK : ALOHA_ERR_CUDA;
     }
   }

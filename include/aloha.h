@@ -211,12 +211,18 @@ int aloha_render_partials(aloha_ctx* ctx, int view, float* rank_images, float* r
 /* IceT stand-in: blend n_ranks float RGBA images front to back in `order`
  * (ordered BLEND, waikikiRenderer.cpp:910-917,1042-1079) into RGBA8.  Mode
  * ALOHA_COMPOSITE_FP32 blends in fp32 and rounds once; _UBYTE quantises each
- * image first and blends in 8 bits.  Context-free. */
+ * image first and blends in 8 bits.  Context-free.  With images and fb in
+ * device memory, at most 1024 ranks and a stream that is not being captured,
+ * the call only enqueues the blend: order the reading of fb, and the release
+ * or reuse of both, after it on `stream`, and find a failure of the kernel in
+ * the stream's next status.  With any of them in host or managed memory the
+ * call returns after the stream has finished. */
 int aloha_composite_over(const float* rank_images, const int* order, int n_ranks, int width, int height,
                          int mode, uint32_t* fb, void* stream);
 
 /* IceT stand-in for external RGBA8 rank images ([n_ranks][height][width]
- * uint32, premultiplied), blended in 8 bits front to back in `order`. */
+ * uint32, premultiplied), blended in 8 bits front to back in `order`; waits as
+ * aloha_composite_over does. */
 int aloha_composite_over_rgba8(const uint32_t* rank_fbs, const int* order, int n_ranks, int width, int height,
                                uint32_t* fb, void* stream);
 

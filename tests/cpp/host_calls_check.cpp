@@ -97,6 +97,31 @@ void table() {
   aloha_destroy(c);
 }
 
+// The composite waits for its stream unless images and frame buffer are plain
+// device memory.
+void composite() {
+  const int w = 16, h = 8, n = 3, order[n] = {2, 0, 1};
+  const size_t in_bytes = (size_t)n * w * h * 16, out_bytes = (size_t)w * h * 4;
+  void *dev_in = device(in_bytes), *dev_out = device(out_bytes), *man_in = nullptr, *man_out = nullptr;
+  fake::reserve(&man_in, in_bytes, cudaMemoryTypeManaged);
+  fake::reserve(&man_out, out_bytes, cudaMemoryTypeManaged);
+  std::vector<char> host_in(in_bytes), host_out(out_bytes);
+  for (bool u8 : {false, true})
+    for (void* in : {dev_in, man_in, (void*)host_in.data()})
+      for (void* out : {dev_out, man_out, (void*)host_out.data()}) {
+        std::memset(out, 0, out_bytes);
+        const int waits = fake::waits;
+        const int rc = u8 ? aloha_composite_over_rgba8((uint32_t*)in, order, n, w, h, (uint32_t*)out, kSide)
+                          : aloha_composite_over((float*)in, order, n, w, h, ALOHA_COMPOSITE_FP32, (uint32_t*)out, kSide);
+        CHECK(rc == ALOHA_OK);
+        if (in != dev_in || out != dev_out)
+          CHECK(*(uint32_t*)out == 0x5a5a5a5au);
+        else
+          CHECK(fake::waits == waits);
+        fake::wait_all();
+      }
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -104,6 +129,7 @@ int main(int argc, char** argv) {
     const std::string a = argv[i];
     if (a == "scene_flag") scene_flag();
     else if (a == "table") table();
+    else if (a == "composite") composite();
     else ++failures;
   }
   std::printf("failures %d\n", failures);
