@@ -413,14 +413,21 @@ class Batch:
             pass
 
 
-def _wait_elsewhere(stream, *buffers):
-    """Waits for `stream` if it is not torch's current one and a buffer is a CUDA
-    tensor: the library's call has only been enqueued there, and the tensor's
-    memory may be given to work on the current stream once it is freed."""
-    if any(getattr(b, "is_cuda", False) for b in buffers):
-        import torch
-        if _stream(stream) != torch.cuda.current_stream().cuda_stream:
-            torch.cuda.ExternalStream(_stream(stream)).synchronize()
+def _hand_over(stream, *buffers):
+    """After a call that has only been enqueued on `stream`: keeps its device
+    buffers from being given to other work before it is done.  Tensors are recorded
+    on the stream if it is torch's current one (their memory goes back to the stream
+    that they were allocated on, which may be another); else the stream is waited for."""
+    device = [b for b in buffers if getattr(b, "is_cuda", hasattr(b, "data_ptr"))]
+    if not device:
+        return
+    import torch
+    current = torch.cuda.current_stream()
+    if _stream(stream) == current.cuda_stream and all(isinstance(b, torch.Tensor) for b in device):
+        for b in device:
+            b.record_stream(current)
+    else:
+        torch.cuda.ExternalStream(_stream(stream)).synchronize()
 
 
 def composite_over(rank_images, order, width: int, height: int, mode: int = COMPOSITE_FP32, fb=None, stream=None):
@@ -433,7 +440,7 @@ def composite_over(rank_images, order, width: int, height: int, mode: int = COMP
                                 _stream(stream))
     if rc != OK:
         raise AlohaError(rc, L.aloha_status_string(rc).decode())
-    _wait_elsewhere(stream, rank_images, fb)
+    _hand_over(stream, rank_images, fb)
     return fb
 
 
@@ -445,5 +452,5 @@ def composite_over_rgba8(rank_fbs, order, width: int, height: int, fb=None, stre
     rc = L.aloha_composite_over_rgba8(_addr(rank_fbs), _addr(o), o.size, width, height, _addr(fb), _stream(stream))
     if rc != OK:
         raise AlohaError(rc, L.aloha_status_string(rc).decode())
-    _wait_elsewhere(stream, rank_fbs, fb)
+    _hand_over(stream, rank_fbs, fb)
     return fb
