@@ -947,15 +947,8 @@ int aloha_set_bricks(aloha_ctx* c, const aloha_brick_desc* descs, const float* c
       if (!(std::isfinite(d.space_lo[a]) && std::isfinite(d.space_hi[a]) && d.space_lo[a] < d.space_hi[a]))
         return c->fail(ALOHA_ERR_INVALID_ARGUMENT, "brick %d: empty or non-finite space range", b);
     }
-    const int px = row_pitch(nsz[0]), pz = nsz[2] + 2 * kApron;
-    const long long slice = slice_pitch(px, nsz[1]);
-    const size_t elems = (size_t)slice * pz;
-    if (elems >= (size_t)1 << 31)
+    if (plain_pitch(nsz[0], nsz[1]).quads(nsz[2]) > kMaxBrickQuads)
       return c->fail(ALOHA_ERR_INVALID_ARGUMENT, "brick %d too large for 32-bit voxel offsets; split it", b);
-    offs[b] = total;
-    total += (elems + 15) & ~(size_t)15;  // 256-byte aligned bricks (in quads)
-    db[b].sy = px;
-    db[b].sz = (int)slice;
     for (int a = 0; a < 3; ++a) {
       db[b].n[a] = nsz[a];
       db[b].lo[a] = (float)d.voxel_lo[a];
@@ -968,8 +961,30 @@ int aloha_set_bricks(aloha_ctx* c, const aloha_brick_desc* descs, const float* c
     }
     db[b].inner = inner_box[b];  // unless its values are too large (upload_brick)
   }
+  std::vector<size_t> mc_off(n);
+  size_t mc_total = 0;
+  for (int b = 0; b < n; ++b) {
+    mc_off[b] = mc_total;
+    mc_total += (size_t)macrocells(db[b]);
+  }
+  const size_t range_bytes = mc_total * sizeof(float2), code_bytes = 2 * mc_total;  // the codes, then scratch
+  auto lay_out = [&](bool spread) {
+    total = 0;
+    for (int b = 0; b < n; ++b) {
+      const int* nsz = db[b].n;
+      BrickPitch p = spread_pitch(nsz[0], nsz[1]);
+      if (!spread || p.quads(nsz[2]) > kMaxBrickQuads) p = plain_pitch(nsz[0], nsz[1]);
+      offs[b] = total;
+      total += ((size_t)p.quads(nsz[2]) + 15) & ~(size_t)15;  // 256-byte aligned bricks (in quads)
+      db[b].sy = p.row;
+      db[b].sz = (int)p.slice;
+    }
+  };
   size_t free_b = 0, total_b = 0;
   CUDA_TRY(c, cudaMemGetInfo(&free_b, &total_b));
+  lay_out(true);
+  if (total * sizeof(float4) + range_bytes + code_bytes > free_b + c->voxels.bytes + c->mc_ranges.bytes + c->mc_codes.bytes)
+    lay_out(false);
   if (total * sizeof(float4) > free_b + c->voxels.bytes)
     return c->fail(ALOHA_ERR_OUT_OF_MEMORY, "bricks need %zu bytes, %zu free", total * sizeof(float4), free_b);
   CUDA_TRY(c, cudaDeviceSynchronize());
@@ -977,14 +992,8 @@ int aloha_set_bricks(aloha_ctx* c, const aloha_brick_desc* descs, const float* c
   for (int b = 0; b < n; ++b)
     db[b].base = static_cast<const float4*>(c->voxels.ptr) + offs[b] + (size_t)kApron * db[b].sz +
                  (size_t)kApron * db[b].sy + kApron;
-  std::vector<size_t> mc_off(n);
-  size_t mc_total = 0;
-  for (int b = 0; b < n; ++b) {
-    mc_off[b] = mc_total;
-    mc_total += (size_t)macrocells(db[b]);
-  }
-  CUDA_TRY(c, c->mc_ranges.ensure(mc_total * sizeof(float2)));
-  CUDA_TRY(c, c->mc_codes.ensure(2 * mc_total));  // the codes, then scratch
+  CUDA_TRY(c, c->mc_ranges.ensure(range_bytes));
+  CUDA_TRY(c, c->mc_codes.ensure(code_bytes));
   for (int b = 0; b < n; ++b) db[b].cells = static_cast<const uint8_t*>(c->mc_codes.ptr) + mc_off[b];
   c->mc_offset = mc_off;
   c->mc_total = mc_total;

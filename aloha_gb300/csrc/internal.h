@@ -29,13 +29,24 @@ constexpr int kApron = 2;
 // pixel row that ran along z collided.  Together with the 2x4 quarter warps
 // of tile_x / tile_y: uneven 24-view batch 10.46 -> 10.01 ms, 512^3
 // transfer-function step 6.35 -> 6.16 ms, odd volume's frame 681 -> 626 us.
-inline int row_pitch(int nx) {
-  const int px = nx + 2 * kApron;
-  return px + ((2 - px) & 3);
+// A brick that fits kMaxBrickQuads without this padding only (1024 x 1440 x
+// 1440), and a scene that fits the device's memory without it only, take plain
+// pitches: rows of an even number of
+// quads, slices of their product.
+struct BrickPitch {
+  int row;
+  long long slice;
+  long long quads(int nz) const { return slice * (nz + 2 * kApron); }
+};
+constexpr long long kMaxBrickQuads = (1ll << 31) - 1;  // element offsets are ints
+inline BrickPitch plain_pitch(int nx, int ny) {
+  const int row = (nx + 2 * kApron + 1) & ~1;
+  return {row, (long long)row * (ny + 2 * kApron)};
 }
-inline long long slice_pitch(int px, int ny) {
-  const long long sz = (long long)px * (ny + 2 * kApron);
-  return sz + ((4 - sz) & 7);
+inline BrickPitch spread_pitch(int nx, int ny) {
+  const int px = nx + 2 * kApron, row = px + ((2 - px) & 3);
+  const long long slice = (long long)row * (ny + 2 * kApron);
+  return {row, slice + ((4 - slice) & 7)};
 }
 constexpr int kMaxViews = 4096;
 constexpr int kMaxTF = 2048;  // (n + 4) float4 entries stay under 48 KB of shared memory

@@ -122,6 +122,43 @@ void composite() {
       }
 }
 
+// Bricks up to 2^31 quads of plain pitches, and scenes up to the device's
+// memory of them, are taken.
+void large() {
+  const float* voxels = static_cast<const float*>(device(4096));
+  aloha_ctx* c = nullptr;
+  CHECK(aloha_create(0, &c) == ALOHA_OK);
+  auto set = [&](int nx, int ny, int nz) {
+    const aloha_brick_desc d = brick(nx, ny, nz);
+    return aloha_set_bricks(c, &d, &voxels, 1);
+  };
+  const int sizes[][3] = {{1024, 1440, 1440}, {512, 2036, 2036}, {256, 2860, 2860}, {1, 1, 1}, {128, 128, 128}};
+  for (const auto& n : sizes) {
+    CHECK(set(n[0], n[1], n[2]) == ALOHA_OK);
+    aloha_stats st;
+    CHECK(aloha_get_stats(c, &st) == ALOHA_OK);
+    const long long plain = aloha::plain_pitch(n[0], n[1]).quads(n[2]);
+    CHECK(plain <= aloha::kMaxBrickQuads && st.brick_bytes >= (size_t)plain * 16);
+  }
+  CHECK(set(1025, 1440, 1440) == ALOHA_ERR_INVALID_ARGUMENT);
+  CHECK(set(1024, 1443, 1440) == ALOHA_ERR_INVALID_ARGUMENT);
+  aloha_destroy(c);
+  // memory for plain pitches only: 124^3 is 128^3 quads, padded 130 x 128 + 4
+  CHECK(aloha_create(0, &c) == ALOHA_OK);
+  const size_t plain = (size_t)128 * 128 * 128 * 16, padded = (size_t)(130 * 128 + 4) * 128 * 16, cells = 31 * 31 * 31;
+  CHECK((size_t)aloha::spread_pitch(124, 124).quads(124) * 16 == padded);
+  const size_t all = fake::device_bytes;
+  fake::device_bytes = fake::device_used + plain + 10 * cells + 65536;
+  CHECK(set(124, 124, 124) == ALOHA_OK);
+  fake::device_bytes = fake::device_used - 65536;
+  CHECK(set(128, 124, 124) == ALOHA_ERR_OUT_OF_MEMORY);
+  fake::device_bytes = all;
+  CHECK(set(124, 124, 124) == ALOHA_OK);
+  aloha_stats st;
+  CHECK(aloha_get_stats(c, &st) == ALOHA_OK && st.brick_bytes >= padded);
+  aloha_destroy(c);
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -130,6 +167,7 @@ int main(int argc, char** argv) {
     if (a == "scene_flag") scene_flag();
     else if (a == "table") table();
     else if (a == "composite") composite();
+    else if (a == "large") large();
     else ++failures;
   }
   std::printf("failures %d\n", failures);
