@@ -146,7 +146,7 @@ struct aloha_ctx {
   std::vector<char> brick_inner_box;  // the box part of DevBrick::inner
   std::vector<size_t> brick_offset;  // quad offset of each padded brick in `voxels`
   DeviceBuffer voxels, bricks_dev, staging_in;
-  DeviceBuffer scene_inner;  // int: every brick is InnerCoords
+  DeviceBuffer scene_inner;  // int: scene_is_inner
   PinnedBuffer upload_flags;  // int the upload kernel sets (kVoxel*)
   int* upload_flags_dev = nullptr;
   int scene_inner_host = 0;
@@ -154,6 +154,7 @@ struct aloha_ctx {
   // transfer function
   DeviceBuffer tf;
   int n_tf = 0;
+  bool tf_inner = true;  // entries within +-kInnerTable
   // empty-space macrocells: value range per macrocell (per brick) and the
   // per-transfer-function empty mask, refreshed before the next render
   DeviceBuffer mc_ranges, mc_codes;
@@ -883,13 +884,19 @@ int aloha_set_render_params(aloha_ctx* c, const aloha_render_params* p) {
   return ALOHA_OK;
 }
 
+// InnerCoords, as far as bricks and transfer function go.
+static bool scene_is_inner(const aloha_ctx* c) {
+  bool all = c->tf_inner;
+  for (const DevBrick& b : c->dev_bricks) all = all && b.inner;
+  return all;
+}
+
 // Brings the device's scene_inner up to date.  The kernels drop their clamps on
 // its word, so it has to be there when the call returns: a copy from pageable
 // memory returns before it has landed, and streams that do not wait for the
 // default stream would still read the old value.
 static int upload_scene_inner(aloha_ctx* c) {
-  int all = 1;
-  for (const DevBrick& b : c->dev_bricks) all &= b.inner;
+  const int all = scene_is_inner(c);
   if (all == c->scene_inner_host) return ALOHA_OK;
   CUDA_TRY(c, cudaMemcpy(c->scene_inner.ptr, &all, sizeof all, cudaMemcpyHostToDevice));
   CUDA_TRY(c, cudaStreamSynchronize(0));
@@ -1077,8 +1084,9 @@ int aloha_set_transfer_function(aloha_ctx* c, const float* rgba, int n) {
   CUDA_TRY(c, cudaStreamSynchronize(0));  // landed, for renders on streams that do not wait for this one
   c->empty_dirty = true;
   c->n_tf = n;
+  c->tf_inner = std::all_of(h.begin(), h.begin() + entries, [](float v) { return std::fabs(v) <= kInnerTable; });
   invalidate_training(c);
-  return ALOHA_OK;
+  return c->dev_bricks.empty() ? ALOHA_OK : upload_scene_inner(c);
 }
 
 int aloha_set_ranks(aloha_ctx* c, int n_ranks) {
@@ -1425,8 +1433,7 @@ TrainArgs train_args(aloha_ctx* c) {
 // graph and replayed on another scene).
 bool train_inner(const aloha_ctx* c, int n_views, const int* view_ids) {
   if (!params_inner(c->params)) return false;
-  for (const DevBrick& b : c->dev_bricks)
-    if (!b.inner) return false;
+  if (!scene_is_inner(c)) return false;
   for (int i = 0; i < n_views; ++i)
     if (!view_inner(c->views[view_ids[i]])) return false;
   return true;

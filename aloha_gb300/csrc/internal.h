@@ -79,11 +79,13 @@ constexpr int kCellFull = 0x80;
 //    direction: DevView::inner;
 //  - the step is at most kInnerStep and a constant jitter at most kInnerJitter
 //    steps: FrameArgs::inner.
+// For what the march does with samples of alpha 0 (composite_in_run), the
+// transfer function's entries also lie within +-kInnerTable.
 // Ray parameters then stay below 2^17, and their rounding, the lattice's and
 // the position's add up to less than 1/16 voxel.  Anything else takes the
 // clamped form, which gives the same bits.
 constexpr float kInnerSpace = 16384.0f, kInnerEye = 32768.0f, kInnerValue = 1024.0f, kInnerStep = 1024.0f,
-                kInnerJitter = 16.0f;
+                kInnerJitter = 16.0f, kInnerTable = 1e18f;
 
 // One brick as the kernels see it (80 bytes).
 struct DevBrick {
@@ -124,7 +126,7 @@ struct FrameArgs {
   float heat_map_scale;
   int composite_mode, island_id, num_islands;
   int inner;                    // InnerCoords
-  const int* scene_inner;       // 1 when every brick is InnerCoords
+  const int* scene_inner;       // 1 when every brick and the transfer function are InnerCoords
   // outputs
   uint32_t* fb;                 // [H*W] (single view) RGBA8
   float4* rank_images;          // [n_ranks][H*W] or null

@@ -464,6 +464,22 @@ __device__ __forceinline__ float cell_exit(const Cell& c, const float d[3], floa
                      (face(c.z, d[2]) - offz) * idz), t1);
 }
 
+// composite_step of a sample in a run, which may lie in an empty macrocell.  Its
+// alpha is exactly 0 there, which leaves the colour unchanged as long as its
+// shade and its colours are finite.  With InnerCoords they are (values, so
+// gradients, and table entries are bounded; but for a gradient of exactly -1e-4
+// along all three axes, whose shade divides by 0).  Elsewhere, next to a fill
+// value of 1e38 say, they need not be: there such a sample is looked up, and in
+// an empty macrocell it is left out, as a jump over it would have.
+template <bool INNER, class At>
+__device__ __forceinline__ void composite_in_run(float4& color, const float4& c, float shade, At cell) {
+  if constexpr (!INNER) {
+    const float zero = fmaf(0.0f, shade, 0.0f * ((c.x + c.y) + (c.z + c.w)));
+    if (zero != 0.0f && cell().empty()) return;
+  }
+  composite_step(color, c, shade);
+}
+
 // A march hook sees every sample, full or skipped, before it is taken: its
 // t, the samples already taken in the brick and the colour so far.  The
 // render passes NoHook; the differentiable forward stores checkpoints.  An
@@ -563,8 +579,8 @@ __device__ __forceinline__ uint32_t march_brick(const DevBrick& b, const float4*
       }
     }
     if (jumps == kMarchJumps) continue;
-    // Up to kMarchRun samples without another lookup (a full sample in an empty
-    // macrocell leaves the colour unchanged as well).
+    // Up to kMarchRun samples without another lookup (one in an empty macrocell
+    // leaves the colour unchanged as well: composite_in_run).
     int k = 0;
     auto step = [&]() {
       if (!(k < kMarchRun && t < t1 && color.w < et && n < cap)) return false;
@@ -582,7 +598,7 @@ __device__ __forceinline__ uint32_t march_brick(const DevBrick& b, const float4*
         s = stencil<INNER>(base, sy, sz, nx, ny, nz, ux, uy, uz);
       const float shade = shade_factor(s, r);
       const float4 c = tf_lookup<INNER>(tf_s, n_tf, nf, s.value);
-      composite_step(color, c, shade);
+      composite_in_run<INNER>(color, c, shade, [&] { return cell_at(cells, mnx, mny, nx, ny, nz, ux, uy, uz); });
       t = t + dt;
       return true;
     };
@@ -770,13 +786,18 @@ __device__ __forceinline__ uint32_t march_brick_pair(const DevBrick& b, const fl
       const float os = __shfl_xor_sync(g.mask, shade, 1);
       const float ox = __shfl_xor_sync(g.mask, c.x, 1), oy = __shfl_xor_sync(g.mask, c.y, 1);
       const float oz = __shfl_xor_sync(g.mask, c.z, 1), ow = __shfl_xor_sync(g.mask, c.w, 1);
-      composite_step(color, make_float4(first ? c.x : ox, first ? c.y : oy, first ? c.z : oz, first ? c.w : ow),
-                     first ? shade : os);
+      const auto cell = [&] {  // at t, in both lanes
+        return cell_at(cells, mnx, mny, nx, ny, nz, fmaf(t, r.d[0], r.o[0]) - lox, fmaf(t, r.d[1], r.o[1]) - loy,
+                       fmaf(t, r.d[2], r.o[2]) - loz);
+      };
+      composite_in_run<INNER>(color, make_float4(first ? c.x : ox, first ? c.y : oy, first ? c.z : oz, first ? c.w : ow),
+                              first ? shade : os, cell);
       ++n;
       t = t2;
       if (two && color.w < et) {
-        composite_step(color, make_float4(first ? ox : c.x, first ? oy : c.y, first ? oz : c.z, first ? ow : c.w),
-                       first ? os : shade);
+        composite_in_run<INNER>(color,
+                                make_float4(first ? ox : c.x, first ? oy : c.y, first ? oz : c.z, first ? ow : c.w),
+                                first ? os : shade, cell);
         ++n;
         t = t + dt;
       }
