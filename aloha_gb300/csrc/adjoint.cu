@@ -213,7 +213,7 @@ __device__ __forceinline__ uint32_t train_subtile(const TrainArgs& a, const Trai
       if (!slab(ray, b.space_lo, b.space_hi, hook.tmin, 1e10f, t0, t1)) continue;
       const float ils = jitter(a.jitter_mode, a.jitter_value, pixel, (uint32_t)a.accum_id, hook.draw++);
       hook.j = j;
-      n += march_brick<INNER>(b, tf_s, a.n_tf, ray, t0, t1, ils, a.dt, a.et_alpha, color, hook);
+      n += march_brick<INNER>(b, tf_s, a.n_tf, ray, t0, t1, ils, a.dt, a.et_alpha, a.tame, color, hook);
       hook.tmin = t1 + 1e-20f;
       if (!(color.w < a.et_alpha)) break;
     }

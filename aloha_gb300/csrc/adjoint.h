@@ -53,6 +53,7 @@ struct TrainArgs {
   int jitter_mode;
   float jitter_value;
   int accum_id;
+  bool tame;                  // kSceneTame
   unsigned k;                 // checkpoint interval (samples) of every view of the launch
   const TrainView* tv;        // [n_views] the launch's views
   int n_views;

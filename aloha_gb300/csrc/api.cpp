@@ -144,17 +144,18 @@ struct aloha_ctx {
   std::vector<DevBrick> dev_bricks;
   std::vector<char> brick_present;
   std::vector<char> brick_inner_box;  // the box part of DevBrick::inner
+  std::vector<char> brick_tame;       // values within +-kTame
   std::vector<size_t> brick_offset;  // quad offset of each padded brick in `voxels`
   DeviceBuffer voxels, bricks_dev, staging_in;
-  DeviceBuffer scene_inner;  // int: scene_is_inner
+  DeviceBuffer scene_flags;  // int: kScene* (compute_scene_flags)
   PinnedBuffer upload_flags;  // int the upload kernel sets (kVoxel*)
   int* upload_flags_dev = nullptr;
-  int scene_inner_host = 0;
+  int scene_flags_host = 0;
   float bounds_lo[3] = {0, 0, 0}, bounds_hi[3] = {0, 0, 0};
   // transfer function
   DeviceBuffer tf;
   int n_tf = 0;
-  bool tf_inner = true;  // entries within +-kInnerTable
+  bool tf_tame = true;  // entries within +-kTame
   // empty-space macrocells: value range per macrocell (per brick) and the
   // per-transfer-function empty mask, refreshed before the next render
   DeviceBuffer mc_ranges, mc_codes;
@@ -689,7 +690,7 @@ FrameArgs frame_args(aloha_ctx* c) {
   a.island_id = p.island_id;
   a.num_islands = p.num_islands;
   a.inner = params_inner(p);
-  a.scene_inner = static_cast<const int*>(c->scene_inner.ptr);
+  a.scene_flags = static_cast<const int*>(c->scene_flags.ptr);
   a.counter = static_cast<unsigned long long*>(c->counter.ptr);
   return a;
 }
@@ -843,8 +844,8 @@ int aloha_create(int device, aloha_ctx** out) {
   if (c->views_dev.ensure(sizeof(DevView) * kMaxViews) != cudaSuccess ||
       c->counter.ensure(sizeof(unsigned long long)) != cudaSuccess || c->upload_flags.ensure(sizeof(int)) != cudaSuccess ||
       !(c->upload_flags_dev = static_cast<int*>(c->upload_flags.device())) ||
-      c->work.ensure(sizeof(unsigned int)) != cudaSuccess || c->scene_inner.ensure(sizeof(int)) != cudaSuccess ||
-      cudaMemset(c->scene_inner.ptr, 0, sizeof(int)) != cudaSuccess) {
+      c->work.ensure(sizeof(unsigned int)) != cudaSuccess || c->scene_flags.ensure(sizeof(int)) != cudaSuccess ||
+      cudaMemset(c->scene_flags.ptr, 0, sizeof(int)) != cudaSuccess) {
     delete c;
     return ALOHA_ERR_OUT_OF_MEMORY;
   }
@@ -860,7 +861,7 @@ int aloha_destroy(aloha_ctx* c) {
     if (v.accum) cudaFree(v.accum);
     v.train.release();
   }
-  for (DeviceBuffer* b : {&c->voxels, &c->bricks_dev, &c->scene_inner, &c->staging_in, &c->tf, &c->views_dev, &c->sched_dev,
+  for (DeviceBuffer* b : {&c->voxels, &c->bricks_dev, &c->scene_flags, &c->staging_in, &c->tf, &c->views_dev, &c->sched_dev,
                           &c->counter, &c->staging_out, &c->mc_ranges, &c->mc_codes,
                           &c->work, &c->grad4, &c->split_images, &c->split_masks, &c->split_items,
                           &c->split_done, &c->chunk_order, &c->train_tables, &c->train_counts})
@@ -884,23 +885,23 @@ int aloha_set_render_params(aloha_ctx* c, const aloha_render_params* p) {
   return ALOHA_OK;
 }
 
-// InnerCoords, as far as bricks and transfer function go.
-static bool scene_is_inner(const aloha_ctx* c) {
-  bool all = c->tf_inner;
-  for (const DevBrick& b : c->dev_bricks) all = all && b.inner;
-  return all;
+static int compute_scene_flags(const aloha_ctx* c) {
+  bool inner = true, tame = c->tf_tame;
+  for (const DevBrick& b : c->dev_bricks) inner = inner && b.inner;
+  for (char t : c->brick_tame) tame = tame && t;
+  return (inner && tame ? kSceneInner : 0) | (tame ? kSceneTame : 0);
 }
 
-// Brings the device's scene_inner up to date.  The kernels drop their clamps on
+// Brings the device's scene_flags up to date.  The kernels drop their clamps on
 // its word, so it has to be there when the call returns: a copy from pageable
 // memory returns before it has landed, and streams that do not wait for the
 // default stream would still read the old value.
-static int upload_scene_inner(aloha_ctx* c) {
-  const int all = scene_is_inner(c);
-  if (all == c->scene_inner_host) return ALOHA_OK;
-  CUDA_TRY(c, cudaMemcpy(c->scene_inner.ptr, &all, sizeof all, cudaMemcpyHostToDevice));
+static int upload_scene_flags(aloha_ctx* c) {
+  const int flags = compute_scene_flags(c);
+  if (flags == c->scene_flags_host) return ALOHA_OK;
+  CUDA_TRY(c, cudaMemcpy(c->scene_flags.ptr, &flags, sizeof flags, cudaMemcpyHostToDevice));
   CUDA_TRY(c, cudaStreamSynchronize(0));
-  c->scene_inner_host = all;
+  c->scene_flags_host = flags;
   return ALOHA_OK;
 }
 
@@ -926,9 +927,9 @@ static int upload_brick(aloha_ctx* c, int b, const float* src) {
   c->empty_dirty = true;
   CUDA_TRY(c, cudaStreamSynchronize(0));
   const int flags = *flags_host;
+  db.inner = c->brick_inner_box[b] && !(flags & (kVoxelWide | kVoxelNonfinite));
+  c->brick_tame[b] = !(flags & (kVoxelHuge | kVoxelNonfinite));
   if (flags & kVoxelNonfinite) return c->fail(ALOHA_ERR_INVALID_ARGUMENT, "brick %d holds a non-finite voxel", b);
-  const int inner = c->brick_inner_box[b] && !(flags & kVoxelWide);
-  db.inner = inner;
   c->brick_present[b] = 1;
   invalidate_training(c);
   return ALOHA_OK;
@@ -1010,6 +1011,7 @@ int aloha_set_bricks(aloha_ctx* c, const aloha_brick_desc* descs, const float* c
   c->brick_offset = offs;
   c->brick_present.assign(n, 0);
   c->brick_inner_box = inner_box;
+  c->brick_tame.assign(n, 1);
   c->boxes.resize(n);
   for (int a = 0; a < 3; ++a) {
     c->bounds_lo[a] = 1e30f;
@@ -1026,7 +1028,7 @@ int aloha_set_bricks(aloha_ctx* c, const aloha_brick_desc* descs, const float* c
   CUDA_TRY(c, cudaMemcpy(c->bricks_dev.ptr, db.data(), sizeof(DevBrick) * n, cudaMemcpyHostToDevice));
   // what the boxes say goes first: a launch recorded earlier may be replayed
   // even if a brick below is refused
-  int rc = upload_scene_inner(c);
+  int rc = upload_scene_flags(c);
   if (rc) return rc;
   for (int b = 0; b < n; ++b) {
     rc = upload_brick(c, b, voxels[b]);
@@ -1035,7 +1037,7 @@ int aloha_set_bricks(aloha_ctx* c, const aloha_brick_desc* descs, const float* c
       return rc;
     }
   }
-  rc = upload_scene_inner(c);
+  rc = upload_scene_flags(c);
   if (rc) return rc;
   c->staging_in.release();
   c->sched_stride = 0;
@@ -1048,7 +1050,8 @@ int aloha_update_brick(aloha_ctx* c, int brick, const float* voxels) {
   CUDA_TRY(c, cudaSetDevice(c->device));
   CUDA_TRY(c, cudaDeviceSynchronize());
   const int rc = upload_brick(c, brick, voxels);
-  return rc ? rc : upload_scene_inner(c);
+  const int flags_rc = upload_scene_flags(c);  // also of a brick that was refused: its array is overwritten
+  return rc ? rc : flags_rc;
 }
 
 int aloha_drop_brick(aloha_ctx* c, int brick) {
@@ -1084,9 +1087,9 @@ int aloha_set_transfer_function(aloha_ctx* c, const float* rgba, int n) {
   CUDA_TRY(c, cudaStreamSynchronize(0));  // landed, for renders on streams that do not wait for this one
   c->empty_dirty = true;
   c->n_tf = n;
-  c->tf_inner = std::all_of(h.begin(), h.begin() + entries, [](float v) { return std::fabs(v) <= kInnerTable; });
+  c->tf_tame = std::all_of(h.begin(), h.begin() + entries, [](float v) { return std::fabs(v) <= kTame; });
   invalidate_training(c);
-  return c->dev_bricks.empty() ? ALOHA_OK : upload_scene_inner(c);
+  return c->dev_bricks.empty() ? ALOHA_OK : upload_scene_flags(c);
 }
 
 int aloha_set_ranks(aloha_ctx* c, int n_ranks) {
@@ -1424,6 +1427,7 @@ TrainArgs train_args(aloha_ctx* c) {
   a.jitter_mode = p.jitter_mode;
   a.jitter_value = p.jitter_value;
   a.accum_id = p.accum_id;
+  a.tame = compute_scene_flags(c) & kSceneTame;
   a.counter = static_cast<unsigned long long*>(c->counter.ptr);
   return a;
 }
@@ -1433,7 +1437,7 @@ TrainArgs train_args(aloha_ctx* c) {
 // graph and replayed on another scene).
 bool train_inner(const aloha_ctx* c, int n_views, const int* view_ids) {
   if (!params_inner(c->params)) return false;
-  if (!scene_is_inner(c)) return false;
+  if (!(compute_scene_flags(c) & kSceneInner)) return false;
   for (int i = 0; i < n_views; ++i)
     if (!view_inner(c->views[view_ids[i]])) return false;
   return true;

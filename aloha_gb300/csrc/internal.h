@@ -79,13 +79,20 @@ constexpr int kCellFull = 0x80;
 //    direction: DevView::inner;
 //  - the step is at most kInnerStep and a constant jitter at most kInnerJitter
 //    steps: FrameArgs::inner.
-// For what the march does with samples of alpha 0 (composite_in_run), the
-// transfer function's entries also lie within +-kInnerTable.
+//  - the scene is tame (below): kSceneInner.
 // Ray parameters then stay below 2^17, and their rounding, the lattice's and
 // the position's add up to less than 1/16 voxel.  Anything else takes the
 // clamped form, which gives the same bits.
 constexpr float kInnerSpace = 16384.0f, kInnerEye = 32768.0f, kInnerValue = 1024.0f, kInnerStep = 1024.0f,
-                kInnerJitter = 16.0f, kInnerTable = 1e18f;
+                kInnerJitter = 16.0f;
+
+// A scene is tame (kSceneTame) when its voxels and its transfer function's
+// entries lie within +-kTame: then every sample's lookup is finite and, but for a
+// gradient of exactly -1e-4 along all three axes (whose shade divides by 0), so
+// is its shade, and a sample of alpha 0 leaves the colour unchanged even if it is
+// evaluated.
+constexpr float kTame = 1e18f;
+constexpr int kSceneInner = 1, kSceneTame = 2;  // FrameArgs::scene_flags
 
 // One brick as the kernels see it (80 bytes).
 struct DevBrick {
@@ -126,7 +133,7 @@ struct FrameArgs {
   float heat_map_scale;
   int composite_mode, island_id, num_islands;
   int inner;                    // InnerCoords
-  const int* scene_inner;       // 1 when every brick and the transfer function are InnerCoords
+  const int* scene_flags;       // kSceneInner: every brick is InnerCoords; kSceneTame
   // outputs
   uint32_t* fb;                 // [H*W] (single view) RGBA8
   float4* rank_images;          // [n_ranks][H*W] or null
@@ -251,8 +258,8 @@ cudaError_t launch_composite_u8(const uint32_t* imgs, const int* order, const in
                                 uint32_t* fb, cudaStream_t s);
 // Fills a brick's padded array from its voxels (x fastest) and the value range
 // of each macrocell.  Sets flag bits: kVoxelNonfinite, kVoxelWide (a value
-// beyond +-kInnerValue).
-constexpr int kVoxelNonfinite = 1, kVoxelWide = 2;
+// beyond +-kInnerValue), kVoxelHuge (beyond +-kTame).
+constexpr int kVoxelNonfinite = 1, kVoxelWide = 2, kVoxelHuge = 4;
 cudaError_t launch_fill_brick(const DevBrick& b, const float* src, float4* dst_alloc, float2* ranges, int* flags,
                               cudaStream_t s);
 // Persistent render launch; `batch` selects the instance tuned for batches.

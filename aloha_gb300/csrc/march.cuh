@@ -464,22 +464,6 @@ __device__ __forceinline__ float cell_exit(const Cell& c, const float d[3], floa
                      (face(c.z, d[2]) - offz) * idz), t1);
 }
 
-// composite_step of a sample in a run, which may lie in an empty macrocell.  Its
-// alpha is exactly 0 there, which leaves the colour unchanged as long as its
-// shade and its colours are finite.  With InnerCoords they are (values, so
-// gradients, and table entries are bounded; but for a gradient of exactly -1e-4
-// along all three axes, whose shade divides by 0).  Elsewhere, next to a fill
-// value of 1e38 say, they need not be: there such a sample is looked up, and in
-// an empty macrocell it is left out, as a jump over it would have.
-template <bool INNER, class At>
-__device__ __forceinline__ void composite_in_run(float4& color, const float4& c, float shade, At cell) {
-  if constexpr (!INNER) {
-    const float zero = fmaf(0.0f, shade, 0.0f * ((c.x + c.y) + (c.z + c.w)));
-    if (zero != 0.0f && cell().empty()) return;
-  }
-  composite_step(color, c, shade);
-}
-
 // A march hook sees every sample, full or skipped, before it is taken: its
 // t, the samples already taken in the brick and the colour so far.  The
 // render passes NoHook; the differentiable forward stores checkpoints.  An
@@ -509,7 +493,7 @@ constexpr int kMarchJumps = 2, kMarchRun = 6;
 template <bool INNER, class Hook, class Loads = DirectLoads>
 __device__ __forceinline__ uint32_t march_brick(const DevBrick& b, const float4* __restrict__ tf_s, int n_tf,
                                                 const Ray& r, float t0, float t1, float ils, float dt, float et,
-                                                float4& color, Hook& hook, Loads& loads) {
+                                                bool tame, float4& color, Hook& hook, Loads& loads) {
   const float4* __restrict__ base = b.base;
   const int sy = b.sy, sz = b.sz, nx = b.n[0], ny = b.n[1], nz = b.n[2];
   const float lox = b.lo[0], loy = b.lo[1], loz = b.lo[2];
@@ -529,6 +513,7 @@ __device__ __forceinline__ uint32_t march_brick(const DevBrick& b, const float4*
   float t = first_sample_t(t0, dt, ils);
   const bool exact = exact_steps(t, t1, dt);
   const float inv_dt = 1.0f / dt;
+  const int run = INNER || tame ? kMarchRun : 1;
   loads.begin_brick();
   while (t < t1 && color.w < et && n < cap) {
     // Up to kMarchJumps steps over empty boxes, until the ray is at a sample in
@@ -580,10 +565,10 @@ __device__ __forceinline__ uint32_t march_brick(const DevBrick& b, const float4*
     }
     if (jumps == kMarchJumps) continue;
     // Up to kMarchRun samples without another lookup (one in an empty macrocell
-    // leaves the colour unchanged as well: composite_in_run).
+    // leaves the colour unchanged as well), or one if the scene is not tame.
     int k = 0;
     auto step = [&]() {
-      if (!(k < kMarchRun && t < t1 && color.w < et && n < cap)) return false;
+      if (!(k < run && t < t1 && color.w < et && n < cap)) return false;
       const float ux = fmaf(t, r.d[0], r.o[0]) - lox;
       const float uy = fmaf(t, r.d[1], r.o[1]) - loy;
       const float uz = fmaf(t, r.d[2], r.o[2]) - loz;
@@ -598,7 +583,7 @@ __device__ __forceinline__ uint32_t march_brick(const DevBrick& b, const float4*
         s = stencil<INNER>(base, sy, sz, nx, ny, nz, ux, uy, uz);
       const float shade = shade_factor(s, r);
       const float4 c = tf_lookup<INNER>(tf_s, n_tf, nf, s.value);
-      composite_in_run<INNER>(color, c, shade, [&] { return cell_at(cells, mnx, mny, nx, ny, nz, ux, uy, uz); });
+      composite_step(color, c, shade);
       t = t + dt;
       return true;
     };
@@ -619,9 +604,9 @@ __device__ __forceinline__ uint32_t march_brick(const DevBrick& b, const float4*
 template <bool INNER, class Hook>
 __device__ __forceinline__ uint32_t march_brick(const DevBrick& b, const float4* __restrict__ tf_s, int n_tf,
                                                 const Ray& r, float t0, float t1, float ils, float dt, float et,
-                                                float4& color, Hook& hook) {
+                                                bool tame, float4& color, Hook& hook) {
   DirectLoads direct;
-  return march_brick<INNER>(b, tf_s, n_tf, r, t0, t1, ils, dt, et, color, hook, direct);
+  return march_brick<INNER>(b, tf_s, n_tf, r, t0, t1, ils, dt, et, tame, color, hook, direct);
 }
 
 // ---- Sample-parallel lane groups ------------------------------------------
@@ -738,7 +723,7 @@ constexpr int kPairRun = 8;
 template <bool INNER>
 __device__ __forceinline__ uint32_t march_brick_pair(const DevBrick& b, const float4* __restrict__ tf_s, int n_tf,
                                                      const Ray& r, float t0, float t1, float ils, float dt, float et,
-                                                     float4& color, const LaneGroup& g) {
+                                                     bool tame, float4& color, const LaneGroup& g) {
   const float4* __restrict__ base = b.base;
   const int sy = b.sy, sz = b.sz, nx = b.n[0], ny = b.n[1], nz = b.n[2];
   const float lox = b.lo[0], loy = b.lo[1], loz = b.lo[2];
@@ -756,6 +741,7 @@ __device__ __forceinline__ uint32_t march_brick_pair(const DevBrick& b, const fl
   float t = first_sample_t(t0, dt, ils);
   const bool exact = exact_steps(t, t1, dt);
   const float inv_dt = 1.0f / dt;
+  const int run = INNER || tame ? kPairRun : 1;  // 1: of the first lane's samples alone
   while (t < t1 && color.w < et && n < cap) {
     int jumps = 0;  // as in march_brick, by both lanes
     for (; jumps < kMarchJumps && t < t1 && n < cap; ++jumps) {
@@ -772,11 +758,11 @@ __device__ __forceinline__ uint32_t march_brick_pair(const DevBrick& b, const fl
     }
     if (jumps == kMarchJumps) continue;
 #pragma unroll 1
-    for (int k = 0; k < kPairRun && t < t1 && color.w < et && n < cap; k += 2) {
+    for (int k = 0; k < run && t < t1 && color.w < et && n < cap; k += 2) {
       // past the ray's end the second lane takes the first one's sample again
       // (its coordinates are known to be the brick's) and drops it
       const float t2 = t + dt;
-      const bool two = t2 < t1 && n + 1 < cap;
+      const bool two = t2 < t1 && n + 1 < cap && (INNER || run > 1);
       const float tk = !first && two ? t2 : t;
       const StencilOut s =
           stencil<INNER>(base, sy, sz, nx, ny, nz, fmaf(tk, r.d[0], r.o[0]) - lox, fmaf(tk, r.d[1], r.o[1]) - loy,
@@ -786,18 +772,13 @@ __device__ __forceinline__ uint32_t march_brick_pair(const DevBrick& b, const fl
       const float os = __shfl_xor_sync(g.mask, shade, 1);
       const float ox = __shfl_xor_sync(g.mask, c.x, 1), oy = __shfl_xor_sync(g.mask, c.y, 1);
       const float oz = __shfl_xor_sync(g.mask, c.z, 1), ow = __shfl_xor_sync(g.mask, c.w, 1);
-      const auto cell = [&] {  // at t, in both lanes
-        return cell_at(cells, mnx, mny, nx, ny, nz, fmaf(t, r.d[0], r.o[0]) - lox, fmaf(t, r.d[1], r.o[1]) - loy,
-                       fmaf(t, r.d[2], r.o[2]) - loz);
-      };
-      composite_in_run<INNER>(color, make_float4(first ? c.x : ox, first ? c.y : oy, first ? c.z : oz, first ? c.w : ow),
-                              first ? shade : os, cell);
+      composite_step(color, make_float4(first ? c.x : ox, first ? c.y : oy, first ? c.z : oz, first ? c.w : ow),
+                     first ? shade : os);
       ++n;
       t = t2;
       if (two && color.w < et) {
-        composite_in_run<INNER>(color,
-                                make_float4(first ? ox : c.x, first ? oy : c.y, first ? oz : c.z, first ? ow : c.w),
-                                first ? os : shade, cell);
+        composite_step(color, make_float4(first ? ox : c.x, first ? oy : c.y, first ? oz : c.z, first ? ow : c.w),
+                       first ? os : shade);
         ++n;
         t = t + dt;
       }
@@ -827,6 +808,8 @@ __device__ __forceinline__ uint32_t quantize8(float x) {
 __device__ __forceinline__ uint32_t pack_rgba(float4 c) {
   return quantize8(c.x) | (quantize8(c.y) << 8) | (quantize8(c.z) << 16) | (quantize8(c.w) << 24);
 }
+
+__device__ __forceinline__ bool scene_inner(const FrameArgs& a) { return __ldg(a.scene_flags) & kSceneInner; }
 
 // Loads the transfer function into shared memory with two zero entries on
 // each side (border addressing).
@@ -859,12 +842,13 @@ __device__ __forceinline__ float4 march_rank(const FrameArgs& a, const DevView& 
       const float tnear = (t0 > tmin ? t0 : 0.0f) + tmin;
       z = fminf(z, tnear / v.max_depth);
       NoHook none;
+      const bool tame = INNER || (__ldg(a.scene_flags) & kSceneTame);
       if constexpr (G == 2) {
-        ns += march_brick_pair<INNER>(b, tf_s, a.n_tf, ray, t0, t1, ils, a.dt, a.et_alpha, color, g);
+        ns += march_brick_pair<INNER>(b, tf_s, a.n_tf, ray, t0, t1, ils, a.dt, a.et_alpha, tame, color, g);
       } else if constexpr (G > 1) {
         ns += march_brick_group<G>(b, tf_s, a.n_tf, ray, t0, t1, ils, a.dt, a.et_alpha, color, g);
       } else {
-        ns += march_brick<INNER>(b, tf_s, a.n_tf, ray, t0, t1, ils, a.dt, a.et_alpha, color, none, loads);
+        ns += march_brick<INNER>(b, tf_s, a.n_tf, ray, t0, t1, ils, a.dt, a.et_alpha, tame, color, none, loads);
       }
       tmin = t1 + 1e-20f;
       if (!(color.w < a.et_alpha)) break;

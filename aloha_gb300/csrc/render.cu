@@ -21,7 +21,7 @@ __device__ __forceinline__ uint32_t render_half_chunk(const BatchArgs& b, const 
   const LaneGroup g{lane & 1, 3u << (lane & 30), lane & 30};
   const size_t at = (size_t)x + (size_t)v.width * y;
   uint32_t ns;
-  if (INNER || (b.f.inner && v.inner && *b.f.scene_inner))
+  if (INNER || (b.f.inner && v.inner && scene_inner(b.f)))
     ns = render_pixel<true, Loads, 2, true>(b.f, v, tf_s, x, y, fb, at, loads, g);
   else
     ns = render_pixel<false, Loads, 2, true>(b.f, v, tf_s, x, y, fb, at, loads, g);
@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(kRenderThreads, MINB) render_warps_kernel(Batc
   if constexpr (STAGE == 1) loads.init(tf_s + (b.f.n_tf + 4));
   // pairs are for InnerCoords scenes alone here (fewer copies of the march)
   const bool may_pair =
-      LG == 2 && b.pair_chunks && b.f.inner && b.f.views[b.single_view].inner && *b.f.scene_inner;
+      LG == 2 && b.pair_chunks && b.f.inner && b.f.views[b.single_view].inner && scene_inner(b.f);
   wait_for_primary();  // the chunk order and the cleared counters
   const int lane = threadIdx.x & 31;
   const int pairs = LG == kRingPairs ? b.total_tiles : (may_pair ? __ldcg(b.pair_chunks) : 0);
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kRenderThreads, MINB) render_warps_kernel(Batc
     // branch cost what it saved; the clamped march as an out-of-line call made
     // the 72-register instances spill around it (uneven batch 10.8 ms, against
     // 9.7 ms this way and 9.6 ms without a clamped form).
-    const bool inner = Loads::kInner && b.f.inner && v.inner && *b.f.scene_inner;
+    const bool inner = Loads::kInner && b.f.inner && v.inner && scene_inner(b.f);
 #pragma unroll 1
     for (int sub = 0; sub < (CW / 8) * (CH / 4); ++sub) {
       const int x = x0 + (sub % (CW / 8)) * 8 + tile_x(lane);
@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(kRenderThreads, MINB) render_split_kernel(Spli
   const int cxn = (W + 7) / 8, cyn = (H + 3) / 4;
   const uint32_t n_items = *s.n_items;
   float4* __restrict__ planes = s.f.rank_images;
-  const bool inner = s.f.inner && s.f.views[s.view].inner && *s.f.scene_inner;
+  const bool inner = s.f.inner && s.f.views[s.view].inner && scene_inner(s.f);
   uint32_t n = 0;
   for (;;) {
     uint32_t item = 0;
@@ -435,7 +435,7 @@ __global__ void composite_u8_kernel(const uint32_t* __restrict__ imgs, const __g
 // Fills a brick's padded array: element (x,y,z) holds V(x,y,z), V(x,y,z+1),
 // V(x,y+1,z), V(x,y+1,z+1) with every index clamped to the brick (the apron and
 // the quads' far rows and slices repeat edge values); flags non-finite voxels
-// and values too large for InnerCoords (in page-locked host memory); and takes each macrocell's value range:
+// and values too large for InnerCoords or a tame scene (in page-locked host memory); and takes each macrocell's value range:
 // a sample whose value-tap cell is c (c = clamp(floor(u), 0, n-1)) reads voxels
 // c and c+1 (clamped), so macrocell m covers voxels [m*kMacro, m*kMacro +
 // kMacro] per axis.  A CTA takes kMacro rows of kMacro slices, each thread one
@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(kFillThreads) fill_brick_kernel(const float* _
   const int mnx = (nx + kMacro - 1) >> kMacroShift, mny = (ny + kMacro - 1) >> kMacroShift;
   const bool in_cells = my >= 0 && my < mny && mz >= 0 && mz * kMacro < nz;
   const int t = (int)threadIdx.x;
-  bool bad = false, wide = false;
+  bool bad = false, wide = false, huge = false;
   for (int x0 = -kMacro; x0 < px - kApron; x0 += kFillColumns) {
     const int x = x0 + t, xc = min(max(x, 0), nx - 1);
     float v[N][N];  // [z][y]
@@ -473,6 +473,7 @@ __global__ void __launch_bounds__(kFillThreads) fill_brick_kernel(const float* _
         bad |= !isfinite(v[k][j]);
       }
     wide |= hi > kInnerValue || lo < -kInnerValue;
+    huge |= hi > kTame || lo < -kTame;
     if (t < kFillColumns && x >= -kApron && x < px - kApron) {
 #pragma unroll
       for (int k = 0; k < kMacro; ++k)
@@ -502,7 +503,8 @@ __global__ void __launch_bounds__(kFillThreads) fill_brick_kernel(const float* _
       }
     }
   }
-  if (bad || wide) atomicOr_system(flags, (bad ? kVoxelNonfinite : 0) | (wide ? kVoxelWide : 0));
+  if (bad || wide)
+    atomicOr_system(flags, (bad ? kVoxelNonfinite : 0) | (wide ? kVoxelWide : 0) | (huge ? kVoxelHuge : 0));
 }
 
 // Macrocell codes.  A macrocell is empty when every transfer-function entry

@@ -32,7 +32,7 @@ inline std::map<cudaStream_t, std::vector<std::function<void()>>> pending;
 inline size_t device_bytes = size_t(280) << 30, device_used = 0;
 inline int waits = 0;                         // waits of the host for a stream or the device
 inline std::vector<aloha::BatchArgs> renders;  // launches of the pixel render
-inline std::vector<int> rendered_inner;       // *scene_inner as each of them would read it
+inline std::vector<int> rendered_flags;       // *scene_flags as each of them would read it
 inline int fill_flags = 0;                    // what the next uploads find (kVoxel*)
 
 inline const Block* find(const void* p) {
@@ -177,7 +177,7 @@ cudaError_t launch_fill_brick(const DevBrick&, const float*, float4*, float2*, i
 cudaError_t launch_render_warps(const BatchArgs& a, int, int, int, bool, cudaStream_t s, int, bool, bool, bool) {
   fake::finish(s);  // the launch runs at once; other streams' work may still be on its way
   fake::renders.push_back(a);
-  fake::rendered_inner.push_back(*a.f.scene_inner);
+  fake::rendered_flags.push_back(*a.f.scene_flags);
   return cudaSuccess;
 }
 cudaError_t launch_macrocell_codes(const DevBrick*, int, int, const float2*, const int*, int, uint8_t*, uint8_t*,

@@ -49,33 +49,43 @@ aloha_ctx* context(const aloha_brick_desc& d, const float* voxels) {
   return c;
 }
 
-// The flag that lets kernels drop their clamps is the scene's when a render is
-// launched on any stream, also one that does not wait for the default stream.
+// The flags that let kernels drop their clamps and lookups are the scene's when
+// a render is launched on any stream, also one that does not wait for the default stream.
 void scene_flag() {
   const float* voxels = static_cast<const float*>(device(8 * 8 * 8 * 4));
   uint32_t* fb = static_cast<uint32_t*>(device(8 * 8 * 4));
   const aloha_brick_desc inside = brick(8, 8, 8), beyond = brick(8, 8, 8, 1.0f);
   aloha_ctx* c = context(inside, voxels);
-  auto inner = [&] {
+  auto flags = [&] {
     CHECK(aloha_render(c, 0, fb, kSide) == ALOHA_OK);
-    return fake::rendered_inner.back();
+    return fake::rendered_flags.back();
   };
-  CHECK(inner() == 1);
+  const int kAll = aloha::kSceneInner | aloha::kSceneTame;
+  CHECK(flags() == kAll);
   CHECK(aloha_set_bricks(c, &beyond, &voxels, 1) == ALOHA_OK);
-  CHECK(inner() == 0);
+  CHECK(flags() == aloha::kSceneTame);
   CHECK(aloha_set_bricks(c, &inside, &voxels, 1) == ALOHA_OK);
-  CHECK(inner() == 1);
+  CHECK(flags() == kAll);
   fake::fill_flags = aloha::kVoxelWide;
   CHECK(aloha_update_brick(c, 0, voxels) == ALOHA_OK);
-  CHECK(inner() == 0);
+  CHECK(flags() == aloha::kSceneTame);
+  fake::fill_flags = aloha::kVoxelWide | aloha::kVoxelHuge;
+  CHECK(aloha_update_brick(c, 0, voxels) == ALOHA_OK);
+  CHECK(flags() == 0);
   fake::fill_flags = 0;
   CHECK(aloha_update_brick(c, 0, voxels) == ALOHA_OK);
-  CHECK(inner() == 1);
+  CHECK(flags() == kAll);
+  float tf[8] = {0, 0, 0, 0, 1, 2e18f, 1, 1};
+  CHECK(aloha_set_transfer_function(c, tf, 2) == ALOHA_OK);
+  CHECK(flags() == 0);
+  tf[5] = 1e18f;
+  CHECK(aloha_set_transfer_function(c, tf, 2) == ALOHA_OK);
+  CHECK(flags() == kAll);
   // bricks that are refused half-way: a recorded launch may still be replayed
   fake::fill_flags = aloha::kVoxelNonfinite;
-  const int* flag = fake::renders.back().f.scene_inner;
+  const int* flag = fake::renders.back().f.scene_flags;
   CHECK(aloha_set_bricks(c, &beyond, &voxels, 1) == ALOHA_ERR_INVALID_ARGUMENT);
-  CHECK(*flag == 0);
+  CHECK((*flag & aloha::kSceneInner) == 0);
   fake::fill_flags = 0;
   aloha_destroy(c);
 }
