@@ -503,8 +503,22 @@ __global__ void __launch_bounds__(kFillThreads) fill_brick_kernel(const float* _
       }
     }
   }
-  if (bad || wide)
-    atomicOr_system(flags, (bad ? kVoxelNonfinite : 0) | (wide ? kVoxelWide : 0) | (huge ? kVoxelHuge : 0));
+  // One thread per CTA brings what it found to the host's word, and only bits that
+  // are not there yet: a volume of scanner units is wide throughout (256^3: 162 us
+  // with an atomic of every thread over the host link, 87 this way, 83 for values
+  // in range).
+  const int found = (bad ? kVoxelNonfinite : 0) | (wide ? kVoxelWide : 0) | (huge ? kVoxelHuge : 0);
+  if (__syncthreads_or(found)) {
+    __shared__ int found_s[kFillThreads / 32];
+    const int of_warp = (int)__reduce_or_sync(0xffffffffu, (unsigned)found);
+    if ((t & 31) == 0) found_s[t >> 5] = of_warp;
+    __syncthreads();
+    if (t == 0) {
+      int all = 0;
+      for (int w = 0; w < kFillThreads / 32; ++w) all |= found_s[w];
+      if (all & ~*static_cast<volatile int*>(flags)) atomicOr_system(flags, all);
+    }
+  }
 }
 
 // Macrocell codes.  A macrocell is empty when every transfer-function entry
