@@ -364,7 +364,7 @@ int prepare_view(aloha_ctx* c, int view, cudaStream_t s, bool* enqueued = nullpt
     int most = 0;
     for (const DevBrick& b : c->dev_bricks) most = std::max(most, macrocells(b));
     uint8_t* codes = static_cast<uint8_t*>(c->mc_codes.ptr);
-    CUDA_TRY(c, launch_macrocell_codes(static_cast<const DevBrick*>(c->bricks_dev.ptr), (int)c->dev_bricks.size(), most,
+    CUDA_TRY(c, launch_macrocell_codes(static_cast<const DevBrick*>(c->bricks_dev.ptr), (int)c->dev_bricks.size(), most, c->mc_total,
                                        static_cast<const float2*>(c->mc_ranges.ptr),
                                        reinterpret_cast<const int*>(static_cast<const float*>(c->tf.ptr) + 4 * (size_t)c->n_tf), c->n_tf, codes, codes + c->mc_total,
                                        s));

@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include "../../include/aloha.h"
+#include "reach.h"
 
 namespace aloha {
 
@@ -65,8 +66,6 @@ constexpr int kMaxTF = 2048;  // (n + 4) float4 entries stay under 48 KB of shar
 // reach 8, 756 / 7.66 / 3.77; 8^3 cells of reach 5, 763 / 8.23 / 3.90.
 constexpr int kMacroShift = 2;
 constexpr int kMacro = 1 << kMacroShift;
-constexpr int kMaxReach = 8;
-constexpr int kCellFull = 0x80;
 
 // InnerCoords.  When a sample's voxel coordinates provably lie in [-1/4, n +
 // 1/4] along every axis of its brick, the stencil's indices need no clamps (the
@@ -294,7 +293,7 @@ cudaError_t launch_render_warps(const BatchArgs& a, int chunk_w, int chunk_h, in
 // The macrocell codes of all bricks from their value ranges; prefix[k] = number
 // of transfer-function entries below k with non-zero alpha.  Cells of brick b
 // start at bricks[b].cells - cells in each array; tmp is scratch of their size.
-cudaError_t launch_macrocell_codes(const DevBrick* bricks, int n_bricks, int most_cells, const float2* ranges,
+cudaError_t launch_macrocell_codes(const DevBrick* bricks, int n_bricks, int most_cells, size_t all_cells, const float2* ranges,
                                    const int* prefix, int n_tf, uint8_t* cells, uint8_t* tmp, cudaStream_t s);
 inline int macrocells(const DevBrick& b) {
   return ((b.n[0] + kMacro - 1) >> kMacroShift) * ((b.n[1] + kMacro - 1) >> kMacroShift) *

@@ -524,70 +524,90 @@ __global__ void __launch_bounds__(kFillThreads) fill_brick_kernel(const float* _
 // Macrocell codes.  A macrocell is empty when every transfer-function entry
 // its lookups can touch has alpha 0: indices floor(v*n - 1/2) and +1 for v in
 // [lo, hi], with one index of margin on each side for rounding of the
-// interpolated value.  The Chebyshev distance to the other kind is separable:
-// along x first (here, from the kinds of a row's neighbours in shared memory),
-// then over y, then over z, each the smallest max(step, distance there), where
-// a cell of the other kind has distance 0.
-constexpr int kCodeThreads = 256;
+// interpolated value.  The reach is found along x first (here, from the kinds of
+// the neighbours as bits), then over y, then over z (reach.h).  A table change
+// waits for all three passes.  The 17.6 million cells of 1024^3 in 64 bricks take
+// 80 + 63 + 61 us (512^3: 14 + 11 + 11): the first waits for its ranges, 141 MB,
+// four loads in flight per thread; the others are bound by instructions, some 50
+// per cell.  With a loop over each cell's neighbours in every pass and a grid for
+// the largest brick of each, 152 + 170 + 170 (23 + 24 + 24).
+constexpr int kCodeThreads = 256, kKindLoads = 4, kKindCells = kKindLoads * kCodeThreads - 2 * (kMaxReach - 1);
 __global__ void __launch_bounds__(kCodeThreads) macrocell_kinds_kernel(const DevBrick* __restrict__ bricks,
                                                                        const uint8_t* cells,
                                                                        const float2* __restrict__ ranges,
                                                                        const int* __restrict__ prefix, int n,
                                                                        uint8_t* __restrict__ out) {
   constexpr int W = kMaxReach - 1;
-  __shared__ uint8_t kind[kCodeThreads + 2 * W];
+  __shared__ uint32_t full_bits[kKindLoads * kCodeThreads / 32 + 1];
   const DevBrick& b = bricks[blockIdx.y];
   const size_t first = (size_t)(b.cells - cells);
   const int mnx = (b.n[0] + kMacro - 1) >> kMacroShift;
   const int count = mnx * ((b.n[1] + kMacro - 1) >> kMacroShift) * ((b.n[2] + kMacro - 1) >> kMacroShift);
   const float nf = (float)n;
-  for (int i0 = blockIdx.x * kCodeThreads; i0 < count; i0 += gridDim.x * kCodeThreads) {
-    __syncthreads();
-    for (int k = threadIdx.x; k < kCodeThreads + 2 * W; k += kCodeThreads) {
-      const int i = i0 - W + k;
-      if (i < 0 || i >= count) continue;
-      const float2 r = ranges[first + i];
-      const float xl = fminf(fmaxf(r.x * nf - 0.5f, -8.0f), nf + 8.0f);
-      const float xh = fminf(fmaxf(r.y * nf - 0.5f, -8.0f), nf + 8.0f);
+  const int t = (int)threadIdx.x;
+  if (t == 0) full_bits[kKindLoads * kCodeThreads / 32] = 0u;
+  // kKindCells cells per CTA and trip, and W more on either side
+  for (int i0 = blockIdx.x * kKindCells; i0 < count; i0 += gridDim.x * kKindCells) {
+    float2 r[kKindLoads];
+    bool full[kKindLoads];
+#pragma unroll
+    for (int q = 0; q < kKindLoads; ++q) {
+      const int i = i0 - W + q * kCodeThreads + t;
+      r[q] = i >= 0 && i < count ? __ldcs(ranges + first + i) : make_float2(0.0f, 0.0f);
+    }
+#pragma unroll
+    for (int q = 0; q < kKindLoads; ++q) {
+      const float xl = fminf(fmaxf(r[q].x * nf - 0.5f, -8.0f), nf + 8.0f);
+      const float xh = fminf(fmaxf(r[q].y * nf - 0.5f, -8.0f), nf + 8.0f);
       const int lo = max((int)floorf(xl) - 1, 0);
       const int hi = min((int)floorf(xh) + 2, n - 1);
-      kind[k] = lo <= hi && __ldg(prefix + hi + 1) != __ldg(prefix + lo) ? kCellFull : 0;
+      full[q] = lo <= hi && __ldg(prefix + hi + 1) != __ldg(prefix + lo);
+    }
+    __syncthreads();  // the previous cells' readers
+#pragma unroll
+    for (int q = 0; q < kKindLoads; ++q) {
+      const uint32_t bits = __ballot_sync(0xffffffffu, full[q]);
+      if ((t & 31) == 0) full_bits[(q * kCodeThreads + t) >> 5] = bits;
     }
     __syncthreads();
-    const int i = i0 + (int)threadIdx.x;
-    if (i >= count) continue;
-    const uint8_t* at = kind + W + threadIdx.x;
-    const int x = i % mnx, me = at[0];
-    int reach = 1;
-    while (reach < kMaxReach && (x - reach < 0 || at[-reach] == me) && (x + reach >= mnx || at[reach] == me)) ++reach;
-    out[first + i] = (uint8_t)(me | reach);
+#pragma unroll
+    for (int q = 0; q < kKindLoads; ++q) {
+      const int at = q * kCodeThreads + t - W, i = i0 + at;
+      if (at >= 0 && at < kKindCells && i < count) {
+        const uint32_t window = __funnelshift_r(full_bits[at >> 5], full_bits[(at >> 5) + 1], at & 31);
+        out[first + i] = (uint8_t)((full[q] ? kCellFull : 0) | row_reach(window, i % mnx, mnx));
+      }
+    }
   }
 }
 
+// The pass along y (AXIS 1) or z: a thread takes kReachCells cells in a row along
+// the axis, whose neighbours' codes it loads once, coalesced along x.
+constexpr int kReachCells = 8;
 template <int AXIS>
 __global__ void __launch_bounds__(kCodeThreads) macrocell_reach_kernel(const DevBrick* __restrict__ bricks,
                                                                        const uint8_t* cells,
                                                                        const uint8_t* __restrict__ in,
                                                                        uint8_t* __restrict__ out) {
+  constexpr int W = kMaxReach - 1, N = kReachCells + 2 * W;
   const DevBrick& b = bricks[blockIdx.y];
   const size_t first = (size_t)(b.cells - cells);
   const int mnx = (b.n[0] + kMacro - 1) >> kMacroShift, mny = (b.n[1] + kMacro - 1) >> kMacroShift,
             mnz = (b.n[2] + kMacro - 1) >> kMacroShift;
-  const int count = mnx * mny * mnz, stride = AXIS == 1 ? mnx : mnx * mny, len = AXIS == 1 ? mny : mnz;
-  for (int i = blockIdx.x * kCodeThreads + threadIdx.x; i < count; i += gridDim.x * kCodeThreads) {
-    const int p = (i / stride) % len;
-    const int code = in[first + i], me = code & kCellFull;
-    int reach = code & (kCellFull - 1);
-    auto see = [&](int j, int step) {
-      const int c = in[first + i + j * stride];
-      const int there = (c & kCellFull) == me ? c & (kCellFull - 1) : 0;
-      reach = min(reach, max(step, there));
-    };
-    for (int j = 1; j < reach; ++j) {
-      if (p >= j) see(-j, j);
-      if (p + j < len) see(j, j);
-    }
-    out[first + i] = (uint8_t)(me | reach);
+  const int len = AXIS == 1 ? mny : mnz, stride = AXIS == 1 ? mnx : mnx * mny;
+  const int runs = (len + kReachCells - 1) / kReachCells;
+  const int items = mnx * runs * (AXIS == 1 ? mnz : mny);
+  for (int i = blockIdx.x * kCodeThreads + threadIdx.x; i < items; i += gridDim.x * kCodeThreads) {
+    const int x = i % mnx, rest = i / mnx;
+    const int p0 = kReachCells * (AXIS == 1 ? rest % runs : rest / mny);
+    const size_t row = first + x + (AXIS == 1 ? (rest / runs) * mnx * mny : (rest % mny) * mnx);
+    const int8_t* at = reinterpret_cast<const int8_t*>(in) + row;
+    int s[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) s[k] = __ldg(at + min(max(p0 + k - W, 0), len - 1) * stride);
+#pragma unroll
+    for (int k = 0; k < kReachCells; ++k)
+      if (p0 + k < len) out[row + (p0 + k) * stride] = (uint8_t)axis_code(s + W + k);
   }
 }
 
@@ -596,13 +616,19 @@ static size_t render_smem(int n_tf, int stage) {
   return tf_smem(n_tf) + (stage == ALOHA_STAGING_NEXT_SAMPLE ? kStageBytes : 0);
 }
 
-cudaError_t launch_macrocell_codes(const DevBrick* bricks, int n_bricks, int most_cells, const float2* ranges,
+cudaError_t launch_macrocell_codes(const DevBrick* bricks, int n_bricks, int most_cells, size_t all_cells, const float2* ranges,
                                    const int* prefix, int n_tf, uint8_t* cells, uint8_t* tmp, cudaStream_t s) {
   for (int b0 = 0; b0 < n_bricks; b0 += 65535) {  // a grid's y extent
-    const dim3 grid(min((most_cells + kCodeThreads - 1) / kCodeThreads, 152 * 8), min(n_bricks - b0, 65535));
-    macrocell_kinds_kernel<<<grid, kCodeThreads, 0, s>>>(bricks + b0, cells, ranges, prefix, n_tf, cells);
-    macrocell_reach_kernel<1><<<grid, kCodeThreads, 0, s>>>(bricks + b0, cells, cells, tmp);
-    macrocell_reach_kernel<2><<<grid, kCodeThreads, 0, s>>>(bricks + b0, cells, tmp, cells);
+    // the largest brick's share of the CTAs that fill the GPU, and no more than it
+    // has work for: CTAs that find none cost as much as the passes do
+    const int share = (int)((152ll * 8 * most_cells + (long long)all_cells - 1) / (long long)all_cells);
+    auto grid = [&](int per_cta) {
+      return dim3(min((most_cells + per_cta - 1) / per_cta, share), min(n_bricks - b0, 65535));
+    };
+    macrocell_kinds_kernel<<<grid(kKindCells), kCodeThreads, 0, s>>>(bricks + b0, cells, ranges, prefix, n_tf, cells);
+    const dim3 runs = grid(kCodeThreads * kReachCells);
+    macrocell_reach_kernel<1><<<runs, kCodeThreads, 0, s>>>(bricks + b0, cells, cells, tmp);
+    macrocell_reach_kernel<2><<<runs, kCodeThreads, 0, s>>>(bricks + b0, cells, tmp, cells);
   }
   return cudaGetLastError();
 }

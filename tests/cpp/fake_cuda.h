@@ -180,7 +180,7 @@ cudaError_t launch_render_warps(const BatchArgs& a, int, int, int, bool, cudaStr
   fake::rendered_flags.push_back(*a.f.scene_flags);
   return cudaSuccess;
 }
-cudaError_t launch_macrocell_codes(const DevBrick*, int, int, const float2*, const int*, int, uint8_t*, uint8_t*,
+cudaError_t launch_macrocell_codes(const DevBrick*, int, int, size_t, const float2*, const int*, int, uint8_t*, uint8_t*,
                                    cudaStream_t) {
   return cudaSuccess;
 }
