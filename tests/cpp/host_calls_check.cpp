@@ -1,6 +1,8 @@
 // Checks of what the host side of the C ABI (api.cpp) leaves done when a call
 // returns, on a stand-in for the CUDA runtime.  Arguments: the checks to run.
 // Prints one line per failure; status 1 if there was any.
+#include <cmath>
+#include <random>
 #include <string>
 
 #include "aloha.h"
@@ -169,6 +171,61 @@ void large() {
   aloha_destroy(c);
 }
 
+// A view whose rays may take unclamped coordinates has an eye within the limit
+// and a proper direction at every pixel; ordinary cameras are such views.
+void views() {
+  const float* voxels = static_cast<const float*>(device(8 * 8 * 8 * 4));
+  uint32_t* fb = static_cast<uint32_t*>(device(64 * 64 * 4));
+  aloha_ctx* c = context(brick(8, 8, 8), voxels);
+  std::mt19937_64 rng(11u);
+  std::uniform_real_distribution<float> u(-1.0f, 1.0f);
+  int inner = 0, degenerate = 0;
+  for (int k = 0; k < 4000; ++k) {
+    float org[3], d00[3], du[3], dv[3];
+    const float scale = ldexpf(1.0f, (int)(rng() % 60) - 40);  // eyes and pixels of all sizes
+    for (int a = 0; a < 3; ++a) {
+      org[a] = u(rng) * (k % 4 ? 30000.0f : 60000.0f);
+      d00[a] = u(rng) * scale;
+      du[a] = u(rng) * 0.02f * scale;
+      dv[a] = u(rng) * 0.02f * scale;
+    }
+    const int w = 1 + (int)(rng() % 64), h = 1 + (int)(rng() % 64), form = k % 8;
+    const int px = (int)(rng() % w), py = (int)(rng() % h);
+    const float along = u(rng);
+    for (int a = 0; a < 3; ++a) {
+      if (form == 1) dv[a] = du[a] * 2.0f;                           // one line of directions
+      if (form == 3 && (k & 8)) dv[a] = du[a] * 3.0f;
+      if (form == 2) du[a] = dv[a] = 0.0f;                           // one direction
+      if (form == 3) d00[a] = -(px + 0.5f) * du[a] - (py + 0.5f) * dv[a];  // none at a pixel
+      if (form == 4) dv[a] = k & 8 ? nextafterf(du[a], 1e30f) : du[a] * 3.0f;  // almost one line
+      if (form == 5) d00[a] = du[a] * along + dv[a];                  // the eye in the image's plane
+    }
+    degenerate += form >= 1 && form <= 5;
+    CHECK(aloha_set_camera(c, 0, org, d00, du, dv) == ALOHA_OK && aloha_resize(c, 0, w, h) == ALOHA_OK);
+    CHECK(aloha_render(c, 0, fb, kSide) == ALOHA_OK);
+    fake::wait_all();
+    const aloha::DevView& v = fake::renders.back().f.views[0];
+    if (!v.inner) continue;
+    ++inner;
+    CHECK(form != 1 && form != 2 && form != 3 && form != 5);
+    bool proper = true;
+    for (int a = 0; a < 3; ++a) proper = proper && std::fabs(org[a]) <= aloha::kInnerEye;
+    for (int y = 0; y < h; ++y)
+      for (int x = 0; x < w; ++x) {  // generate_ray
+        float d[3], len2 = 0.0f, unit2 = 0.0f;
+        for (int a = 0; a < 3; ++a) d[a] = fmaf(y + 0.5f, dv[a], fmaf(x + 0.5f, du[a], d00[a]));
+        len2 = fmaf(d[2], d[2], fmaf(d[1], d[1], d[0] * d[0]));
+        const float inv = 1.0f / sqrtf(len2);
+        for (int a = 0; a < 3; ++a) unit2 += d[a] * inv * (d[a] * inv);
+        proper = proper && std::fabs(unit2 - 1.0f) < 1e-5f;
+      }
+    CHECK(proper);
+  }
+  CHECK(inner > 500 && degenerate > 2000);
+  fake::renders.clear();
+  aloha_destroy(c);
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -178,6 +235,7 @@ int main(int argc, char** argv) {
     else if (a == "table") table();
     else if (a == "composite") composite();
     else if (a == "large") large();
+    else if (a == "views") views();
     else ++failures;
   }
   std::printf("failures %d\n", failures);
