@@ -189,9 +189,10 @@ struct aloha_ctx {
   int chunk_w = 0, chunk_h = 0;  // 0 = automatic
   int grid_n_tf = -1, grid_blocks = 0, grid_cw = 0, grid_ch = 0;
   bool grid_few = false;
-  // cost-ordered chunks of single-view renders: mode, probe costs | max | order
+  // cost-ordered chunks of single-view renders: mode, keys | chunk ids | order,
+  // and the counters (ChunkOrderArgs::readers, pairs, hist)
   int chunk_order_mode = ALOHA_CHUNKS_AUTO;
-  DeviceBuffer chunk_order;
+  DeviceBuffer chunk_order, chunk_counts;
   // rank-split render: mode, scratch rank images, per-chunk tickets, grid
   int split_mode = ALOHA_SPLIT_AUTO;
   int staging = ALOHA_STAGING_NONE;  // stencil loads of the single-view render kernel
@@ -200,7 +201,6 @@ struct aloha_ctx {
   int grid_blocks_lg = 0, grid_lg_n_tf = -1;
   DeviceBuffer split_images, split_masks, split_items, split_done;
   int split_grid_n_tf = -1, split_grid_blocks = 0;
-  int chunk_order_slots = -1;  // slot count of the chunk-order buffer's current layout
   bool split_grid_many = false;
   uint64_t last_samples = 0;
   bool samples_valid = false;
@@ -457,6 +457,10 @@ int prepare_accum(aloha_ctx* c, int view, cudaStream_t s, float4** out) {
   return ALOHA_OK;
 }
 
+// Chunk-order counters allocated and cleared with the context (frames to 36
+// million pixels), so that no recorded launch is the first to need them.
+constexpr size_t kChunkCountBytes = (2 + (size_t)kOrderClasses * 1100) * sizeof(uint32_t);
+
 constexpr size_t kSplitScratchCap = size_t(16) << 30;  // rank split scratch limit
 
 // Bytes of scratch the rank split of `v` needs: rank image planes, masks,
@@ -556,26 +560,27 @@ int plan_chunk_order(aloha_ctx* c, const FrameArgs& f, int view, int cw, int ch,
   o.ch = ch;
   o.n_slots = ring_slots(v.width, v.height, cw, ch);
   const size_t n_chunks = (size_t)((v.width + cw - 1) / cw) * ((v.height + ch - 1) / ch);
-  const size_t slots = (size_t)o.n_slots, hist = (size_t)kOrderClasses * chunk_order_blocks(o.n_slots) + 2;
+  const size_t slots = (size_t)o.n_slots;
   const size_t key_words = (slots + 3) / 4;  // uint8 keys, padded to whole words
-  const size_t before = c->chunk_order.bytes;
-  CUDA_TRY(c, c->chunk_order.ensure((key_words + slots + hist + n_chunks) * sizeof(uint32_t)));
+  CUDA_TRY(c, c->chunk_order.ensure((key_words + slots + n_chunks) * sizeof(uint32_t)));
   uint32_t* w = static_cast<uint32_t*>(c->chunk_order.ptr);
   o.key = reinterpret_cast<uint8_t*>(w);
   o.cid = reinterpret_cast<int*>(w + key_words);
-  o.hist = w + key_words + slots;
-  o.readers = o.hist + hist - 2;
-  o.pairs = reinterpret_cast<int*>(o.hist + hist - 1);
+  o.order = reinterpret_cast<int*>(w + key_words + slots);
+  // The counters lie in a buffer of their own, at the same place for every frame
+  // size, and the kernels leave them zero: no frame and no recorded launch finds
+  // another's data there, whichever ran last.
+  const size_t count_bytes = (2 + (size_t)kOrderClasses * chunk_order_blocks(o.n_slots)) * sizeof(uint32_t);
+  if (count_bytes > c->chunk_counts.bytes) {
+    CUDA_TRY(c, c->chunk_counts.ensure(count_bytes));
+    CUDA_TRY(c, cudaMemsetAsync(c->chunk_counts.ptr, 0, count_bytes, s));
+  }
+  o.readers = static_cast<uint32_t*>(c->chunk_counts.ptr);
+  o.pairs = static_cast<int*>(c->chunk_counts.ptr) + 1;
+  o.hist = o.readers + 2;
   o.warps = c->num_sms * kFewChunkRenderBlocks * (kRenderThreads / 32);
   if (pairs) *pairs = o.pairs;
-  o.order = reinterpret_cast<int*>(w + key_words + slots + hist);
   o.n_chunks = (int)n_chunks;
-  // the histogram is zero between launches of one layout (the scatter clears
-  // it); a new buffer or another slot count puts it elsewhere
-  if (c->chunk_order.bytes != before || c->chunk_order_slots != o.n_slots) {
-    CUDA_TRY(c, cudaMemsetAsync(o.hist, 0, hist * sizeof(uint32_t), s));
-    c->chunk_order_slots = o.n_slots;
-  }
   o.zero_work = zero_work;
   o.zero_samples = zero_samples;
   CUDA_TRY(c, launch_chunk_order(o, s));
@@ -845,7 +850,9 @@ int aloha_create(int device, aloha_ctx** out) {
       c->counter.ensure(sizeof(unsigned long long)) != cudaSuccess || c->upload_flags.ensure(sizeof(int)) != cudaSuccess ||
       !(c->upload_flags_dev = static_cast<int*>(c->upload_flags.device())) ||
       c->work.ensure(sizeof(unsigned int)) != cudaSuccess || c->scene_flags.ensure(sizeof(int)) != cudaSuccess ||
-      cudaMemset(c->scene_flags.ptr, 0, sizeof(int)) != cudaSuccess) {
+      cudaMemset(c->scene_flags.ptr, 0, sizeof(int)) != cudaSuccess ||
+      c->chunk_counts.ensure(kChunkCountBytes) != cudaSuccess ||
+      cudaMemset(c->chunk_counts.ptr, 0, kChunkCountBytes) != cudaSuccess) {
     delete c;
     return ALOHA_ERR_OUT_OF_MEMORY;
   }
@@ -864,7 +871,7 @@ int aloha_destroy(aloha_ctx* c) {
   for (DeviceBuffer* b : {&c->voxels, &c->bricks_dev, &c->scene_flags, &c->staging_in, &c->tf, &c->views_dev, &c->sched_dev,
                           &c->counter, &c->staging_out, &c->mc_ranges, &c->mc_codes,
                           &c->work, &c->grad4, &c->split_images, &c->split_masks, &c->split_items,
-                          &c->split_done, &c->chunk_order, &c->train_tables, &c->train_counts})
+                          &c->split_done, &c->chunk_order, &c->chunk_counts, &c->train_tables, &c->train_counts})
     b->release();
   c->counts_host.release();
   c->upload_flags.release();

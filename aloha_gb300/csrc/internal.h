@@ -178,7 +178,7 @@ struct ChunkOrderArgs {
   uint32_t* hist;    // [kOrderClasses][chunk_order_blocks(n_slots)] counts; zero between launches
   int warps;         // resident warps of the render
   int* pairs;        // set: chunks at the head of the order that two lanes per ray render sooner
-  uint32_t* readers; // the word after hist: scatter CTAs that have read it; zero between launches
+  uint32_t* readers; // scatter CTAs that have read hist; zero between launches
   int* order;        // [chunks] chunk ids, most expensive first
   int n_chunks;      // chunks of the grid (entries of `order`)
   // counters of the render launch that follows, zeroed by the probe (or null)

@@ -295,8 +295,10 @@ cudaError_t launch_chunk_order(const ChunkOrderArgs& a, cudaStream_t s) {
     e = launch_beside(class_scatter_kernel<false>, blocks, kSortThreads, 0, s, true, a);
   }
   if (e == cudaSuccess) e = cudaGetLastError();
-  if (e != cudaSuccess)  // counts may stay behind: clear them for the next launch
-    cudaMemsetAsync(a.hist, 0, ((size_t)kOrderClasses * blocks + 1) * sizeof(uint32_t), s);
+  if (e != cudaSuccess) {  // counts may stay behind: clear them for the next launch
+    cudaMemsetAsync(a.hist, 0, (size_t)kOrderClasses * blocks * sizeof(uint32_t), s);
+    cudaMemsetAsync(a.readers, 0, sizeof(uint32_t), s);
+  }
   return e;
 }
 

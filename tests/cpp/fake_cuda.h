@@ -33,6 +33,8 @@ inline size_t device_bytes = size_t(280) << 30, device_used = 0;
 inline int waits = 0;                         // waits of the host for a stream or the device
 inline std::vector<aloha::BatchArgs> renders;  // launches of the pixel render
 inline std::vector<int> rendered_flags;       // *scene_flags as each of them would read it
+inline cudaStream_t capturing = reinterpret_cast<cudaStream_t>(-1);  // its work is recorded, not run
+inline int dirty_counts = 0;                  // chunk orders whose counters were not zero when they ran
 inline int fill_flags = 0;                    // what the next uploads find (kVoxel*)
 
 inline const Block* find(const void* p) {
@@ -49,6 +51,7 @@ inline cudaError_t reserve(void** p, size_t bytes, cudaMemoryType type) {
   return cudaSuccess;
 }
 inline void finish(cudaStream_t s) {
+  if (s == capturing) return;
   auto work = std::move(pending[s]);
   pending[s].clear();
   for (auto& w : work) w();
@@ -136,8 +139,8 @@ cudaError_t cudaDeviceSynchronize() {
   fake::wait_all();
   return cudaSuccess;
 }
-cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* st) {
-  *st = cudaStreamCaptureStatusNone;
+cudaError_t cudaStreamIsCapturing(cudaStream_t s, cudaStreamCaptureStatus* st) {
+  *st = s == fake::capturing ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
   return cudaSuccess;
 }
 cudaError_t cudaGetDeviceCount(int* n) {
@@ -160,7 +163,19 @@ const char* cudaGetErrorString(cudaError_t) { return "error"; }
 namespace aloha {
 
 int chunk_order_blocks(int n_slots) { return (n_slots + 1023) / 1024; }
-cudaError_t launch_chunk_order(const ChunkOrderArgs&, cudaStream_t) { return cudaSuccess; }
+// Writes all that the kernels write, and leaves the counters zero as they do.
+cudaError_t launch_chunk_order(const ChunkOrderArgs& a, cudaStream_t s) {
+  fake::pending[s].push_back([a] {
+    bool zero = *a.readers == 0u;
+    for (int i = 0; i < kOrderClasses * chunk_order_blocks(a.n_slots); ++i) zero = zero && a.hist[i] == 0u;
+    fake::dirty_counts += !zero;
+    std::memset(a.key, 0xab, a.n_slots);
+    std::memset(a.cid, 0xab, 4 * (size_t)a.n_slots);
+    std::memset(a.order, 0xab, 4 * (size_t)a.n_chunks);
+    *a.pairs = 3;
+  });
+  return cudaSuccess;
+}
 cudaError_t launch_composite_f32(const float4*, const int*, const int*, int, int npx, int, uint32_t* fb,
                                  cudaStream_t s) {
   fake::pending[s].push_back([=] { std::memset(fb, 0x5a, (size_t)npx * 4); });

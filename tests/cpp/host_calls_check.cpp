@@ -226,6 +226,46 @@ void views() {
   aloha_destroy(c);
 }
 
+// The chunk order's counters are zero whenever its kernels run: after other frame
+// sizes, after a recorded frame that was never replayed, and when one is replayed
+// after frames of other sizes.
+void chunk_counters() {
+  const float* voxels = static_cast<const float*>(device(8 * 8 * 8 * 4));
+  uint32_t* fb = static_cast<uint32_t*>(device(4096 * 4096 * 4));
+  aloha_ctx* c = context(brick(8, 8, 8), voxels);
+  CHECK(aloha_set_chunk_order(c, ALOHA_CHUNKS_PROBED) == ALOHA_OK);
+  const cudaStream_t recorded = reinterpret_cast<cudaStream_t>(0x2000);
+  auto frame = [&](int w, int h, cudaStream_t s) {
+    CHECK(aloha_resize(c, 0, w, h) == ALOHA_OK && aloha_render(c, 0, fb, s) == ALOHA_OK);
+    fake::wait_all();
+  };
+  frame(1024, 1024, kSide);
+  frame(100, 60, kSide);
+  frame(1024, 1024, kSide);
+  frame(3000, 2000, kSide);
+  frame(640, 480, kSide);
+  CHECK(aloha_resize(c, 0, 800, 600) == ALOHA_OK);
+  int n = 0, order[1];
+  CHECK(aloha_get_composite_order(c, 0, order, 1, &n) == ALOHA_OK);  // the view's state is on the device
+  fake::capturing = recorded;
+  CHECK(aloha_render(c, 0, fb, recorded) == ALOHA_OK);
+  const auto graph = fake::pending[recorded];
+  fake::pending[recorded].clear();
+  fake::capturing = reinterpret_cast<cudaStream_t>(-1);
+  frame(800, 600, kSide);
+  auto replay = [&] {
+    for (const auto& work : graph) work();
+  };
+  replay();
+  for (int w : {160, 2048, 700}) {
+    frame(w, w, kSide);
+    replay();
+    frame(w, w, kSide);
+  }
+  CHECK(fake::dirty_counts == 0);
+  aloha_destroy(c);
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -236,6 +276,7 @@ int main(int argc, char** argv) {
     else if (a == "composite") composite();
     else if (a == "large") large();
     else if (a == "views") views();
+    else if (a == "chunk_counters") chunk_counters();
     else ++failures;
   }
   std::printf("failures %d\n", failures);

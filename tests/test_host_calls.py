@@ -25,7 +25,7 @@ def check(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("name", ["scene_flag", "table", "composite", "large", "views"])
+@pytest.mark.parametrize("name", ["scene_flag", "table", "composite", "large", "views", "chunk_counters"])
 def test_calls_leave_the_device_ready(check, name):
     out = subprocess.run([check, name], capture_output=True, text=True, timeout=120)
     assert out.returncode == 0, out.stdout + out.stderr
