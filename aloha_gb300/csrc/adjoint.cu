@@ -734,9 +734,9 @@ __global__ void __launch_bounds__(128, 5) backward_kernel(TrainArgs a) {
 // pending sums instead of eight.  Bound by the L1 data pipe (83 % busy), mostly
 // with the stencil's 96 bytes per sample: so two lanes take a segment's samples
 // in turn, and a quarter warp, the unit of 16-byte loads, covers 2x2 rays by two
-// samples, whose quads collide in fewer banks than those of 2x4 rays (a model of
-// the pipe, confirmed for the first: 55 -> 41 cycles for a warp's seven loads at
-// 0.83 voxels per pixel).  The two lanes want the same bins, and adding to a
+// samples, whose quads collide in fewer banks than those of 2x4 rays (counting
+// the quads that share a 16-byte bank group: 41 instead of 55 cycles for a warp's
+// seven loads at 0.83 voxels per pixel).  The two lanes want the same bins, and adding to a
 // float in shared memory is a loop until no other lane interferes, so the bins
 // are kept in COPIES, interleaved so that a lane's copy has banks of its own.
 // Per pass of a 512^3 1024^2 transfer-function step, ms: one lane and one copy

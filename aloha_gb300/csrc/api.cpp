@@ -157,7 +157,7 @@ struct aloha_ctx {
   int n_tf = 0;
   bool tf_tame = true;  // entries within +-kTame
   // empty-space macrocells: value range per macrocell (per brick) and the
-  // per-transfer-function empty mask, refreshed before the next render
+  // cells' codes for the transfer function, refreshed before the next render
   DeviceBuffer mc_ranges, mc_codes;
   std::vector<size_t> mc_offset;
   size_t mc_total = 0;
@@ -478,10 +478,13 @@ bool rank_split_possible(const aloha_ctx* c, const FrameArgs& f, const ViewState
 }
 
 // Automatic mode: the pixel split for few ranks, the rank split for many.
-// 8 bricks of a 512^3 volume at 1024^2: pixels 0.99 ms, ranks 1.15 ms (the
-// longest chunks spend most of their samples inside one brick).  64 bricks of
-// a 1024^3 volume at 2048^2: pixels 7.08 ms, ranks 6.58 ms (each pixel walks
-// 64 ranks in the pixel split; most chunks are covered by few of them).
+// 8 bricks of a 512^3 volume at 1024^2: pixels 0.59 ms, ranks 0.69 (the longest
+// chunks spend most of their samples inside one brick).  64 bricks of a 1024^3
+// volume at 2048^2: pixels 4.49 ms, ranks 3.86 (each pixel walks 64 ranks in the
+// pixel split; most chunks are covered by few of them).  512^3 at 1024^2: 12
+// bricks 0.62 / 0.70, 24 0.69 / 0.79, 32 0.75 / 0.85, 64 0.99 / 0.94, so there the
+// two cross between 32 and 64 ranks; the line has been at 32 since the march
+// evaluated more of its samples.
 constexpr int kAutoRankSplitRanks = 32;
 
 bool use_rank_split(const aloha_ctx* c, const FrameArgs& f, const ViewState& v) {

@@ -1,4 +1,5 @@
-// march.cuh -- device functions of the volume march (sm_103a).
+// march.cuh -- device functions of the volume march (sm_103a).  (On the times in
+// the comments see internal.h.)
 //
 // Restates the reference's per-pixel path (deviceCode.cpp:94-107 ray
 // generation, 41-57 slab test, 245-254 firstSampleT, 256-298 integrateBrick,
@@ -235,10 +236,11 @@ __device__ __forceinline__ uint32_t inner_origin(int sy, int sz) {
 // INNER: the brick's samples all lie inside it (InnerCoords), no index needs
 // a clamp.  Else ROUND_DOWN picks axis_coord (one conversion per axis) over
 // axis_coord_floors.  All give the same bits.  The march around it is bound by
-// instruction issue and the L1 data pipe in turn (512^3 frame: 63 % of issue
-// slots, 53 % of wavefronts), so both count: unclamped, packed and indexed by
-// floor u it executes 10 % fewer instructions and half the conversions, and
-// loads the same 96 bytes.  512^3 frame 857 -> 815 us, 64^3 frame 104 -> 97,
+// the L1 data pipe in batches (83 % of its cycles; 60 % of issue slots) and by
+// latency, issue and the pipe together in a single frame (512^3: 56 % of issue
+// slots, 60 % of the pipe), so instructions count: unclamped, packed and indexed
+// by floor u it executes 10 % fewer and half the conversions, and loads the same
+// 96 bytes.  512^3 frame 857 -> 815 us, 64^3 frame 104 -> 97,
 // 1024^3 frame of 64 ranks 4.86 -> 4.57 ms, uneven batch 10.0 -> 9.7 ms.
 template <bool INNER, bool ROUND_DOWN = false>
 __device__ __forceinline__ StencilOut stencil(const float4* __restrict__ base, int sy, int sz, int nx, int ny,

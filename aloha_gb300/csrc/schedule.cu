@@ -39,7 +39,7 @@ constexpr int kScanThreads = 1024;
 // chain of dependent table reads of the longest ray, so it reads one code per
 // box of equal cells, not one per stride; with the launches beside each other
 // (launch_chunk_order) a 701x395 frame of 181x113x237 voxels at 2 spp and dt 0.3
-// takes 383 -> 353 us, 512^3 at 1024^2 688 -> 679.
+// took 383 -> 353 us, 512^3 at 1024^2 688 -> 679.
 __device__ uint32_t probe_ray(const ChunkOrderArgs& a, const DevView& v, const int* __restrict__ order,
                               const int* __restrict__ rstart, const int* __restrict__ rbricks, int x, int y) {
   const Ray ray = generate_ray(v, x, y);
@@ -173,6 +173,8 @@ __global__ void __launch_bounds__(kScanThreads) class_scan_kernel(ChunkOrderArgs
 //   wins:   (.23, 18) 148 / 115   (.34, 37) 352 / 298   (.36, 53) 579 / 371
 //           (.38, 26) 199 / 157   (.43, 15) 111 / 99    (.45, 31) 239 / 209   (.50, 53) 561 / 394
 //   losses: (.47, 7) 224 / 252    (.49, 18) 261 / 287   (.51, 7) 68 / 74      (.74, 31) 249 / 254
+// The line below runs between these eleven, narrowly: it leaves (.43, 15) .004 and
+// (.49, 18) .013, where either way costs some 10 %, and a frame near it changes whole.
 // One warp: classes 2 lane and 2 lane + 1 hold t0 and t1 chunks.
 __device__ __forceinline__ void pair_rule(const ChunkOrderArgs& a, int lane, uint32_t t0, uint32_t t1) {
   const float c0 = exp2f(0.25f * (float)(kOrderClasses - 1 - 2 * lane)) - 1.0f;
@@ -276,8 +278,10 @@ int chunk_order_blocks(int n_slots) { return (n_slots + kSortThreads - 1) / kSor
 // again.  Up to kScanBlocks sort blocks the scatter scans the table itself: one
 // launch less, but every CTA reads the whole table, so the work grows with the
 // square of the blocks.  Against the scan kernel, frames of a 64^3 volume:
-// 512^2 (17 blocks) 62.2 -> 58.5 us, 2048^2 (257) 376 -> 368, 4096^2 (1027)
-// 1441 -> 1423; the line lies just above the last.  The scatter, and the render
+// 512^2 (17 blocks) 62.2 -> 58.5 us, 2048^2 (258) 467 -> 458, 4096^2 (1027)
+// 1777 -> 1760, 5120^2 (1603) 2767 -> 2747, 6144^2 (2308) 3956 -> 3968, 8192^2
+// (4101) 6976 -> 7143, 16000^2 (15633) 26510 -> 30400.  The two cross near 2000
+// blocks; the line lies below that, where either is within 1 %.  The scatter, and the render
 // after it, start beside the kernel before them and wait for it when they need
 // its results (programmatic dependent launch).
 cudaError_t launch_chunk_order(const ChunkOrderArgs& a, cudaStream_t s) {

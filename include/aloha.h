@@ -165,7 +165,7 @@ int aloha_set_render_split(aloha_ctx* ctx, int mode);
 /* The order in which warps take the chunks of a single-view render (and of
  * the rank split's (chunk, rank) items, and of aloha_forward).
  * ALOHA_CHUNKS_RING: centre-out square rings.  ALOHA_CHUNKS_PROBED:
- * most expensive first, by a coarse probe of each chunk's centre ray through
+ * most expensive first, by a coarse probe of four rays of each chunk through
  * the empty-space tables (two small kernels before the render), so that the
  * frame does not end on a long chunk started late.  Frames are bit-identical
  * either way.  ALOHA_CHUNKS_AUTO (the default) probes frames of 512^2 pixels
